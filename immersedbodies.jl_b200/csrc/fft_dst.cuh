@@ -4,7 +4,7 @@
 // DST-I (FFTW RODFT00 over both dims, src/fluid.jl:113-115 and 145-166).  Here
 // a 2D solve is three passes over the (nx-1) x (ny-1) field:
 //   X pass   : DST along x of every row            (rows are contiguous)
-//   Y pass   : DST along y, multiply, DST along y  (coalesced column blocks)
+//   Y pass   : the multiplier along y, as a direct solve per column (ytri.cuh)
 //   X pass   : DST along x, with a fused epilogue
 // Each length-(M-1) DST-I is one complex M-point FFT of two packed real lines
 // z = a + i b, pre-twiddled with v_j = sin(pi j/M)(z_j + z_{M-j}) + (z_j - z_{M-j})/2.

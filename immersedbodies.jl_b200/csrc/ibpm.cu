@@ -47,10 +47,8 @@ __global__ void tc_mult_kernel(Mult m, int P, float *tab) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
     if (r >= P) return;
     const int kx = tc_blk(c, P), ky = tc_blk(r, P);
-    tab[(size_t)c * P + r] = (kx != 0 && ky != 0) ? (float)m(m.coef(0), kx, ky) : 0.0f;
+    tab[(size_t)c * P + r] = (kx != 0 && ky != 0) ? (float)m(kx, ky) : 0.0f;
 }
-
-constexpr int kNGWide = 4, kWideBatch = 16;  // Y-pass groups per block for launches over >= kWideBatch fields
 
 thread_local std::string g_create_error;
 
@@ -120,9 +118,9 @@ bool make_plan(int M, PlanT<T> &pl) {
 }
 
 // ---- pass-shape autotuner ----
-// The Y pass (DST along y, spectral multiply, DST along y) runs with NG line
-// pairs (2 NG columns) per block, NG in {1, 2, 4, 8}.  Every NG evaluates the
-// same per-line arithmetic, so the choice changes speed only, never results.
+// The Y pass (ytri.cuh) runs with NG column pairs per block, NG in {1, 2, 4, 8}
+// (8 runs as 4).  Every NG evaluates the same per-column arithmetic, so the
+// choice changes speed only, never results.
 // The best NG depends on the transform length, the precision and how many
 // fields one launch covers (one level, all levels, an ensemble group, a batch
 // of B columns), so the table is keyed by (GPU name, transform length,
@@ -130,7 +128,7 @@ bool make_plan(int M, PlanT<T> &pl) {
 // own scratch fields for each key it will launch (before any graph capture) and
 // keeps the fastest; IBPM_TUNE_CACHE names a text file the table is read from
 // at first use and appended to after tuning, so later processes start tuned.
-// Keys never tuned use the fixed rule (NG = 2, NG = 4 from 16 fields).
+// Keys never tuned use the fixed rule (ytri_wshift).
 // IBPM_TUNE_FORCE_NG forces one NG everywhere (a test knob).
 constexpr int kTuneNGs[4] = {1, 2, 4, 8};
 inline int batch_bucket(int nb) { return nb <= 1 ? 0 : nb <= 4 ? 1 : nb <= 15 ? 2 : nb <= 63 ? 3 : 4; }
@@ -241,6 +239,8 @@ struct Engine final : ibpm_handle {
     Grid g{};
     int nx = 0, ny = 0, L = 0, np = 0, nbody = 0;
     long long nq = 0, ng = 0, nu = 0, nbc = 0;
+    int ldt = 0;       // row pitch and size of a scratch field between passes
+    long long nt = 0;
     std::vector<int> body_kind, body_start;
     std::vector<double> ref_xb, ref_ds;
     bool static_bodies = true;
@@ -327,7 +327,7 @@ struct Engine final : ibpm_handle {
     double fs_last[2] = {0, 0}, gm_last[6] = {0, 0, 0, 0, 0, 0};
     // work
     int kbatch = 1;  // columns per batch in the B setup
-    T *t1 = nullptr, *t2 = nullptr, *rhs = nullptr, *rest = nullptr, *qs1 = nullptr;
+    T *t1 = nullptr, *rhs = nullptr, *rest = nullptr, *qs1 = nullptr;
     double *Ftmp = nullptr, *part = nullptr;
     T *patch = nullptr;
     long long patch_stride = 0;
@@ -399,27 +399,24 @@ struct Engine final : ibpm_handle {
     void resize_batch_buffers(int kb) {
         CK(cudaStreamSynchronize(st));
         const int k2 = std::max(kb, L);
-        const size_t sizes[7] = {sizeof(T) * (size_t)(ng * k2),        sizeof(T) * (size_t)(ng * k2),
-                                 sizeof(T) * (size_t)(patch_stride * kb), sizeof(T) * (size_t)(ng * L * kb),
-                                 sizeof(T) * (size_t)(ng * L * kb),     sizeof(T) * (size_t)(nq * kb),
-                                 sizeof(double) * 2 * (size_t)np * kb};
-        void *fresh[7] = {};
+        const size_t sizes[6] = {sizeof(T) * (size_t)(nt * k2),     sizeof(T) * (size_t)(patch_stride * kb),
+                                 sizeof(T) * (size_t)(ng * L * kb), sizeof(T) * (size_t)(ng * L * kb),
+                                 sizeof(T) * (size_t)(nq * kb),     sizeof(double) * 2 * (size_t)np * kb};
+        void *fresh[6] = {};
         try {
-            for (int k = 0; k < 7; ++k) fresh[k] = dalloc<unsigned char>(sizes[k]);
+            for (int k = 0; k < 6; ++k) fresh[k] = dalloc<unsigned char>(sizes[k]);
         } catch (...) {
             for (void *p : fresh) dfree(p);
             throw;
         }
         drop_graphs();
-        for (void *p : {(void *)t1, (void *)t2, (void *)patch, (void *)Gw, (void *)psiw, (void *)qw, (void *)fcol})
-            dfree(p);
+        for (void *p : {(void *)t1, (void *)patch, (void *)Gw, (void *)psiw, (void *)qw, (void *)fcol}) dfree(p);
         t1 = static_cast<T *>(fresh[0]);
-        t2 = static_cast<T *>(fresh[1]);
-        patch = static_cast<T *>(fresh[2]);
-        Gw = static_cast<T *>(fresh[3]);
-        psiw = static_cast<T *>(fresh[4]);
-        qw = static_cast<T *>(fresh[5]);
-        fcol = static_cast<double *>(fresh[6]);
+        patch = static_cast<T *>(fresh[1]);
+        Gw = static_cast<T *>(fresh[2]);
+        psiw = static_cast<T *>(fresh[3]);
+        qw = static_cast<T *>(fresh[4]);
+        fcol = static_cast<double *>(fresh[5]);
         kbatch = kb;
     }
 
@@ -509,22 +506,6 @@ struct Engine final : ibpm_handle {
         check_launch();
         prof_end(pe, IBPM_KCLASS_XPASS, 2.0 * sizeof(R) * (double)ng * nbatch);
     }
-    template <class D>
-    void ypass_t(const PlanT<typename D::Real> &pl, const typename D::Real *in, typename D::Real *out, long long bs,
-                 int nbatch, Mult m) {
-        int ngy = ypass_ng<typename D::Real>(pl.M, nbatch, D::MC > 0);
-        ypass_ng_launch<D>(ngy, pl, in, out, bs, nbatch, m);
-    }
-    template <class D>
-    void ypass_ng_launch(int ngy, const PlanT<typename D::Real> &pl, const typename D::Real *in,
-                         typename D::Real *out, long long bs, int nbatch, Mult m) {
-        switch (ngy) {
-            case 1: ypass_launch<D, 1>(pl, in, out, bs, nbatch, m); break;
-            case 4: ypass_launch<D, 4>(pl, in, out, bs, nbatch, m); break;
-            case 8: ypass_launch<D, 8>(pl, in, out, bs, nbatch, m); break;
-            default: ypass_launch<D, 2>(pl, in, out, bs, nbatch, m); break;
-        }
-    }
     // the autotuner's key of a Y pass of length M over nbatch fields
     std::string devname;  // the GPU's name, read once at setup (a tuning key's first part)
     template <class R>
@@ -532,21 +513,26 @@ struct Engine final : ibpm_handle {
         return devname + " ypass M=" + std::to_string(M) + (sizeof(R) == 8 ? " fp64" : " fp32") +
                " batch=" + std::to_string(batch_bucket(nbatch));
     }
-    // line pairs per block of a Y pass: forced, tuned, or the fixed rule
+    // column pairs per block of a Y pass: forced, tuned, or the fixed rule
     template <class R>
-    int ypass_ng(int M, int nbatch, bool compile_time) {
+    int ypass_ng(int M, int nbatch) {
         if (const int f = tune_forced_ng()) return f;
         int v = 0;
         if (tune_table().find(ypass_key<R>(M, nbatch), &v)) return v;
-        return compile_time && nbatch >= kWideBatch ? kNGWide : kNG;
+        return 1 << (ytri_wshift<R>(nx - 1, M, nbatch) - 1);
     }
-    // Times every NG of the Y pass over nbatch fields (scratch in -> out, at
-    // least nbatch * ng elements each) and records the fastest; eager only.
+    template <class R>
+    void ypass_launch(int ngy, const R *in, R *out, int nbatch, const YSolve &m) {
+        const int wshift = ngy <= 1 ? 1 : ngy == 2 ? 2 : 3;  // at most kYMaxW columns a block
+        CK(launch_ytri<R>(in, out, nt, ldt, nx - 1, ny, nbatch, wshift, m, st));
+    }
+    // Times every block shape of the Y pass over nbatch fields of scratch (in ->
+    // out, pitched, at least nbatch * nt elements each) and records the fastest;
+    // eager only.
     template <class R>
     void tune_ypass(const R *in, R *out, int nbatch) {
         if (!tune_enabled() || tune_forced_ng()) return;
-        const PlanT<R> &pl = plan_y<R>();
-        const std::string key = ypass_key<R>(pl.M, nbatch);
+        const std::string key = ypass_key<R>(ny, nbatch);
         int have = 0;
         if (tune_table().find(key, &have)) return;
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -558,19 +544,7 @@ struct Engine final : ibpm_handle {
         float best = 1e30f;
         int best_ng = kNG;
         for (int ngy : kTuneNGs) {
-            auto run = [&] {
-                switch (pl.M) {
-                    case 1024: ypass_ng_launch<Pow2Dst<1024, R>>(ngy, pl, in, out, ng, nbatch, mult(MULT_LAPINV, 1, 0)); break;
-                    case 512: ypass_ng_launch<Pow2Dst<512, R>>(ngy, pl, in, out, ng, nbatch, mult(MULT_LAPINV, 1, 0)); break;
-                    case 256: ypass_ng_launch<Pow2Dst<256, R>>(ngy, pl, in, out, ng, nbatch, mult(MULT_LAPINV, 1, 0)); break;
-                    case 384: ypass_ng_launch<MixDst<384, R>>(ngy, pl, in, out, ng, nbatch, mult(MULT_LAPINV, 1, 0)); break;
-                    default: ypass_ng_launch<GenericDst<R>>(ngy, pl, in, out, ng, nbatch, mult(MULT_LAPINV, 1, 0)); break;
-                }
-                CK(cudaGetLastError());
-            };
-            // a block of NG line pairs must fit the shared memory a block may use
-            const size_t need = (size_t)ngy * (size_t)(pl.M + 1 + (pl.M + 1) / 16 + 1) * 2 * sizeof(R) + 16 * 8 * ngy;
-            if (need > 220 * 1024) continue;
+            auto run = [&] { ypass_launch<R>(ngy, in, out, nbatch, ysolve(MULT_LAPINV, 1, 0)); };
             run();
             run();
             CK(cudaEventRecord(e0, st));
@@ -588,35 +562,11 @@ struct Engine final : ibpm_handle {
         cudaEventDestroy(e1);
         tune_table().put(key, best_ng);
     }
-    // Y pass with NGY line pairs (2 NGY columns) per block.  Launches over many
-    // fields (the B assembly) have waves to spare, and wider blocks read longer
-    // segments of each row.
-    template <class D, int NGY>
-    void ypass_launch(const PlanT<typename D::Real> &pl, const typename D::Real *in, typename D::Real *out, long long bs,
-                      int nbatch, Mult m) {
-        const dim3 grid((nx - 1 + 2 * NGY - 1) / (2 * NGY), nbatch);
-        const size_t sm = pass_smem<D>(pl.M, NGY, NGY);
-        if (sm > 48 * 1024) {
-            // one M per compile-time transform, so one size; the attribute is per device
-            static std::atomic<unsigned long long> attr_devices{0};
-            if (need_attr(attr_devices)) {
-                CK(cudaFuncSetAttribute(ypass_kernel<D, NGY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-                attr_devices.fetch_or(device_bit());
-            }
-        }
-        ypass_kernel<D, NGY><<<grid, NGY * D::TPF, sm, st>>>(in, out, bs, nx - 1, pl, m);
-    }
+    // Y pass of nbatch pitched scratch fields (nt elements apart), in place or not
     template <class R = T>
-    void ypass(const R *in, R *out, long long bs, int nbatch, Mult m) {
-        const PlanT<R> &pl = plan_y<R>();
+    void ypass(const R *in, R *out, int nbatch, const YSolve &m) {
         const int pe = prof_begin();
-        switch (pl.M) {
-            case 1024: ypass_t<Pow2Dst<1024, R>>(pl, in, out, bs, nbatch, m); break;
-            case 512: ypass_t<Pow2Dst<512, R>>(pl, in, out, bs, nbatch, m); break;
-            case 256: ypass_t<Pow2Dst<256, R>>(pl, in, out, bs, nbatch, m); break;
-            case 384: ypass_t<MixDst<384, R>>(pl, in, out, bs, nbatch, m); break;
-            default: ypass_t<GenericDst<R>>(pl, in, out, bs, nbatch, m); break;
-        }
+        ypass_launch<R>(ypass_ng<R>(ny, nbatch), in, out, nbatch, m);
         check_launch();
         prof_end(pe, IBPM_KCLASS_YPASS, 2.0 * sizeof(R) * (double)ng * nbatch);
     }
@@ -631,96 +581,41 @@ struct Engine final : ibpm_handle {
     const PlanT<R> &plan_y() const {
         if constexpr (std::is_same<R, T>::value) return ply; else return ply_d;
     }
-    double *psi1_hi = nullptr, *qs1_hi = nullptr, *t1_hi = nullptr, *t2_hi = nullptr;
-    // Merged trial solve over all L levels: Gamma_new = Ainv(A Gamma + rest)
-    // nb batches of ng (L for one case; cases x L for an ensemble group, whose
-    // per-batch coefficients dt / (2 Re hc^2) come from ctab)
-    // The merged trial solve on fields of element type R, with scratch t1_, t2_,
-    // rhs_ (nb fields each) and the plans of R: the first X pass and the Y pass
-    // each take the compile-time transform of their own length (nx and ny may
-    // differ), then the plain X pass.
-    template <class D, class R = typename D::Real>
-    void trial_xpart(const R *Gold, const R *rest_, int nb, R *t1_, R *t2_, const PlanT<R> &px) {
-        const dim3 grid((ny - 1 + kNG - 1) / kNG, nb);
-        const size_t sm = pass_smem<D>(px.M, kNG, kNG);
-        const int pe = prof_begin();
-        xpass_trial_kernel<D, kNG><<<grid, kNG * D::TPF, sm, st>>>(Gold, rest_, t1_, t2_, ng, nx - 1, px, ny - 1);
-        check_launch();
-        prof_end(pe, IBPM_KCLASS_XTRIAL, 4.0 * sizeof(R) * (double)ng * nb);
-    }
-    template <class D, int NG = kNG, class R = typename D::Real>
-    void trial_ypart(int nb, const double *ctab, R *t1_, R *t2_, R *rhs_, const PlanT<R> &py) {
-        // many fields per launch (ensemble groups) take 2 NG columns per block
-        if constexpr (NG == kNG) {
-            if (nb >= 16 && py.M <= 512) {
-                trial_ypart<D, 2 * kNG>(nb, ctab, t1_, t2_, rhs_, py);
-                return;
-            }
-        }
-        const dim3 grid((nx - 1 + 2 * NG - 1) / (2 * NG), nb);
-        const size_t sm = pass_smem<D>(py.M, 2 * NG, NG);
-        // the cap must cover the largest M this instantiation serves (kMaxM); the
-        // attribute is per device
-        static std::atomic<unsigned long long> attr_devices{0};
-        if (need_attr(attr_devices)) {
-            const int cap = (int)pass_smem<D>(kMaxM, 2 * NG, NG);
-            CK(cudaFuncSetAttribute(ypass_trial_kernel<D, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
-            attr_devices.fetch_or(device_bit());
-        }
-        const int pe = prof_begin();
-        Mult m = mult(MULT_AIMPL, 1, 1);
-        m.coef_tab = ctab;
-        ypass_trial_kernel<D, NG><<<grid, NG * D::TPF, sm, st>>>(t1_, t2_, rhs_, ng, nx - 1, py, m);
-        check_launch();
-        prof_end(pe, IBPM_KCLASS_YTRIAL, 3.0 * sizeof(R) * (double)ng * nb);
-    }
+    double *psi1_hi = nullptr, *qs1_hi = nullptr, *t1_hi = nullptr;
+    // The trial solve of get_trial_state (src/fluid.jl:485-496), Gamma_new =
+    // Ainv (A Gamma + dt (1.5 N1 - 0.5 N2) + rhsbc) of nb fields; the nonlinear
+    // kernel has formed the right-hand side (rest_)
     template <class R>
-    void trial_core(const R *Gold, const R *rest_, R *Gnew, int nb, const double *ctab, R *t1_, R *t2_, R *rhs_,
-                    const PlanT<R> &px, const PlanT<R> &py) {
-        switch (px.M) {
-            case 1024: trial_xpart<Pow2Dst<1024, R>>(Gold, rest_, nb, t1_, t2_, px); break;
-            case 512: trial_xpart<Pow2Dst<512, R>>(Gold, rest_, nb, t1_, t2_, px); break;
-            case 256: trial_xpart<Pow2Dst<256, R>>(Gold, rest_, nb, t1_, t2_, px); break;
-            case 384: trial_xpart<MixDst<384, R>>(Gold, rest_, nb, t1_, t2_, px); break;
-            default: trial_xpart<GenericDst<R>>(Gold, rest_, nb, t1_, t2_, px); break;
-        }
-        switch (py.M) {
-            case 1024: trial_ypart<Pow2Dst<1024, R>>(nb, ctab, t1_, t2_, rhs_, py); break;
-            case 512: trial_ypart<Pow2Dst<512, R>>(nb, ctab, t1_, t2_, rhs_, py); break;
-            case 256: trial_ypart<Pow2Dst<256, R>>(nb, ctab, t1_, t2_, rhs_, py); break;
-            case 384: trial_ypart<MixDst<384, R>>(nb, ctab, t1_, t2_, rhs_, py); break;
-            default: trial_ypart<GenericDst<R>>(nb, ctab, t1_, t2_, rhs_, py); break;
-        }
-        xpass<R>(InPlain<R>{rhs_, ng, nx - 1}, OutPlain<R>{Gnew, ng, nx - 1}, nb);
-    }
-    // the merged trial solve of one FP64 level (IBPM_MIXED_L1's level 1)
-    void trial_d(const double *Gold, const double *rest_, double *Gnew) {
-        trial_core<double>(Gold, rest_, Gnew, 1, nullptr, t1d, t2d, rhsd, plan_x<double>(), plan_y<double>());
-    }
-    // Merged trial solve over all L levels: Gamma_new = Ainv(A Gamma + rest)
-    // nb batches of ng (L for one case; cases x L for an ensemble group, whose
-    // per-batch coefficients dt / (2 Re hc^2) come from ctab)
-    void trial(const T *Gold, const T *rest_, T *Gnew, int nb = 0, const double *ctab = nullptr) {
-        if (nb == 0) nb = L;
-        trial_core<T>(Gold, rest_, Gnew, nb, ctab, t1, t2, rhs, plx, ply);
+    void trial(const R *rest_, R *Gnew, int nb, const YSolve &m, R *scratch) {
+        xpass<R>(InPlain<R>{rest_, ng, nx - 1}, OutPlain<R>{scratch, nt, ldt}, nb);
+        ypass<R>(scratch, scratch, nb, m);
+        xpass<R>(InPlain<R>{scratch, nt, ldt}, OutPlain<R>{Gnew, ng, nx - 1}, nb);
     }
 
-    Mult mult(int mode, int lev0, int levstep) const {
-        Mult m;
-        m.mode = mode;
-        m.cx = cx;
-        m.cy = cy;
-        m.scale = 1.0 / (double)(4 * (long long)nx * (long long)ny);
-        m.h = g.h;
-        m.Re = g.Re;
-        m.dt = g.dt;
-        m.lev0 = lev0;
-        m.levstep = levstep;
-        m.coef_tab = nullptr;
-        return m;
+    double coef(int lev) const {  // dt / (2 Re hc^2)
+        const double hc = ldexp(g.h, lev - 1);
+        return g.dt / (2 * g.Re * (hc * hc));
+    }
+    Mult mult(int mode, int lev) const {
+        return Mult{mode, cx, cy, 1.0 / (double)(4 * (long long)nx * (long long)ny), coef(lev)};
+    }
+    // tables of the y solves: the Laplacian inverse's, then the implicit
+    // diffusion's of levels 1..L
+    YCol *ycols = nullptr;
+    double *ydiff = nullptr;
+    double2 *yphase = nullptr;
+    // the y solve of batches at levels lev0, lev0 + levstep, ...
+    YSolve ysolve(int mode, int lev0, int levstep) const {
+        const long long k = mode == MULT_LAPINV ? 0 : lev0;
+        return YSolve{ycols + k * (nx - 1), ydiff + k * kYDiff, yphase, mode == MULT_LAPINV ? 0LL : (long long)levstep * (nx - 1),
+                      mode == MULT_LAPINV ? 0LL : (long long)levstep * kYDiff};
     }
     InPlain<T> in_plain(const T *p, long long bs) const { return InPlain<T>{p, bs, nx - 1}; }
     OutPlain<T> out_plain(T *p, long long bs) const { return OutPlain<T>{p, bs, nx - 1}; }
+    // the solves' scratch fields between the passes: rows ldt apart (a multiple of
+    // 32 bytes, so a block's columns start on a sector), fields nt apart
+    InPlain<T> in_scratch(const T *p) const { return InPlain<T>{p, nt, ldt}; }
+    OutPlain<T> out_scratch(T *p) const { return OutPlain<T>{p, nt, ldt}; }
 
     // The tensor-core transforms for nf fields of nprod products: creates (or
     // re-creates) the plan and the level-1 multiplier tables outside any capture.
@@ -749,7 +644,7 @@ struct Engine final : ibpm_handle {
             }
     }
     void tc_mult_table(int mode, int level, float *tab) {
-        tc_mult_kernel<<<dim3((nx + 127) / 128, nx), 128, 0, st>>>(mult(mode, level, 0), nx, tab);
+        tc_mult_kernel<<<dim3((nx + 127) / 128, nx), 128, 0, st>>>(mult(mode, level), nx, tab);
         check_launch();
     }
     // One batched solve x = S(m S(b)) on the tensor cores: b from the solve's
@@ -804,11 +699,11 @@ struct Engine final : ibpm_handle {
                 // batch strides ng and nq
                 const T *coarse = L > 1 ? psi_ + ng : nullptr;
                 if (coarse)
-                    xpass<double>(InBC<T>{Gl, coarse, bs, bs, g}, OutPlain<double>{t1_hi, ng, nx - 1}, nbatch);
+                    xpass<double>(InBC<T>{Gl, coarse, bs, bs, g}, OutPlain<double>{t1_hi, nt, ldt}, nbatch);
                 else
-                    xpass<double>(in_plain(Gl, bs), OutPlain<double>{t1_hi, ng, nx - 1}, nbatch);
-                ypass<double>(t1_hi, t2_hi, ng, nbatch, mult(MULT_LAPINV, 1, 0));
-                xpass<double>(InPlain<double>{t2_hi, ng, nx - 1}, OutPlain<double>{psi1_hi, ng, nx - 1}, nbatch);
+                    xpass<double>(in_plain(Gl, bs), OutPlain<double>{t1_hi, nt, ldt}, nbatch);
+                ypass<double>(t1_hi, t1_hi, nbatch, ysolve(MULT_LAPINV, 1, 0));
+                xpass<double>(InPlain<double>{t1_hi, nt, ldt}, OutPlain<double>{psi1_hi, ng, nx - 1}, nbatch);
                 const dim3 blk(64, 4);
                 const dim3 grd((nx + 1 + 63) / 64, (ny + 1 + 3) / 4, nbatch);
                 curl_kernel<double, double, T><<<grd, blk, 0, st>>>(qs1_hi, nq, psi1_hi, ng, coarse, bs, g);
@@ -843,16 +738,16 @@ struct Engine final : ibpm_handle {
                 if constexpr (std::is_same<T, double>::value) cen = central && lev >= 2;
                 if (lev == L) {
                     if constexpr (std::is_same<T, double>::value)
-                        if (cen) xpass(centred(in_plain(Gl, bs)), out_plain(t1, ng), nbatch);
-                    if (!cen) xpass(in_plain(Gl, bs), out_plain(t1, ng), nbatch);
+                        if (cen) xpass(centred(in_plain(Gl, bs)), out_scratch(t1), nbatch);
+                    if (!cen) xpass(in_plain(Gl, bs), out_scratch(t1), nbatch);
                 } else {
                     const InBC<T> in{Gl, psi_ + lev * ng, bs, bs, g};
                     if constexpr (std::is_same<T, double>::value)
-                        if (cen) xpass(centred(in), out_plain(t1, ng), nbatch);
-                    if (!cen) xpass(in, out_plain(t1, ng), nbatch);
+                        if (cen) xpass(centred(in), out_scratch(t1), nbatch);
+                    if (!cen) xpass(in, out_scratch(t1), nbatch);
                 }
-                ypass(t1, t2, ng, nbatch, mult(MULT_LAPINV, 1, 0));
-                xpass(in_plain(t2, ng), out_plain(Pl, bs), nbatch, lev == 1 ? win : nullptr);
+                ypass(t1, t1, nbatch, ysolve(MULT_LAPINV, 1, 0));
+                xpass(in_scratch(t1), out_plain(Pl, bs), nbatch, lev == 1 ? win : nullptr);
             }
             if (curl_all || lev == 1) {
                 const dim3 blk(64, 4);
@@ -889,12 +784,12 @@ struct Engine final : ibpm_handle {
             }
         }
         if (!solved) {
-            xpass(in, out_plain(t1, ng), nbatch, P.bbox, 1);  // rot of the patch: zero outside its rows
-            ypass(t1, t2, ng, nbatch, mult(MULT_AIMPL, 1, 0));
+            xpass(in, out_scratch(t1), nbatch, P.bbox, 1);  // rot of the patch: zero outside its rows
+            ypass(t1, t1, nbatch, ysolve(MULT_AIMPL, 1, 0));
             // Gw's levels 2..L hold the level-1 vorticity coarsified and zeros elsewhere:
             // vort2flux's coarsify rewrites their central block, and nothing else ever
             // writes them, so the zeros of the allocation stay
-            xpass(in_plain(t2, ng), out_plain(Gw, ng * L), nbatch);
+            xpass(in_scratch(t1), out_plain(Gw, ng * L), nbatch);
         }
         // E reads the bbox only; Gw's coarse levels are zero outside coarsify!'s block
         vort2flux(psiw, qw, Gw, ng * L, nq, nbatch, false, false, P.bbox, true);
@@ -948,8 +843,8 @@ struct Engine final : ibpm_handle {
     // psi1, nl1 and FP64 scratch); the float arrays hold levels 2..L
     bool l1d = false;
     double *G1[2] = {nullptr, nullptr}, *nl1[2] = {nullptr, nullptr};
-    double *q1 = nullptr, *psi1 = nullptr, *rest1 = nullptr, *t1d = nullptr, *t2d = nullptr, *rhsd = nullptr;
-    double *patch_d = nullptr, *q0d = nullptr, *coef_coarse = nullptr;
+    double *q1 = nullptr, *psi1 = nullptr, *rest1 = nullptr, *t1d = nullptr;
+    double *patch_d = nullptr, *q0d = nullptr;
     void step_body_l1d();
     void vort2flux_l1d(const double *G1v, T *Gm, T *qout, double *psi1_out, double *q1_out, bool curl_all);
     ibpm_problem problem_copy{};
@@ -1043,6 +938,19 @@ void Engine<T>::setup() {
     };
     tables(nx, twx, snx, cx, plx);
     tables(ny, twy, sny, cy, ply);
+    {
+        std::vector<double> hc(L);
+        for (int lev = 1; lev <= L; ++lev) hc[lev - 1] = coef(lev);
+        double *cd = dalloc<double>(L);
+        ycols = dalloc<YCol>((size_t)(nx - 1) * (L + 1));
+        ydiff = dalloc<double>((size_t)kYDiff * (L + 1));
+        yphase = dalloc<double2>((kYChunks + 1) * kYFull);
+        CK(cudaMemcpyAsync(cd, hc.data(), sizeof(double) * L, cudaMemcpyHostToDevice, st));
+        CK(launch_ycols(ycols, ydiff, yphase, cx, cy, nx, ny, nullptr, 1, st));
+        CK(launch_ycols(ycols + (nx - 1), ydiff + kYDiff, yphase, cx, cy, nx, ny, cd, L, st));
+        CK(cudaStreamSynchronize(st));
+        dfree(cd);
+    }
     if (!std::is_same<T, double>::value) {
         hi_level1 = true;
         if (const char *e = getenv("IBPM_FP32_LEVEL1")) hi_level1 = e[0] != '0';
@@ -1068,8 +976,7 @@ void Engine<T>::setup() {
         dtables(ny, ply_d);
         psi1_hi = dalloc<double>(ng);
         qs1_hi = dalloc<double>(nq);
-        t1_hi = dalloc<double>(ng);
-        t2_hi = dalloc<double>(ng);
+        t1_hi = dalloc<double>(nt);
         l1d = opt.precision == IBPM_MIXED_L1;
         if (l1d) {
             if (!static_bodies)
@@ -1081,19 +988,9 @@ void Engine<T>::setup() {
             q1 = dalloc<double>(nq);
             psi1 = dalloc<double>(ng);
             rest1 = dalloc<double>(ng);
-            t1d = dalloc<double>(ng);
-            t2d = dalloc<double>(ng);
-            rhsd = dalloc<double>(ng);
+            t1d = dalloc<double>(nt);
             q0d = dalloc<double>(nq);
             patch_d = dalloc<double>(2LL * (nx + 1) * (ny + 1));
-            // dt / (2 Re hc^2) of levels 2..L, as Mult::coef forms it on the device
-            std::vector<double> cc(std::max(L - 1, 1), 0.0);
-            for (int lev = 2; lev <= L; ++lev) {
-                const double hc = ldexp(g.h, lev - 1);
-                cc[lev - 2] = g.dt / (2 * g.Re * (hc * hc));
-            }
-            coef_coarse = dalloc<double>(cc.size());
-            CK(cudaMemcpyAsync(coef_coarse, cc.data(), sizeof(double) * cc.size(), cudaMemcpyHostToDevice, st));
         }
     }
 
@@ -1136,9 +1033,8 @@ void Engine<T>::setup() {
     if (!static_bodies) kbatch = 2;  // the warm start applies B to two vectors at once
     kbatch = std::min(kbatch, 2 * np);
     const int kb = std::max(kbatch, L);
-    t1 = dalloc<T>(ng * kb);
-    t2 = dalloc<T>(ng * kb);
-    rhs = dalloc<T>(ng * L);
+    t1 = dalloc<T>(nt * kb);
+    rhs = dalloc<T>(nt);
     rest = dalloc<T>(ng * L);
     qs1 = dalloc<T>(nq);
     Ftmp = dalloc<double>(2 * np);
@@ -1187,13 +1083,13 @@ void Engine<T>::setup() {
     for (int b = 0; b < nbody; ++b)
         if (body_kind[b] == IBPM_BODY_STATIC) update_weights(body_start[b], body_start[b + 1]);
     check_region_error();
-    // pass shapes for one level and for all levels at once (scratch t1 -> t2)
-    tune_ypass<T>(t1, t2, 1);
-    if (L > 1) tune_ypass<T>(t1, t2, L);
+    // pass shapes for one level and for all levels at once
+    tune_ypass<T>(t1, t1, 1);
+    if (L > 1) tune_ypass<T>(t1, t1, L);
     if (static_bodies) {
         compute_bbox();
         if (std::is_same<T, double>::value) {
-            if (kbatch > L) tune_ypass<T>(Gw, psiw, kbatch);
+            if (kbatch > L) tune_ypass<T>(t1, t1, kbatch);
             build_Binv();
             shrink_batch_buffers();
         } else {
@@ -1697,7 +1593,7 @@ void Engine<T>::step_body() {
         check_launch();
         prof_end(pe, IBPM_KCLASS_NONLINEAR, 8.0 * (double)(nq + 4 * ng) * L);
     }
-    trial(Gold, rest, Gnew);
+    trial<T>(rest, Gnew, L, ysolve(MULT_AIMPL, 1, 1), t1);
     nc = 1 - nc;  // _cycle!(state.nonlin)
     // couple_surface_rigid (src/coupling.jl:236-250).  The FP32 engine computes the
     // level-1 trial flux that E interpolates in FP64: B^-1 amplifies white noise in
@@ -1801,9 +1697,9 @@ void Engine<T>::step_body() {
     }
     // project_circ (src/coupling.jl:218-230): Gamma = Gamma_s; Gamma_1 -= Ainv_1 rot(E^T F~b)
     reg_patch(Fbt, 1);
-    xpass(InRegRot<T>{Patch<T>{patch, P.bbox, patch_stride}}, out_plain(t1, ng), 1, P.bbox, 1);
-    ypass(t1, t2, ng, 1, mult(MULT_AIMPL, 1, 0));
-    xpass(in_plain(t2, ng), OutSub<T>{Gnew, ng, nx - 1}, 1);
+    xpass(InRegRot<T>{Patch<T>{patch, P.bbox, patch_stride}}, out_scratch(t1), 1, P.bbox, 1);
+    ypass(t1, t1, 1, ysolve(MULT_AIMPL, 1, 0));
+    xpass(in_scratch(t1), OutSub<T>{Gnew, ng, nx - 1}, 1);
     // vort2flux!(state.psi, state.q, state.Gamma)
     vort2flux(psi, q, Gnew, 0, 0, 1, true);
     gc = 1 - gc;
@@ -1838,8 +1734,8 @@ void Engine<T>::step_body_l1d() {
         nonlinear_kernel<T, T, true><<<grd, blk, 0, st>>>(a);
         check_launch();
     }
-    trial_d(G1o, rest1, G1n);
-    if (L > 1) trial(Gold + ng, rest + ng, Gnew + ng, L - 1, coef_coarse);
+    trial<double>(rest1, G1n, 1, ysolve(MULT_AIMPL, 1, 0), t1d);
+    if (L > 1) trial<T>(rest + ng, Gnew + ng, L - 1, ysolve(MULT_AIMPL, 2, 1), t1);
     nc = 1 - nc;  // _cycle!(state.nonlin)
     // couple_surface_rigid from the FP64 level-1 trial flux
     vort2flux_l1d(G1n, Gnew, nullptr, psi1_hi, qs1_hi, false);
@@ -1854,10 +1750,10 @@ void Engine<T>::step_body_l1d() {
     // project_circ (src/coupling.jl:218-230) on the FP64 level 1
     launch_reg_patch<double>(P, Fbt, 2 * np, patch_d, patch_stride, 1, g, st);
     check_launch();
-    xpass<double>(InRegRot<double>{Patch<double>{patch_d, P.bbox, patch_stride}}, OutPlain<double>{t1d, ng, nx - 1}, 1,
+    xpass<double>(InRegRot<double>{Patch<double>{patch_d, P.bbox, patch_stride}}, OutPlain<double>{t1d, nt, ldt}, 1,
                   P.bbox, 1);
-    ypass<double>(t1d, t2d, ng, 1, mult(MULT_AIMPL, 1, 0));
-    xpass<double>(InPlain<double>{t2d, ng, nx - 1}, OutSub<double>{G1n, ng, nx - 1}, 1);
+    ypass<double>(t1d, t1d, 1, ysolve(MULT_AIMPL, 1, 0));
+    xpass<double>(InPlain<double>{t1d, nt, ldt}, OutSub<double>{G1n, ng, nx - 1}, 1);
     // vort2flux!(state.psi, state.q, state.Gamma)
     vort2flux_l1d(G1n, Gnew, q, psi1, q1, true);
     gc = 1 - gc;
@@ -1883,11 +1779,11 @@ void Engine<T>::vort2flux_l1d(const double *G1v, T *Gm, T *qout, double *psi1_ou
     for (int lev = L; lev >= 2; --lev) {
         T *Gl = Gm + (lev - 1) * ng, *Pl = psi + (lev - 1) * ng;
         if (lev == L)
-            xpass(in_plain(Gl, 0), out_plain(t1, ng), 1);
+            xpass(in_plain(Gl, 0), out_scratch(t1), 1);
         else
-            xpass(InBC<T>{Gl, psi + lev * ng, 0, 0, g}, out_plain(t1, ng), 1);
-        ypass(t1, t2, ng, 1, mult(MULT_LAPINV, 1, 0));
-        xpass(in_plain(t2, ng), out_plain(Pl, 0), 1);
+            xpass(InBC<T>{Gl, psi + lev * ng, 0, 0, g}, out_scratch(t1), 1);
+        ypass(t1, t1, 1, ysolve(MULT_LAPINV, 1, 0));
+        xpass(in_scratch(t1), out_plain(Pl, 0), 1);
         if (curl_all) {
             curl_kernel<T, T, T><<<qgrd, qblk, 0, st>>>(qout + (lev - 1) * nq, 0, Pl, 0,
                                                         lev < L ? psi + lev * ng : nullptr, 0, g);
@@ -1896,11 +1792,11 @@ void Engine<T>::vort2flux_l1d(const double *G1v, T *Gm, T *qout, double *psi1_ou
     }
     const T *coarse = L > 1 ? psi + ng : nullptr;
     if (coarse)
-        xpass<double>(InBC<double, T>{G1v, coarse, 0, 0, g}, OutPlain<double>{t1d, ng, nx - 1}, 1);
+        xpass<double>(InBC<double, T>{G1v, coarse, 0, 0, g}, OutPlain<double>{t1d, nt, ldt}, 1);
     else
-        xpass<double>(InPlain<double>{G1v, 0, nx - 1}, OutPlain<double>{t1d, ng, nx - 1}, 1);
-    ypass<double>(t1d, t2d, ng, 1, mult(MULT_LAPINV, 1, 0));
-    xpass<double>(InPlain<double>{t2d, ng, nx - 1}, OutPlain<double>{psi1_out, ng, nx - 1}, 1);
+        xpass<double>(InPlain<double>{G1v, 0, nx - 1}, OutPlain<double>{t1d, nt, ldt}, 1);
+    ypass<double>(t1d, t1d, 1, ysolve(MULT_LAPINV, 1, 0));
+    xpass<double>(InPlain<double>{t1d, nt, ldt}, OutPlain<double>{psi1_out, ng, nx - 1}, 1);
     curl_kernel<double, double, T><<<qgrd, qblk, 0, st>>>(q1_out, 0, psi1_out, 0, coarse, 0, g);
     check_launch();
 }
@@ -1995,6 +1891,8 @@ void Engine<T>::init(const ibpm_problem *p, const ibpm_options &o) {
     nq = nu + (long long)p->nx * (p->ny + 1);
     ng = (long long)(p->nx - 1) * (p->ny - 1);
     nbc = 2LL * (p->nx + 1) + 2LL * (p->ny + 1);
+    ldt = (p->nx + 3) / 4 * 4;
+    nt = (long long)ldt * (p->ny - 1);
     g = Grid{p->nx, p->ny, p->nlevel, p->h, p->x0, p->y0, p->Re, p->dt, p->grid_moving ? 1 : 0};
     body_kind.assign(p->body_kind, p->body_kind + p->nbody);
     body_start.assign(p->body_start, p->body_start + p->nbody + 1);
@@ -2348,10 +2246,17 @@ void Engine<T>::diag_solve(int op, int level, const double *b, double *x) {
         }
     }
     upload(rhs, b, (size_t)ng);
-    xpass(in_plain(rhs, ng), out_plain(t1, ng), 1);
-    ypass(t1, t2, ng, 1, mult(mode, level, 0));
-    xpass(in_plain(t2, ng), out_plain(rhs, ng), 1);
-    download(x, rhs, (size_t)ng);
+    xpass(in_plain(rhs, ng), out_scratch(t1), 1);
+    // the explicit stencil is not in place
+    T *y = mode == MULT_AEXPL ? rhs : t1, *sol = mode == MULT_AEXPL ? t1 : rhs;
+    if (mode == MULT_AEXPL) {
+        yexpl_kernel<T><<<dim3((nx + 30) / 32, (ny + 6) / 8), dim3(32, 8), 0, st>>>(t1, y, ldt, nx, ny, coef(level), cx);
+        check_launch();
+    } else {
+        ypass(t1, y, 1, ysolve(mode, level, 0));
+    }
+    xpass(in_scratch(y), out_plain(sol, ng), 1);
+    download(x, sol, (size_t)ng);
     CK(cudaStreamSynchronize(st));
 }
 
@@ -2438,9 +2343,16 @@ struct CaseGroup {
     int device = 0;
     cudaStream_t st = nullptr;
     T *q = nullptr, *psi = nullptr, *G[2] = {nullptr, nullptr}, *nl[2] = {nullptr, nullptr};
-    T *t1 = nullptr, *t2 = nullptr, *rhs = nullptr, *rest = nullptr, *qs1 = nullptr;
-    double *t1_hi = nullptr, *t2_hi = nullptr, *psi1_hi = nullptr, *qs1_hi = nullptr;
-    double *coef_all = nullptr, *coef_lev1 = nullptr, *re_tab = nullptr;
+    T *t1 = nullptr, *rest = nullptr, *qs1 = nullptr;
+    double *t1_hi = nullptr, *psi1_hi = nullptr, *qs1_hi = nullptr;
+    double *re_tab = nullptr;
+    // the implicit diffusion's y-solve tables, case-major (batch b = case L + level - 1)
+    YCol *ycols = nullptr;
+    double *ydiff = nullptr;
+    // the y solve of every step-th batch: 1 all levels of all cases, L level 1 of every case
+    YSolve ysolve(int step) const {
+        return YSolve{ycols, ydiff, e0->yphase, (long long)step * (e0->nx - 1), (long long)step * kYDiff};
+    }
     StepDev *prm_tab = nullptr;
     CaseView *views = nullptr;  // each case's panels and force-solve buffers (device)
     int *bbox_tab = nullptr;    // each case's face window, 4 ints per case (device)
@@ -2496,35 +2408,28 @@ struct CaseGroup {
         G[1] = alloc<T>(ngL * C);
         nl[0] = alloc<T>(ngL * C);
         nl[1] = alloc<T>(ngL * C);
-        t1 = alloc<T>(ngL * C);
-        t2 = alloc<T>(ngL * C);
-        rhs = alloc<T>(ngL * C);
+        t1 = alloc<T>((size_t)(e0->nt * L) * C);
         rest = alloc<T>(ngL * C);
         qs1 = alloc<T>((size_t)nq * C);
         if (e0->hi_level1) {
-            t1_hi = alloc<double>((size_t)ng * C);
-            t2_hi = alloc<double>((size_t)ng * C);
+            t1_hi = alloc<double>((size_t)e0->nt * C);
             psi1_hi = alloc<double>((size_t)ng * C);
             qs1_hi = alloc<double>((size_t)nq * C);
         }
         prm_tab = alloc<StepDev>(C);
-        // dt / (2 Re hc^2) per (case, level), as Mult::coef forms it on the device
-        std::vector<double> ca((size_t)C * L), c1(C), re(C);
+        // dt / (2 Re hc^2) per (case, level)
+        std::vector<double> ca((size_t)C * L), re(C);
         for (int c = 0; c < C; ++c) {
-            const Grid &g = cs[c]->g;
-            re[c] = g.Re;
-            for (int lev = 1; lev <= L; ++lev) {
-                const double hc = ldexp(g.h, lev - 1);
-                ca[(size_t)c * L + lev - 1] = g.dt / (2 * g.Re * (hc * hc));
-            }
-            c1[c] = ca[(size_t)c * L];
+            re[c] = cs[c]->g.Re;
+            for (int lev = 1; lev <= L; ++lev) ca[(size_t)c * L + lev - 1] = cs[c]->coef(lev);
         }
-        coef_all = alloc<double>(ca.size());
-        coef_lev1 = alloc<double>(C);
+        double *coef_all = alloc<double>(ca.size());
         re_tab = alloc<double>(C);
+        ycols = alloc<YCol>((size_t)(e0->nx - 1) * C * L);
+        ydiff = alloc<double>((size_t)kYDiff * C * L);
         CK(cudaMemcpyAsync(coef_all, ca.data(), sizeof(double) * ca.size(), cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(coef_lev1, c1.data(), sizeof(double) * C, cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(re_tab, re.data(), sizeof(double) * C, cudaMemcpyHostToDevice, st));
+        CK(launch_ycols(ycols, ydiff, e0->yphase, e0->cx, e0->cy, e0->nx, e0->ny, coef_all, C * L, st));
         std::vector<CaseView> hv(C);
         views = alloc<CaseView>(C);
         bbox_tab = alloc<int>(4 * (size_t)C);
@@ -2537,7 +2442,7 @@ struct CaseGroup {
         }
         CK(cudaMemcpyAsync(views, hv.data(), sizeof(CaseView) * C, cudaMemcpyHostToDevice, st));
         CK(cudaStreamSynchronize(st));
-        e0->template tune_ypass<T>(t1, t2, C);  // the group's Y passes cover C fields
+        e0->template tune_ypass<T>(t1, t1, C);  // the group's Y passes cover C fields
         // move every case's state into its slot and point the case there
         for (int c = 0; c < C; ++c) {
             Engine<T> &e = *cs[c];
@@ -2628,33 +2533,24 @@ struct CaseGroup {
     struct Borrow {
         Engine<T> &e;
         cudaStream_t st;
-        T *t1, *t2, *rhs;
-        double *t1_hi, *t2_hi, *psi1_hi, *qs1_hi;
+        T *t1;
+        double *t1_hi, *psi1_hi, *qs1_hi;
         Borrow(Engine<T> &e_, CaseGroup &gr) : e(e_) {
             st = e.st;
             t1 = e.t1;
-            t2 = e.t2;
-            rhs = e.rhs;
             t1_hi = e.t1_hi;
-            t2_hi = e.t2_hi;
             psi1_hi = e.psi1_hi;
             qs1_hi = e.qs1_hi;
             e.st = gr.st;
             e.t1 = gr.t1;
-            e.t2 = gr.t2;
-            e.rhs = gr.rhs;
             e.t1_hi = gr.t1_hi;
-            e.t2_hi = gr.t2_hi;
             e.psi1_hi = gr.psi1_hi;
             e.qs1_hi = gr.qs1_hi;
         }
         ~Borrow() {
             e.st = st;
             e.t1 = t1;
-            e.t2 = t2;
-            e.rhs = rhs;
             e.t1_hi = t1_hi;
-            e.t2_hi = t2_hi;
             e.psi1_hi = psi1_hi;
             e.qs1_hi = qs1_hi;
         }
@@ -2674,7 +2570,7 @@ struct CaseGroup {
             nonlinear_kernel<T, T, true><<<grd, blk, 0, st>>>(a);
             e.check_launch();
         }
-        e.trial(Gold, rest, Gnew, C * L, coef_all);
+        e.template trial<T>(rest, Gnew, C * L, ysolve(1), t1);
         nc = 1 - nc;
         e.vort2flux(psi, e.hi_level1 ? nullptr : qs1, Gnew, bsG, nq, C, false, e.hi_level1, nullptr);
         // per case, one launch over all cases each: E qs, F~b = B^-1 Ftmp,
@@ -2691,12 +2587,10 @@ struct CaseGroup {
         e.check_launch();
         launch_reg_patch_multi<T>(views, C, e.g, st);
         e.check_launch();
-        e.xpass(InRegRotTab<T>{views}, e.out_plain(t1, ng), C, bbox_tab, 1, 4);
+        e.xpass(InRegRotTab<T>{views}, e.out_scratch(t1), C, bbox_tab, 1, 4);
         // project_circ's solve at level 1 of every case, then vort2flux!
-        Mult m = e.mult(MULT_AIMPL, 1, 0);
-        m.coef_tab = coef_lev1;
-        e.ypass(t1, t2, ng, C, m);
-        e.xpass(e.in_plain(t2, ng), OutSub<T>{Gnew, bsG, e.nx - 1}, C);
+        e.ypass(t1, t1, C, ysolve(L));
+        e.xpass(e.in_scratch(t1), OutSub<T>{Gnew, bsG, e.nx - 1}, C);
         e.vort2flux(psi, q, Gnew, bsG, bsQ, C, true);
         gc = 1 - gc;
     }

@@ -6,6 +6,7 @@
 #include <type_traits>
 #include "common.cuh"
 #include "fft_pow2.cuh"
+#include "ytri.cuh"
 
 namespace ibpm {
 
@@ -138,47 +139,6 @@ struct OutSub {
     }
 };
 
-// 1/d: the hardware reciprocal approximation refined by two Newton-Raphson
-// steps (e = 1 - d y, y += y e); within an ulp or two of the correctly rounded
-// quotient, for the positive, normal d of the spectral multipliers.
-__device__ __forceinline__ double recip(double d) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    double e = fma(-d, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-d, y, 1.0);
-    return fma(y, e, y);
-}
-
-// Spectral multipliers scale / Lambda (src/fluid.jl:117-134)
-enum { MULT_LAPINV = 0, MULT_AEXPL = 1, MULT_AIMPL = 2 };
-struct Mult {
-    int mode;
-    const double *cx;   // cos(pi i / nx), i = 0..nx
-    const double *cy;   // cos(pi j / ny), j = 0..ny
-    double scale;       // 1 / (4 nx ny)
-    double h, Re, dt;
-    int lev0, levstep;  // level of batch b: lev0 + b * levstep
-    const double *coef_tab;  // device, may be null: c of batch b (cases of an ensemble differ in Re)
-    // c = dt / (2 Re hc^2) of the batch's level; the reference's (lam dt) / (2 Re hc^2)
-    // becomes lam c (within one rounding), which leaves one division per element.
-    __device__ __forceinline__ double coef(int b) const {
-        if (coef_tab) return coef_tab[b];
-        const int lev = lev0 + b * levstep;
-        const double hc = ldexp(h, lev - 1);
-        return dt / (2 * Re * (hc * hc));
-    }
-    __device__ __forceinline__ double eval(double c, double cxi, double cyj) const {
-        const double lam = -2 * ((cxi + cyj) - 2);
-        if (mode == MULT_LAPINV) return scale * recip(lam);
-        if (mode == MULT_AEXPL) return scale * (1 - lam * c);  // scale / (1 / (1 - lam c))
-        return scale * recip(1 + lam * c);
-    }
-    __device__ __forceinline__ double operator()(double c, int i, int j) const {
-        return eval(c, __ldg(&cx[i]), __ldg(&cy[j]));
-    }
-};
-
 // X pass: DST along x of rows (ja, jb) = (2p+1, 2p+2) of each batch field.
 // D is the line transform (Pow2Dst<M> or GenericDst); NG line pairs per block.
 // rows (device, may be null): the body's face window i0, i1, j0, j1 (batch b's
@@ -274,287 +234,6 @@ __global__ void __launch_bounds__(D::TPF *NG, D::OCC / (D::TPF * NG))
     }
 }
 
-// Y pass: for each column i, x[i, :] = DST_y(mult(i, :) * DST_y(in[i, :])).
-// A block owns 2*NG adjacent columns; loads and stores are row-coalesced.
-template <class D, int NG>
-__global__ void __launch_bounds__(D::TPF *NG, D::OCC / (D::TPF * NG))
-    ypass_kernel(const typename D::Real *__restrict__ in, typename D::Real *__restrict__ out, long long bs, int ncols,
-                 PlanT<typename D::Real> pl, Mult mult) {
-    using T = typename D::Real;
-    using C = typename D::C;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *smem = reinterpret_cast<C *>(smem_raw);
-    constexpr int TPF = D::TPF;
-    const int M = pl.M;
-    const int G = D::smem_len(M);
-    const int g = threadIdx.x / TPF, t = threadIdx.x % TPF;
-    C *buf = smem + g * G;
-    double2 *wt = reinterpret_cast<double2 *>(smem_raw + scratch_offset<D>(M, NG)) + D::NWARP * g;
-    const int b = blockIdx.y;
-    const int c0 = blockIdx.x * 2 * NG;  // 0-based first column of the block
-    const T *src = in + b * bs;
-    T *dst = out + b * bs;
-    constexpr int W = 2 * NG;
-    if constexpr (D::MC > 0) {
-        // compile-time trip count, loads issued in chunks of CH before their stores
-        constexpr int NT = NG * TPF;
-        constexpr int NIT = (W * (D::MC + 1) + NT - 1) / NT;
-        constexpr int CH = 12;
-#pragma unroll
-        for (int k0 = 0; k0 < NIT; k0 += CH) {
-            T v[CH];
-#pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const int e = threadIdx.x + (k0 + k) * NT;
-                const int c = e % W, jj = e / W;
-                const int col = c0 + c;
-                v[k] = (k0 + k < NIT && jj >= 1 && jj < D::MC && col < ncols) ? src[col + (long long)ncols * (jj - 1)]
-                                                                               : (T)0;
-            }
-#pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const int e = threadIdx.x + (k0 + k) * NT;
-                const int c = e % W, jj = e / W;
-                if (k0 + k < NIT && jj <= D::MC) *(reinterpret_cast<T *>(smem + (c >> 1) * G + D::idx(jj)) + (c & 1)) = v[k];
-            }
-        }
-    } else {
-        for (int e = threadIdx.x; e < W * (M + 1); e += blockDim.x) {
-            const int c = e % W, jj = e / W;
-            const int col = c0 + c;
-            T v = 0;
-            if (jj >= 1 && jj < M && col < ncols) v = src[col + (long long)ncols * (jj - 1)];
-            T *slot = reinterpret_cast<T *>(smem + (c >> 1) * G + D::idx(jj)) + (c & 1);
-            *slot = v;
-        }
-    }
-    __syncthreads();
-    // DST, spectral multiply, DST; one loop body so the transform is emitted once
-#pragma unroll 1
-    for (int pass = 0; pass < 2; ++pass) {
-        D::dst(buf, pl, t, wt);
-        if (pass == 1) break;
-        const int ia = c0 + 2 * g + 1, ib = c0 + 2 * g + 2;  // 1-based columns
-        const double cb = mult.coef(b);
-        if constexpr (D::MC > 0) {
-            constexpr int NIT = (D::MC - 1 + TPF - 1) / TPF;
-            const double cxa = ia <= ncols ? __ldg(&mult.cx[ia]) : 0.0, cxb = ib <= ncols ? __ldg(&mult.cx[ib]) : 0.0;
-            double cyv[NIT];
-#pragma unroll
-            for (int k = 0; k < NIT; ++k) {
-                const int jj = 1 + t + k * TPF;
-                cyv[k] = jj < D::MC ? __ldg(&mult.cy[jj]) : 0.0;
-            }
-#pragma unroll
-            for (int k = 0; k < NIT; ++k) {
-                const int jj = 1 + t + k * TPF;
-                if (jj >= D::MC) break;
-                C y = buf[D::idx(jj)];
-                y.x = (T)(y.x * ((ia <= ncols) ? mult.eval(cb, cxa, cyv[k]) : 0.0));
-                y.y = (T)(y.y * ((ib <= ncols) ? mult.eval(cb, cxb, cyv[k]) : 0.0));
-                buf[D::idx(jj)] = y;
-            }
-        } else {
-            for (int jj = 1 + t; jj < M; jj += TPF) {
-                C y = buf[D::idx(jj)];
-                y.x = (T)(y.x * ((ia <= ncols) ? mult(cb, ia, jj) : 0.0));
-                y.y = (T)(y.y * ((ib <= ncols) ? mult(cb, ib, jj) : 0.0));
-                buf[D::idx(jj)] = y;
-            }
-        }
-        __syncthreads();
-    }
-    for (int e = threadIdx.x; e < W * (M + 1); e += blockDim.x) {
-        const int c = e % W, jj = e / W;
-        const int col = c0 + c;
-        if (jj >= 1 && jj < M && col < ncols) {
-            const T *slot = reinterpret_cast<const T *>(smem + (c >> 1) * G + D::idx(jj)) + (c & 1);
-            dst[col + (long long)ncols * (jj - 1)] = *slot;
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Merged trial solve of get_trial_state (src/fluid.jl:485-496):
-//   Gamma_s = Ainv (A Gamma + rest),  rest = dt (1.5 N1 - 0.5 N2) + rhsbc.
-// With S the 2D DST-I and S S = 1/scale:  S(A Gamma) = S(Gamma) / Lambda_e, so
-//   Gamma_s = S( scale / Lambda_i * ( S(Gamma) / Lambda_e + S(rest) ) ),
-// three passes instead of the reference's four transforms in six passes.
-// ---------------------------------------------------------------------------
-
-// X pass: row j of level b as one complex line z = Gamma + i rest.
-template <class D, int NG>
-__global__ void __launch_bounds__(D::TPF *NG, D::OCC / (D::TPF * NG))
-    xpass_trial_kernel(const typename D::Real *__restrict__ gam, const typename D::Real *__restrict__ rest,
-                       typename D::Real *__restrict__ t1, typename D::Real *__restrict__ t2, long long bs, int ld,
-                       PlanT<typename D::Real> pl, int nrows) {
-    using T = typename D::Real;
-    using C = typename D::C;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *smem = reinterpret_cast<C *>(smem_raw);
-    constexpr int TPF = D::TPF;
-    const int M = pl.M;
-    const int G = D::smem_len(M);
-    const int g = threadIdx.x / TPF, t = threadIdx.x % TPF;
-    C *buf = smem + g * G;
-    double2 *wt = reinterpret_cast<double2 *>(smem_raw + scratch_offset<D>(M, NG)) + D::NWARP * g;
-    const int b = blockIdx.y;
-    const int j = blockIdx.x * NG + g + 1;
-    const bool valid = j <= nrows;
-    const long long row = b * bs + (long long)ld * (j - 1);
-    if constexpr (D::MC > 0) {
-        constexpr int NIT = (D::MC + 1 + TPF - 1) / TPF;
-        T za[NIT], zb[NIT];
-#pragma unroll
-        for (int k = 0; k < NIT; ++k) {
-            const int i = t + k * TPF;
-            const bool ok = valid && i >= 1 && i < D::MC;
-            za[k] = ok ? gam[row + i - 1] : (T)0;
-            zb[k] = ok ? rest[row + i - 1] : (T)0;
-        }
-#pragma unroll
-        for (int k = 0; k < NIT; ++k) {
-            const int i = t + k * TPF;
-            if (i <= D::MC) buf[D::idx(i)] = Cx<T>::make(za[k], zb[k]);
-        }
-    } else {
-        for (int i = t; i <= M; i += TPF) {
-            C z = Cx<T>::make(0, 0);
-            if (valid && i >= 1 && i < M) z = Cx<T>::make(gam[row + i - 1], rest[row + i - 1]);
-            buf[D::idx(i)] = z;
-        }
-    }
-    __syncthreads();
-    D::dst(buf, pl, t, wt);
-    if (valid)
-        for (int i = 1 + t; i < M; i += TPF) {
-            const C y = buf[D::idx(i)];
-            t1[row + i - 1] = y.x;
-            t2[row + i - 1] = y.y;
-        }
-}
-
-// Y pass: a block owns 2NG adjacent columns.  Phase 1 transforms each column's
-// (S_x Gamma, S_x rest) pair as one complex line and combines
-//   v = scale / Lambda_i * (S Gamma / Lambda_e + S rest)
-//     = (S Gamma (1 - lam c) + S rest) * scale / (1 + lam c),   c = dt / (2 Re hc^2);
-// phase 2 transforms the real v of two columns packed as one complex line.
-// Resident threads per SM the kernel is compiled for: 512 for FP32 lines of up to
-// 512 points (at most 128 registers a thread), 256 otherwise.
-template <class D>
-constexpr int trial_occ() {
-    return (sizeof(typename D::Real) == 4 && D::MC > 0 && D::MC <= 512) ? 512 : 256;
-}
-template <class D, int NG>
-__global__ void __launch_bounds__(D::TPF *NG, trial_occ<D>() / (D::TPF * NG))
-    ypass_trial_kernel(const typename D::Real *__restrict__ t1, const typename D::Real *__restrict__ t2,
-                       typename D::Real *__restrict__ out, long long bs, int ncols, PlanT<typename D::Real> pl,
-                       Mult mult) {
-    using T = typename D::Real;
-    using C = typename D::C;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *smem = reinterpret_cast<C *>(smem_raw);
-    constexpr int TPF = D::TPF;
-    constexpr int W = 2 * NG;
-    const int M = pl.M;
-    const int G = D::smem_len(M);
-    const int g = threadIdx.x / TPF, t = threadIdx.x % TPF;
-    double2 *wt = reinterpret_cast<double2 *>(smem_raw + scratch_offset<D>(M, W)) + D::NWARP * g;
-    const int b = blockIdx.y;
-    const int c0 = blockIdx.x * W;  // 0-based first column
-    const T *s1 = t1 + b * bs, *s2 = t2 + b * bs;
-    T *dst = out + b * bs;
-    if constexpr (D::MC > 0) {
-        constexpr int NT = NG * TPF;
-        constexpr int NIT = (W * (D::MC + 1) + NT - 1) / NT;
-        constexpr int CH = 8;
-#pragma unroll
-        for (int k0 = 0; k0 < NIT; k0 += CH) {
-            T va[CH], vb[CH];
-#pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const int e = threadIdx.x + (k0 + k) * NT;
-                const int c = e % W, jj = e / W;
-                const int col = c0 + c;
-                const bool ok = k0 + k < NIT && jj >= 1 && jj < D::MC && col < ncols;
-                const long long o = col + (long long)ncols * (jj - 1);
-                va[k] = ok ? s1[o] : (T)0;
-                vb[k] = ok ? s2[o] : (T)0;
-            }
-#pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const int e = threadIdx.x + (k0 + k) * NT;
-                const int c = e % W, jj = e / W;
-                if (k0 + k < NIT && jj <= D::MC) smem[c * G + D::idx(jj)] = Cx<T>::make(va[k], vb[k]);
-            }
-        }
-    } else
-    for (int e = threadIdx.x; e < W * (M + 1); e += blockDim.x) {
-        const int c = e % W, jj = e / W;
-        const int col = c0 + c;
-        C z = Cx<T>::make(0, 0);
-        if (jj >= 1 && jj < M && col < ncols) {
-            const long long o = col + (long long)ncols * (jj - 1);
-            z = Cx<T>::make(s1[o], s2[o]);
-        }
-        smem[c * G + D::idx(jj)] = z;
-    }
-    __syncthreads();
-    const double cb = mult.coef(b);
-    const double scale = mult.scale;
-#pragma unroll 1
-    for (int r = 0; r < 2; ++r) {
-        const int c = r * NG + g;
-        C *buf = smem + c * G;
-        D::dst(buf, pl, t, wt);
-        const int col1 = c0 + c + 1;  // 1-based column
-        const bool ok = col1 <= ncols;
-        const double cxv = ok ? __ldg(&mult.cx[col1]) : 0.0;
-        auto combine = [&](int jj, double cyj) {
-            const C y = buf[D::idx(jj)];
-            double v = 0.0;
-            if (ok) {
-                const double lam = -2 * ((cxv + cyj) - 2);
-                v = ((double)y.x * (1 - lam * cb) + (double)y.y) * (scale * recip(1 + lam * cb));
-            }
-            buf[D::idx(jj)] = Cx<T>::make((T)v, 0);
-        };
-        if constexpr (D::MC > 0) {
-            constexpr int NIT = (D::MC - 1 + TPF - 1) / TPF;
-            double cyv[NIT];
-#pragma unroll
-            for (int k = 0; k < NIT; ++k) {
-                const int jj = 1 + t + k * TPF;
-                cyv[k] = jj < D::MC ? __ldg(&mult.cy[jj]) : 0.0;
-            }
-#pragma unroll
-            for (int k = 0; k < NIT; ++k) {
-                const int jj = 1 + t + k * TPF;
-                if (jj < D::MC) combine(jj, cyv[k]);
-            }
-        } else {
-            for (int jj = 1 + t; jj < M; jj += TPF) combine(jj, __ldg(&mult.cy[jj]));
-        }
-        __syncthreads();
-    }
-    // phase 2: pack columns (2g, 2g+1) into buffer 2g
-    {
-        C *ba = smem + (2 * g) * G;
-        const C *bb = smem + (2 * g + 1) * G;
-        for (int jj = 1 + t; jj < M; jj += TPF) ba[D::idx(jj)].y = bb[D::idx(jj)].x;
-        __syncthreads();
-        D::dst(ba, pl, t, wt);
-    }
-    for (int e = threadIdx.x; e < W * (M + 1); e += blockDim.x) {
-        const int c = e % W, jj = e / W;
-        const int col = c0 + c;
-        if (jj >= 1 && jj < M && col < ncols) {
-            const C y = smem[(c & ~1) * G + D::idx(jj)];
-            dst[col + (long long)ncols * (jj - 1)] = (c & 1) ? y.y : y.x;
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Stencil kernels
 // ---------------------------------------------------------------------------
@@ -567,7 +246,7 @@ struct NonlinArgs {
     const T *gam;         // ng x L
     T *out;               // ng x L (state.nonlin[1])
     const T *n2;          // ng x L (state.nonlin[2]); with rest != nullptr
-    T *rest;              // ng x L: dt (1.5 N1 - 0.5 N2) + rhsbc, or nullptr
+    T *rest;              // ng x L: A Gamma + dt (1.5 N1 - 0.5 N2) + rhsbc, or nullptr
     const StepDev *prm;
     Grid g;
     // Ensembles of cases of one shape, stacked case-major (batch b = case L + level - 1):
@@ -733,10 +412,17 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
         const double n1 = r * (1 / (hc * hc));
         a.out[b * ng + GI(I, J)] = (T)n1;
         if (a.rest) {
-            // rest = dt b1 N1 + dt b2 N2 + rhsbc (fluid.jl:487-493), rhsbc = apply_bc!(0, get_bc(..); fac)
-            double v = (g.dt * 1.5) * n1 + (g.dt * -0.5) * (double)rn[y][x];
+            // rest = A Gamma + dt b1 N1 + dt b2 N2 + rhsbc (fluid.jl:487-493), rhsbc =
+            // apply_bc!(0, get_bc(..); fac).  A = 1 - c (-Laplacian), diagonal under the
+            // 2D DST, is this five-point stencil with zeros beyond the field: taking it
+            // here spares the trial solve a second field through its passes
+            const double rc = g.dt / (re_of() * (hc * hc));
+            const double gc = (double)gm[y + 1][x + 1];
+            const double lap = ((double)gm[y + 1][x] + (double)gm[y + 1][x + 2] - 2 * gc) +
+                               ((double)gm[y][x + 1] + (double)gm[y + 2][x + 1] - 2 * gc);
+            double v = (g.dt * 1.5) * n1 + (g.dt * -0.5) * (double)rn[y][x] + (gc + 0.5 * rc * lap);
             if (lev < g.L && on_ring(g, I, J)) {
-                const double fac = 0.25 * g.dt / (re_of() * (hc * hc));
+                const double fac = 0.25 * rc;
                 v = v + apply_bc_at(0.0, C, g, I, J, fac);
             }
             a.rest[b * ng + GI(I, J)] = (T)v;

@@ -5,7 +5,7 @@
 // Some callers cannot call cudaMalloc at all: code running inside another
 // framework's memory pool or a pre-sized arena, or a host loop that must not
 // allocate between steps.  They pass device pointers for the right-hand side and
-// the result; everything else this solve needs -- two scratch fields and the
+// the result; everything else this solve needs -- a scratch field and the
 // transform tables -- lives in the file-scope array `g_scratch` below, a fixed
 // block of device memory that every GPU loading the library holds until the
 // process exits.  No cudaMalloc, cudaFree or allocating library routine is
@@ -41,8 +41,12 @@ namespace {
 
 constexpr long long kNoAllocMaxCells = 1LL << 18;
 constexpr int kNoAllocMaxM = 1024;
-// field scratch (2 fields) + twiddles and sine/cosine tables for x and y
-constexpr size_t kScratchDoubles = 2 * kNoAllocMaxCells + 2 * (2 * kNoAllocMaxM) + 4 * (kNoAllocMaxM + 1);
+// field scratch (rows padded to a multiple of four) + twiddles and sine/cosine tables for x and y
+constexpr size_t kScratchField = kNoAllocMaxCells + 4 * kNoAllocMaxM;
+// offset of the y solve's tables after the transforms' (a multiple of 16 bytes)
+constexpr size_t kYTables = 2 * (2 * kNoAllocMaxM) + 4 * (kNoAllocMaxM + 1);
+static_assert(sizeof(YCol) == 8 * sizeof(double) && kYTables % 2 == 0 && kYDiff % 2 == 0, "table alignment");
+constexpr size_t kScratchDoubles = kScratchField + kYTables + 8 * kNoAllocMaxM + kYDiff + 2 * (kYChunks + 1) * kYFull;
 
 static __device__ __align__(256) double g_scratch[kScratchDoubles];
 
@@ -114,14 +118,6 @@ cudaError_t xpass_na(const PlanT<double> &pl, In in, Out out, int nrows, cudaStr
     return cudaLaunchKernelEx(&c, xpass_kernel<D, NG, In, Out>, in, out, pl, nrows, (const int *)nullptr, 0, 0);
 }
 
-template <class D>
-cudaError_t ypass_na(const PlanT<double> &pl, const double *in, double *out, int ncols, Mult m, cudaStream_t st) {
-    constexpr int NG = 2;
-    const cudaLaunchConfig_t c =
-        launch_cfg(dim3((ncols + 2 * NG - 1) / (2 * NG), 1), dim3(NG * D::TPF), pass_smem<D>(pl.M, NG, NG), st);
-    return cudaLaunchKernelEx(&c, ypass_kernel<D, NG>, in, out, 0LL, ncols, pl, m);
-}
-
 cudaError_t tables_na(double2 *tw, double *sn, double *cs, int M, cudaStream_t st) {
     const cudaLaunchConfig_t c = launch_cfg(dim3(8), dim3(128), 0, st);
     return cudaLaunchKernelEx(&c, noalloc_tables_kernel, tw, sn, cs, M);
@@ -153,7 +149,7 @@ int ibpm_lap_inv_noalloc(int nx, int ny, const double *b, double *x, void *strea
             slot.base = static_cast<double *>(p);
         }
         base = slot.base;
-        double *tab = base + 2 * kNoAllocMaxCells;
+        double *tab = base + kScratchField;
         double2 *twx = reinterpret_cast<double2 *>(tab), *twy = reinterpret_cast<double2 *>(tab + 2 * kNoAllocMaxM);
         double *snx = tab + 4 * kNoAllocMaxM, *sny = snx + (kNoAllocMaxM + 1);
         double *csx = sny + (kNoAllocMaxM + 1), *csy = csx + (kNoAllocMaxM + 1);
@@ -167,32 +163,30 @@ int ibpm_lap_inv_noalloc(int nx, int ny, const double *b, double *x, void *strea
                             "nx, ny on this device outside stream capture");
             e = tables_na(twx, snx, csx, nx, st);
             if (e == cudaSuccess) e = tables_na(twy, sny, csy, ny, st);
+            if (e == cudaSuccess)
+                e = launch_ycols(reinterpret_cast<YCol *>(tab + kYTables), tab + kYTables + 8 * kNoAllocMaxM,
+                                 reinterpret_cast<double2 *>(tab + kYTables + 8 * kNoAllocMaxM + kYDiff), csx, csy, nx, ny,
+                                 nullptr, 1, st);
             if (e != cudaSuccess) return fail(IBPM_ERR_CUDA, cudaGetErrorString(e));
             slot.nx = nx;
             slot.ny = ny;
         }
     }
-    double *t1 = base, *t2 = base + kNoAllocMaxCells;
-    double *tab = base + 2 * kNoAllocMaxCells;
+    double *t1 = base;
+    double *tab = base + kScratchField;
     plx.tw = reinterpret_cast<const double2 *>(tab);
     ply.tw = reinterpret_cast<const double2 *>(tab + 2 * kNoAllocMaxM);
     plx.sn = tab + 4 * kNoAllocMaxM;
     ply.sn = plx.sn + (kNoAllocMaxM + 1);
-    Mult m{};
-    m.mode = MULT_LAPINV;
-    m.cx = ply.sn + (kNoAllocMaxM + 1);
-    m.cy = m.cx + (kNoAllocMaxM + 1);
-    m.scale = 1.0 / (double)(4 * (long long)nx * (long long)ny);
-    m.h = 1.0;
-    m.Re = 1.0;
-    m.dt = 0.0;
-    m.lev0 = 1;
-    m.levstep = 0;
+    const YSolve m{reinterpret_cast<const YCol *>(tab + kYTables),
+                   tab + kYTables + 8 * kNoAllocMaxM,
+                   reinterpret_cast<const double2 *>(tab + kYTables + 8 * kNoAllocMaxM + kYDiff), 0, 0};
     using D = GenericDst<double>;
-    cudaError_t e = xpass_na<D>(plx, InPlain<double>{b, 0, nx - 1}, OutPlain<double>{t1, 0, nx - 1}, ny - 1, st);
-    if (e == cudaSuccess) e = ypass_na<D>(ply, t1, t2, nx - 1, m, st);
+    const int ld = (nx + 3) / 4 * 4;
+    cudaError_t e = xpass_na<D>(plx, InPlain<double>{b, 0, nx - 1}, OutPlain<double>{t1, 0, ld}, ny - 1, st);
+    if (e == cudaSuccess) e = launch_ytri<double>(t1, t1, 0, ld, nx - 1, ny, 1, ytri_wshift<double>(nx - 1, ny, 1), m, st);
     if (e == cudaSuccess)
-        e = xpass_na<D>(plx, InPlain<double>{t2, 0, nx - 1}, OutPlain<double>{x, 0, nx - 1}, ny - 1, st);
+        e = xpass_na<D>(plx, InPlain<double>{t1, 0, ld}, OutPlain<double>{x, 0, nx - 1}, ny - 1, st);
     if (e != cudaSuccess) return fail(IBPM_ERR_CUDA, cudaGetErrorString(e));
     return IBPM_OK;
 }
