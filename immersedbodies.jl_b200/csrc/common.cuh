@@ -81,19 +81,6 @@ __device__ __forceinline__ double apply_bc_at(double v, const T *__restrict__ r,
     return v;
 }
 
-// float -> double by integer arithmetic, for kernels that load FP32 fields and
-// compute in FP64: exactly the cast's value, without the conversion unit, whose
-// rate held such a kernel back (Y solve of five 1024^2 FP32 fields: 34.2 us with
-// the casts, 22.7 us so; the stores' narrowing casts cost nothing measurable).
-__device__ __forceinline__ double widen(float f) {
-    const unsigned u = __float_as_uint(f);
-    if ((u << 1) >= 0xff000000u) return (double)f;
-    // the float's fields in the double's places, 896 binades low: exact to scale back,
-    // zeros and denormals included
-    return __hiloint2double((int)((u & 0x80000000u) | ((u & 0x7fffffffu) >> 3)), (int)(u << 29)) * 0x1p896;
-}
-__device__ __forceinline__ double widen(double d) { return d; }
-
 // One element global -> shared memory without passing through registers
 // (cp.async, 4 or 8 bytes; both addresses naturally aligned).  Completed by
 // cp_async_wait_all() in the issuing thread, then a barrier for the block.

@@ -327,7 +327,7 @@ struct Engine final : ibpm_handle {
     double fs_last[2] = {0, 0}, gm_last[6] = {0, 0, 0, 0, 0, 0};
     // work
     int kbatch = 1;  // columns per batch in the B setup
-    T *t1 = nullptr, *rhs = nullptr, *rest = nullptr, *qs1 = nullptr;
+    T *t1 = nullptr, *t2 = nullptr, *rhs = nullptr, *rest = nullptr, *qs1 = nullptr;  // t2: FP32 trial solve only
     double *Ftmp = nullptr, *part = nullptr;
     T *patch = nullptr;
     long long patch_stride = 0;
@@ -399,24 +399,28 @@ struct Engine final : ibpm_handle {
     void resize_batch_buffers(int kb) {
         CK(cudaStreamSynchronize(st));
         const int k2 = std::max(kb, L);
-        const size_t sizes[6] = {sizeof(T) * (size_t)(nt * k2),     sizeof(T) * (size_t)(patch_stride * kb),
+        const size_t sizes[7] = {sizeof(T) * (size_t)(nt * k2),     sizeof(T) * (size_t)(patch_stride * kb),
                                  sizeof(T) * (size_t)(ng * L * kb), sizeof(T) * (size_t)(ng * L * kb),
-                                 sizeof(T) * (size_t)(nq * kb),     sizeof(double) * 2 * (size_t)np * kb};
-        void *fresh[6] = {};
+                                 sizeof(T) * (size_t)(nq * kb),     sizeof(double) * 2 * (size_t)np * kb,
+                                 sizeof(double) * (size_t)(line_len() * kb)};
+        void *fresh[7] = {};
         try {
-            for (int k = 0; k < 6; ++k) fresh[k] = dalloc<unsigned char>(sizes[k]);
+            for (int k = 0; k < 7; ++k) fresh[k] = dalloc<unsigned char>(sizes[k]);
         } catch (...) {
             for (void *p : fresh) dfree(p);
             throw;
         }
         drop_graphs();
-        for (void *p : {(void *)t1, (void *)patch, (void *)Gw, (void *)psiw, (void *)qw, (void *)fcol}) dfree(p);
+        for (void *p : {(void *)t1, (void *)patch, (void *)Gw, (void *)psiw, (void *)qw, (void *)fcol, (void *)lines})
+            dfree(p);
         t1 = static_cast<T *>(fresh[0]);
         patch = static_cast<T *>(fresh[1]);
         Gw = static_cast<T *>(fresh[2]);
         psiw = static_cast<T *>(fresh[3]);
         qw = static_cast<T *>(fresh[4]);
         fcol = static_cast<double *>(fresh[5]);
+        lines = static_cast<double *>(fresh[6]);
+        t1_fields = k2;
         kbatch = kb;
     }
 
@@ -480,31 +484,51 @@ struct Engine final : ibpm_handle {
     // ---- line passes ----
     // Dispatch on the transform length: compile-time transforms for
     // M in {256, 384, 512, 1024}, the runtime mixed-radix one otherwise.
-    template <class D, class In, class Out>
-    void xpass_t(const PlanT<typename D::Real> &pl, In in, Out out, int nbatch, const int *rows, int zero_outside,
-                 int rows_stride) {
-        const int pairs = (ny - 1 + 1) / 2;
-        const dim3 grid((pairs + kNG - 1) / kNG, nbatch);
-        const size_t sm = pass_smem<D>(pl.M, kNG, kNG);
-        xpass_kernel<D, kNG, In, Out><<<grid, kNG * D::TPF, sm, st>>>(in, out, pl, ny - 1, rows, zero_outside,
-                                                                       rows_stride);
+    // The rows an X pass covers: see xpass_kernel (rows null: every row)
+    struct XOpt {
+        const int *rows = nullptr;
+        int zero_outside = 0, rows_stride = 0, rows_mod = 1;
+    };
+    // calls f with the line transform (of element type R) of length M
+    template <class R, class F>
+    static void with_dst(int M, F &&f) {
+        switch (M) {
+            case 1024: f(Pow2Dst<1024, R>{}); break;
+            case 512: f(Pow2Dst<512, R>{}); break;
+            case 256: f(Pow2Dst<256, R>{}); break;
+            case 384: f(MixDst<384, R>{}); break;
+            default: f(GenericDst<R>{}); break;
+        }
     }
     // X pass with transforms of element type R (the engine's T, or double for
     // the FP32 engine's FP64 level-1 solve); In/Out convert at the boundary.
-    // rows, zero_outside, rows_stride: see xpass_kernel (rows null: every row).
     template <class R = T, class In, class Out>
-    void xpass(In in, Out out, int nbatch, const int *rows = nullptr, int zero_outside = 0, int rows_stride = 0) {
+    void xpass(In in, Out out, int nbatch, const XOpt &o = {}) {
         const PlanT<R> &pl = plan_x<R>();
+        const int nrows = ny - 1;
         const int pe = prof_begin();
-        switch (pl.M) {
-            case 1024: xpass_t<Pow2Dst<1024, R>>(pl, in, out, nbatch, rows, zero_outside, rows_stride); break;
-            case 512: xpass_t<Pow2Dst<512, R>>(pl, in, out, nbatch, rows, zero_outside, rows_stride); break;
-            case 256: xpass_t<Pow2Dst<256, R>>(pl, in, out, nbatch, rows, zero_outside, rows_stride); break;
-            case 384: xpass_t<MixDst<384, R>>(pl, in, out, nbatch, rows, zero_outside, rows_stride); break;
-            default: xpass_t<GenericDst<R>>(pl, in, out, nbatch, rows, zero_outside, rows_stride); break;
-        }
+        with_dst<R>(pl.M, [&](auto d) {
+            using D = decltype(d);
+            const int pairs = (nrows + 1) / 2;
+            const dim3 grid((pairs + kNG - 1) / kNG, nbatch);
+            xpass_kernel<D, kNG, In, Out><<<grid, kNG * D::TPF, pass_smem<D>(pl.M, kNG, kNG), st>>>(
+                in, out, pl, nrows, o.rows, o.zero_outside, o.rows_stride, o.rows_mod);
+        });
         check_launch();
         prof_end(pe, IBPM_KCLASS_XPASS, 2.0 * sizeof(R) * (double)ng * nbatch);
+    }
+    // the finer level's boundary values alone, from a solved scratch field
+    // (psi_, pbs, win, win_stride: see xlines_kernel)
+    void xlines(const InPlain<T> &in, int nbatch, T *psi_, long long pbs, const int *win, int win_stride) {
+        const int pe = prof_begin();
+        with_dst<T>(plx.M, [&](auto d) {
+            using D = decltype(d);
+            constexpr int NB = 64 / D::TPF;
+            xlines_kernel<D><<<dim3(1 + (ny / 2 + nx + 1) / 2, nbatch), 64, pass_smem<D>(plx.M, NB, NB), st>>>(
+                in, ring_out(), plx, line_w, line_w + nx, psi_, pbs, win, win_stride);
+        });
+        check_launch();
+        prof_end(pe, IBPM_KCLASS_XPASS, 0.5 * sizeof(T) * (double)ng * nbatch);
     }
     // the autotuner's key of a Y pass of length M over nbatch fields
     std::string devname;  // the GPU's name, read once at setup (a tuning key's first part)
@@ -513,25 +537,58 @@ struct Engine final : ibpm_handle {
         return devname + " ypass M=" + std::to_string(M) + (sizeof(R) == 8 ? " fp64" : " fp32") +
                " batch=" + std::to_string(batch_bucket(nbatch));
     }
-    // column pairs per block of a Y pass: forced, tuned, or the fixed rule
+    // The solves' y direction by transforms, as the FP32 engine does it in both
+    // precisions (see ypass_kernel); the FP64 engine only where it assembles the
+    // FP32 engine's B
+    bool by_transforms = !std::is_same<T, double>::value;
+    // column pairs per block of a Y pass: forced, tuned, or the fixed rule (by
+    // transforms: launches over many fields have waves to spare, and wider blocks
+    // read longer segments of each row)
     template <class R>
     int ypass_ng(int M, int nbatch) {
         if (const int f = tune_forced_ng()) return f;
         int v = 0;
         if (tune_table().find(ypass_key<R>(M, nbatch), &v)) return v;
-        return 1 << (ytri_wshift<R>(nx - 1, M, nbatch) - 1);
+        if (!by_transforms) return 1 << (ytri_wshift(nx - 1, nbatch) - 1);
+        return (M == 256 || M == 384 || M == 512 || M == 1024) && nbatch >= 16 ? 4 : kNG;
     }
-    template <class R>
-    void ypass_launch(int ngy, const R *in, R *out, int nbatch, const YSolve &m) {
+    void ypass_launch(int ngy, double *f, int nbatch, const YSolve &m, long long bs, const YRing &ring = {}) {
         const int wshift = ngy <= 1 ? 1 : ngy == 2 ? 2 : 3;  // at most kYMaxW columns a block
-        CK(launch_ytri<R>(in, out, nt, ldt, nx - 1, ny, nbatch, wshift, m, st));
+        CK(launch_ytri(f, bs, ldt, nx - 1, ny, nbatch, wshift, m, st, ring));
     }
-    // Times every block shape of the Y pass over nbatch fields of scratch (in ->
-    // out, pitched, at least nbatch * nt elements each) and records the fastest;
-    // eager only.
+    // by transforms; c null: the Laplacian inverse
     template <class R>
-    void tune_ypass(const R *in, R *out, int nbatch) {
-        if (!tune_enabled() || tune_forced_ng()) return;
+    void ypass_dst_launch(int ngy, R *f, int nbatch, const double *c, int cs) {
+        with_dst<R>(ny, [&](auto d) {
+            using D = decltype(d);
+            switch (ngy) {
+                case 1: ypass_dst_t<D, 1>(f, nbatch, c, cs); break;
+                case 4: ypass_dst_t<D, 4>(f, nbatch, c, cs); break;
+                case 8: ypass_dst_t<D, 8>(f, nbatch, c, cs); break;
+                default: ypass_dst_t<D, 2>(f, nbatch, c, cs); break;
+            }
+        });
+    }
+    template <class D, int NGY, class R = typename D::Real>
+    void ypass_dst_t(R *f, int nbatch, const double *c, int cs) {
+        const size_t sm = pass_smem<D>(ny, NGY, NGY);
+        if (sm > 48 * 1024) {
+            // covers every M the instantiation serves; the attribute is per device
+            static std::atomic<unsigned long long> attr_devices{0};
+            if (need_attr(attr_devices)) {
+                CK(cudaFuncSetAttribute(ypass_kernel<D, NGY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)pass_smem<D>(D::MC > 0 ? ny : kMaxM, NGY, NGY)));
+                attr_devices.fetch_or(device_bit());
+            }
+        }
+        ypass_kernel<D, NGY><<<dim3((nx - 1 + 2 * NGY - 1) / (2 * NGY), nbatch), NGY * D::TPF, sm, st>>>(
+            f, f, nt, ldt, nx - 1, plan_y<R>(), c, cs, cx, cy, mult(MULT_LAPINV, 1).scale);
+    }
+    // Times every block shape of the Y pass over nbatch pitched fields of scratch (at
+    // least nbatch * nt elements) and records the fastest; eager only.
+    template <class R>
+    void tune_ypass(R *f, int nbatch) {
+        if (!tune_enabled() || tune_forced_ng() || (by_transforms && std::is_same<T, double>::value)) return;
         const std::string key = ypass_key<R>(ny, nbatch);
         int have = 0;
         if (tune_table().find(key, &have)) return;
@@ -544,7 +601,13 @@ struct Engine final : ibpm_handle {
         float best = 1e30f;
         int best_ng = kNG;
         for (int ngy : kTuneNGs) {
-            auto run = [&] { ypass_launch<R>(ngy, in, out, nbatch, ysolve(MULT_LAPINV, 1, 0)); };
+            auto run = [&] {
+                if constexpr (std::is_same<T, double>::value)
+                    ypass_launch(ngy, f, nbatch, ysolve(MULT_LAPINV, 1, 0), nt);
+                else
+                    ypass_dst_launch<R>(ngy, f, nbatch, nullptr, 0);
+                CK(cudaGetLastError());
+            };
             run();
             run();
             CK(cudaEventRecord(e0, st));
@@ -562,13 +625,33 @@ struct Engine final : ibpm_handle {
         cudaEventDestroy(e1);
         tune_table().put(key, best_ng);
     }
-    // Y pass of nbatch pitched scratch fields (nt elements apart), in place or not
-    template <class R = T>
-    void ypass(const R *in, R *out, int nbatch, const YSolve &m) {
+    // Y pass, in place, of nbatch pitched scratch fields (bs elements apart; 0: nt);
+    // FP64 with the boundary values of a coarser level or none
+    void ypass(double *f, int nbatch, const YSolve &m, long long bs = 0, const YRing &ring = {}) {
         const int pe = prof_begin();
-        ypass_launch<R>(ypass_ng<R>(ny, nbatch), in, out, nbatch, m);
+        ypass_launch(ypass_ng<double>(ny, nbatch), f, nbatch, m, bs ? bs : nt, ring);
+        check_launch();
+        prof_end(pe, IBPM_KCLASS_YPASS, 16.0 * (double)ng * nbatch);
+    }
+    template <class R>
+    void ypass_dst(R *f, int nbatch, const double *c, int cs) {
+        const int pe = prof_begin();
+        ypass_dst_launch<R>(ypass_ng<R>(ny, nbatch), f, nbatch, c, cs);
         check_launch();
         prof_end(pe, IBPM_KCLASS_YPASS, 2.0 * sizeof(R) * (double)ng * nbatch);
+    }
+    // either way: the Laplacian inverse, and the implicit diffusion of one level
+    template <class R>
+    void ylap(R *f, int nbatch) {
+        if constexpr (std::is_same<T, double>::value)
+            if (!by_transforms) return ypass(f, nbatch, ysolve(MULT_LAPINV, 1, 0));
+        ypass_dst(f, nbatch, nullptr, 0);
+    }
+    template <class R>
+    void yimp(R *f, int nbatch, int lev = 1) {
+        if constexpr (std::is_same<T, double>::value)
+            if (!by_transforms) return ypass(f, nbatch, ysolve(MULT_AIMPL, lev, 0));
+        ypass_dst(f, nbatch, coef_lev + (lev - 1), 0);
     }
     // transform tables of element type R: the engine's own, or FP64 ones kept by
     // the FP32 engine for its level-1 solve
@@ -583,14 +666,54 @@ struct Engine final : ibpm_handle {
     }
     double *psi1_hi = nullptr, *qs1_hi = nullptr, *t1_hi = nullptr;
     // The trial solve of get_trial_state (src/fluid.jl:485-496), Gamma_new =
-    // Ainv (A Gamma + dt (1.5 N1 - 0.5 N2) + rhsbc) of nb fields; the nonlinear
-    // kernel has formed the right-hand side (rest_)
-    template <class R>
-    void trial(const R *rest_, R *Gnew, int nb, const YSolve &m, R *scratch) {
-        xpass<R>(InPlain<R>{rest_, ng, nx - 1}, OutPlain<R>{scratch, nt, ldt}, nb);
-        ypass<R>(scratch, scratch, nb, m);
-        xpass<R>(InPlain<R>{scratch, nt, ldt}, OutPlain<R>{Gnew, ng, nx - 1}, nb);
+    // Ainv (A Gamma + dt (1.5 N1 - 0.5 N2) + rhsbc) of nb fields.  FP64: the
+    // nonlinear kernel has formed the right-hand side (rest_)
+    void trial(const double *rest_, double *Gnew, int nb, const YSolve &m, double *scratch) {
+        xpass<double>(InPlain<double>{rest_, ng, nx - 1}, OutPlain<double>{scratch, nt, ldt}, nb);
+        ypass(scratch, nb, m);
+        xpass<double>(InPlain<double>{scratch, nt, ldt}, OutPlain<double>{Gnew, ng, nx - 1}, nb);
     }
+    // By transforms: Gamma and the rest of the right-hand side as one complex line
+    // (the merged trial kernels); c = dt / (2 Re hc^2) of every field, scratch of nb
+    // fields each
+    template <class D, int NG, class R = typename D::Real>
+    void trial_ypart(int nb, const double *c, R *t1_, R *t2_) {
+        // the cap must cover the largest M this instantiation serves (kMaxM); the
+        // attribute is per device
+        static std::atomic<unsigned long long> attr_devices{0};
+        if (need_attr(attr_devices)) {
+            CK(cudaFuncSetAttribute(ypass_trial_kernel<D, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)pass_smem<D>(kMaxM, 2 * NG, NG)));
+            attr_devices.fetch_or(device_bit());
+        }
+        const int pe = prof_begin();
+        ypass_trial_kernel<D, NG><<<dim3((nx - 1 + 2 * NG - 1) / (2 * NG), nb), NG * D::TPF, pass_smem<D>(ny, 2 * NG, NG), st>>>(
+            t1_, t2_, t1_, ng, nx - 1, plan_y<R>(), c, cx, cy, mult(MULT_AIMPL, 1).scale);
+        check_launch();
+        prof_end(pe, IBPM_KCLASS_YTRIAL, 3.0 * sizeof(R) * (double)ng * nb);
+    }
+    template <class R>
+    void trial_dst(const R *Gold, const R *rest_, R *Gnew, int nb, const double *c, R *t1_, R *t2_) {
+        const int pe = prof_begin();
+        with_dst<R>(nx, [&](auto d) {
+            using D = decltype(d);
+            xpass_trial_kernel<D, kNG><<<dim3((ny - 1 + kNG - 1) / kNG, nb), kNG * D::TPF, pass_smem<D>(nx, kNG, kNG), st>>>(
+                Gold, rest_, t1_, t2_, ng, nx - 1, plan_x<R>(), ny - 1);
+        });
+        check_launch();
+        prof_end(pe, IBPM_KCLASS_XTRIAL, 4.0 * sizeof(R) * (double)ng * nb);
+        with_dst<R>(ny, [&](auto d) {
+            using D = decltype(d);
+            // many fields per launch (ensemble groups) take 2 NG columns per block
+            if (nb >= 16 && ny <= 512)
+                trial_ypart<D, 2 * kNG>(nb, c, t1_, t2_);
+            else
+                trial_ypart<D, kNG>(nb, c, t1_, t2_);
+        });
+        xpass<R>(InPlain<R>{t1_, ng, nx - 1}, OutPlain<R>{Gnew, ng, nx - 1}, nb);
+    }
+    // dt / (2 Re hc^2) of levels 1..L (device)
+    double *coef_lev = nullptr;
 
     double coef(int lev) const {  // dt / (2 Re hc^2)
         const double hc = ldexp(g.h, lev - 1);
@@ -614,6 +737,18 @@ struct Engine final : ibpm_handle {
     OutPlain<T> out_plain(T *p, long long bs) const { return OutPlain<T>{p, bs, nx - 1}; }
     // the solves' scratch fields between the passes: rows ldt apart (a multiple of
     // 32 bytes, so a block's columns start on a sector), fields nt apart
+    // boundary values between the levels of a telescoping solve, one record per
+    // batch, and the sine weights of the two columns (2 nx doubles)
+    double *lines = nullptr, *line_w = nullptr;
+    int *central_win = nullptr;  // rows of each level a B application's vorticity occupies (4 L)
+    int t1_fields = 0;           // fields t1 holds
+    long long line_len() const { return 2LL * (nx + ny); }
+    double *ring_q = nullptr;
+    // modes of one parity couple only (the interpolated part is centred)
+    int ring_step() const { return nx % 4 == 0 ? 2 : 1; }
+    int ring_ld() const { return nx % 4 == 0 ? nx / 2 : nx - 1; }
+    RingOut ring_out() const { return RingOut{lines, line_len(), nx, ny, ring_q, ring_ld(), ring_step()}; }
+    YRing ring_in() const { return YRing{lines, line_len(), nx, ny}; }
     InPlain<T> in_scratch(const T *p) const { return InPlain<T>{p, nt, ldt}; }
     OutPlain<T> out_scratch(T *p) const { return OutPlain<T>{p, nt, ldt}; }
 
@@ -668,17 +803,27 @@ struct Engine final : ibpm_handle {
 
     // vort2flux (src/fluid.jl:178-205) over nbatch independent fields.
     // G, psi: level 1 of batch 0, level stride ng, batch stride bs.
-    // qout: level 1 of batch 0 (level stride nq, batch stride qbs); curl_all=false
-    // computes q only at level 1 (the only level a caller reads).  win (device,
-    // with curl_all=false): the level-1 faces the caller reads (E's support, the
-    // body's bbox); level 1's last X pass and curl then skip what lies outside,
-    // leaving those rows of psi and faces of q unwritten.  central: the coarse
-    // levels of Gm hold zeros outside the central block that coarsify! writes
-    // (a B application's vorticity), so their prologues and coarsening skip the
-    // loads there; the results are the same bits.
+    // qout: level 1 of batch 0 (level stride nq, batch stride qbs).  curl_all=false
+    // computes q only at level 1 (the only level a caller reads) and solves each
+    // coarser level (FP64) as far as its finer level's boundary values: of their psi only
+    // level 2's four lines are written, where a face of bbox (device; batch b's at
+    // bbox + b bbox_stride; null: any face) lies on the domain's boundary.  win (device, with curl_all=false): the level-1 faces the
+    // caller reads (E's support, the body's bbox); level 1's last X pass and curl
+    // then skip what lies outside, leaving those rows of psi and faces of q
+    // unwritten.  central: the coarse levels of Gm hold zeros outside the central
+    // block that coarsify! writes (a B application's vorticity), so their X passes
+    // and coarsening skip the loads there; the results are the same bits.
+    //
+    // FP64: the levels depend on each other only through the boundary values, which
+    // enter in the Y solve (RingOut).  So one X pass transforms every level's
+    // vorticity where the scratch holds them all (a few fields: one launch of five
+    // 1024^2 levels 31 us against 64 one by one with boundary values); launches
+    // over many fields fill the GPU level by level.
     void vort2flux(T *psi_, T *qout, T *Gm, long long bs, long long qbs, int nbatch, bool curl_all,
-                   bool hi1 = false, const int *win = nullptr, bool central = false) {
+                   bool hi1 = false, const int *win = nullptr, bool central = false, const int *bbox = nullptr,
+                   int bbox_stride = 0) {
         if (curl_all) win = nullptr;
+        if (win) bbox = win;
         for (int lev = 2; lev <= L; ++lev) {
             const int nx2 = nx / 2, ny2 = ny / 2;
             const dim3 blk(16, 16), grd((nx2 + 15) / 16, (ny2 + 15) / 16, nbatch);
@@ -686,82 +831,123 @@ struct Engine final : ibpm_handle {
                                                  central && lev - 1 >= 2 ? 1 : 0);
             check_launch();
         }
+        if constexpr (std::is_same<T, double>::value) {
+            if (tc_on) {
+                vort2flux_tc(psi_, Gm, bs, nbatch, win, central);
+                curl(psi_, qout, bs, qbs, nbatch, false, win);
+                return;
+            }
+        }
+        bool direct = false;
+        if constexpr (std::is_same<T, double>::value) direct = !by_transforms;
+        if (direct) {
+            if constexpr (std::is_same<T, double>::value)
+                levels_direct(psi_, Gm, bs, nbatch, curl_all, win, central, bbox, bbox_stride);
+        } else if (!levels_dst(psi_, Gm, bs, nbatch, hi1, win, central)) {
+            return;
+        }
+        curl(psi_, qout, bs, qbs, nbatch, curl_all, win);
+    }
+
+    // vort2flux's solves, the y direction direct
+    void levels_direct(double *psi_, const double *Gm, long long bs, int nbatch, bool curl_all, const int *win, bool central,
+                  const int *bbox, int bbox_stride) {
+        const bool together = L > 1 && (long long)nbatch * L <= t1_fields;
+        auto forward = [&](int lev, int n) {  // X pass of levels lev .. lev + n - 1
+            XOpt o;
+            if (central) o = XOpt{central_win + 4 * (lev - 1), 1, 4, n};
+            xpass(InLevels<T>{(const T *)Gm + (lev - 1) * ng, bs, nx - 1, n, ng}, out_scratch(t1), nbatch * n, o);
+        };
+        if (together) forward(1, L);
+        for (int lev = L; lev >= 1; --lev) {
+            if (!together) forward(lev, 1);
+            T *ts = together ? t1 + (lev - 1) * nt : t1;
+            const long long tb = together ? L * nt : nt;
+            ypass(ts, nbatch, ysolve(MULT_LAPINV, 1, 0), tb, lev < L ? ring_in() : YRing{});
+            const InPlain<T> sol{ts, tb, ldt};
+            if (lev > 1) xlines(sol, nbatch, lev == 2 && !curl_all ? (T *)psi_ + ng : nullptr, bs, bbox, bbox_stride);
+            if (lev == 1 && !curl_all)
+                xpass(sol, out_plain((T *)psi_, bs), nbatch, XOpt{win});
+            else if (curl_all && !together)
+                xpass(sol, out_plain((T *)psi_ + (lev - 1) * ng, bs), nbatch);
+        }
+        if (curl_all && together) xpass(in_scratch(t1), out_plain((T *)psi_, ng), nbatch * L);  // fields are case-major
+    }
+
+    // vort2flux's solves by transforms: level by level, the boundary values added to
+    // the field.
+    // hi1: level 1 in FP64 into psi1_hi and its flux qs1_hi (batch strides ng and
+    // nq), with no psi of level 1; false then.
+    bool levels_dst(T *psi_, const T *Gm, long long bs, int nbatch, bool hi1, const int *win, bool central) {
+        for (int lev = L; lev >= 1; --lev) {
+            const T *Gl = Gm + (lev - 1) * ng;
+            const T *coarse = lev < L ? psi_ + lev * ng : nullptr;
+            if (lev == 1 && hi1) {
+                if (coarse)
+                    xpass<double>(InBC<T>{Gl, coarse, bs, bs, g}, OutPlain<double>{t1_hi, nt, ldt}, nbatch);
+                else
+                    xpass<double>(in_plain(Gl, bs), OutPlain<double>{t1_hi, nt, ldt}, nbatch);
+                ylap(t1_hi, nbatch);
+                xpass<double>(InPlain<double>{t1_hi, nt, ldt}, OutPlain<double>{psi1_hi, ng, nx - 1}, nbatch);
+                const dim3 blk(64, 4), grd((nx + 1 + 63) / 64, (ny + 1 + 3) / 4, nbatch);
+                curl_kernel<double, double, T><<<grd, blk, 0, st>>>(qs1_hi, nq, psi1_hi, ng, coarse, bs, g);
+                check_launch();
+                return false;
+            }
+            XOpt o;  // rows that coarsify! leaves zero: their boundary values alone are not, so only without
+            if (central && coarse == nullptr) o = XOpt{central_win + 4 * (lev - 1), 1, 0, 1};
+            if (coarse)
+                xpass(InBC<T>{Gl, coarse, bs, bs, g}, out_scratch(t1), nbatch);
+            else
+                xpass(in_plain(Gl, bs), out_scratch(t1), nbatch, o);
+            ylap(t1, nbatch);
+            xpass(in_scratch(t1), out_plain(psi_ + (lev - 1) * ng, bs), nbatch, XOpt{lev == 1 ? win : nullptr});
+        }
+        return true;
+    }
+
+    // The flux of level 1 or of every level (curl_all) from psi.
+    void curl(const T *psi_, T *qout, long long bs, long long qbs, int nbatch, bool curl_all, const int *win) {
+        const dim3 blk(64, 4);
+        // with a window and many fields the blocks sweep it (128 x 128 faces per
+        // sweep); a few fields keep one thread per face of the whole grid
+        const bool windowed = win != nullptr && nbatch > 4;
+        const dim3 grd(windowed ? std::min(2, (nx + 1 + 63) / 64) : (nx + 1 + 63) / 64,
+                       windowed ? std::min(32, (ny + 1 + 3) / 4) : (ny + 1 + 3) / 4, curl_all ? nbatch * L : nbatch);
+        const int pe = prof_begin();
+        if (curl_all)  // batch and level strides agree: fields are case-major
+            curl_kernel<T, T, T><<<grd, blk, 0, st>>>(qout, nq, psi_, ng, L > 1 ? psi_ + ng : nullptr, ng, g, nullptr, L);
+        else
+            curl_kernel<T, T, T><<<grd, blk, 0, st>>>(qout, qbs, psi_, bs, L > 1 ? psi_ + ng : nullptr, bs, g, win);
+        check_launch();
+        prof_end(pe, IBPM_KCLASS_CURL, 8.0 * (double)(ng + nq) * grd.z);
+    }
+
+    // The telescoping solves with the tensor-core transforms (a rebuild's B).
+    void vort2flux_tc(T *psi_, T *Gm, long long bs, int nbatch, const int *win, bool central) {
         // the central block coarsify! writes (faces nx/4+1 .. 3nx/4-1 by ny/4+1 .. 3ny/4-1)
         auto centred = [&](const auto &in) {
             using In = std::decay_t<decltype(in)>;
             return InCentral<In>{in, nx / 4 + 1, 3 * nx / 4 - 1, ny / 4 + 1, 3 * ny / 4 - 1};
         };
         for (int lev = L; lev >= 1; --lev) {
-            T *Gl = Gm + (lev - 1) * ng;
-            T *Pl = psi_ + (lev - 1) * ng;
-            if (lev == 1 && hi1) {
-                // level 1 in FP64 from the FP32 coarser levels: psi1_hi and qs1_hi (x E),
-                // batch strides ng and nq
-                const T *coarse = L > 1 ? psi_ + ng : nullptr;
-                if (coarse)
-                    xpass<double>(InBC<T>{Gl, coarse, bs, bs, g}, OutPlain<double>{t1_hi, nt, ldt}, nbatch);
+            T *Gl = Gm + (lev - 1) * ng, *Pl = psi_ + (lev - 1) * ng;
+            // coarse levels: only the lines the next finer level's boundary values
+            // read; level 1: the curl's window
+            TcKeep keep{TC_KEEP_LINES, nullptr, {ny / 4 - 1, 3 * ny / 4 - 1, nx / 4 - 1, 3 * nx / 4 - 1}};
+            if (lev == 1) keep = win ? TcKeep{TC_KEEP_WINDOW, win, {0, 0, 0, 0}} : TcKeep{TC_KEEP_ALL, nullptr, {0, 0, 0, 0}};
+            const bool cen = central && lev >= 2;
+            if (lev == L) {
+                if (cen)
+                    tc_solve(centred(in_plain(Gl, bs)), nbatch, tc_mult[0], Pl, bs, keep);
                 else
-                    xpass<double>(in_plain(Gl, bs), OutPlain<double>{t1_hi, nt, ldt}, nbatch);
-                ypass<double>(t1_hi, t1_hi, nbatch, ysolve(MULT_LAPINV, 1, 0));
-                xpass<double>(InPlain<double>{t1_hi, nt, ldt}, OutPlain<double>{psi1_hi, ng, nx - 1}, nbatch);
-                const dim3 blk(64, 4);
-                const dim3 grd((nx + 1 + 63) / 64, (ny + 1 + 3) / 4, nbatch);
-                curl_kernel<double, double, T><<<grd, blk, 0, st>>>(qs1_hi, nq, psi1_hi, ng, coarse, bs, g);
-                check_launch();
-                continue;
-            }
-            bool solved = false;
-            if constexpr (std::is_same<T, double>::value) {
-                if (tc_on) {
-                    // coarse levels: only the lines the next finer level's boundary
-                    // values read; level 1: the curl's window
-                    TcKeep keep{TC_KEEP_LINES, nullptr, {ny / 4 - 1, 3 * ny / 4 - 1, nx / 4 - 1, 3 * nx / 4 - 1}};
-                    if (lev == 1) keep = win ? TcKeep{TC_KEEP_WINDOW, win, {0, 0, 0, 0}} : TcKeep{TC_KEEP_ALL, nullptr, {0, 0, 0, 0}};
-                    const bool cen = central && lev >= 2;
-                    if (lev == L) {
-                        if (cen)
-                            tc_solve(centred(in_plain(Gl, bs)), nbatch, tc_mult[0], Pl, bs, keep);
-                        else
-                            tc_solve(in_plain(Gl, bs), nbatch, tc_mult[0], Pl, bs, keep);
-                    } else {
-                        const InBC<T> in{Gl, psi_ + lev * ng, bs, bs, g};
-                        if (cen)
-                            tc_solve(centred(in), nbatch, tc_mult[0], Pl, bs, keep);
-                        else
-                            tc_solve(in, nbatch, tc_mult[0], Pl, bs, keep);
-                    }
-                    solved = true;
-                }
-            }
-            if (!solved) {
-                bool cen = false;
-                if constexpr (std::is_same<T, double>::value) cen = central && lev >= 2;
-                if (lev == L) {
-                    if constexpr (std::is_same<T, double>::value)
-                        if (cen) xpass(centred(in_plain(Gl, bs)), out_scratch(t1), nbatch);
-                    if (!cen) xpass(in_plain(Gl, bs), out_scratch(t1), nbatch);
-                } else {
-                    const InBC<T> in{Gl, psi_ + lev * ng, bs, bs, g};
-                    if constexpr (std::is_same<T, double>::value)
-                        if (cen) xpass(centred(in), out_scratch(t1), nbatch);
-                    if (!cen) xpass(in, out_scratch(t1), nbatch);
-                }
-                ypass(t1, t1, nbatch, ysolve(MULT_LAPINV, 1, 0));
-                xpass(in_scratch(t1), out_plain(Pl, bs), nbatch, lev == 1 ? win : nullptr);
-            }
-            if (curl_all || lev == 1) {
-                const dim3 blk(64, 4);
-                // with a window and many fields the blocks sweep it (128 x 128 faces per
-                // sweep); a few fields keep one thread per face of the whole grid
-                const bool windowed = lev == 1 && win != nullptr && nbatch > 4;
-                const dim3 grd(windowed ? std::min(2, (nx + 1 + 63) / 64) : (nx + 1 + 63) / 64,
-                               windowed ? std::min(32, (ny + 1 + 3) / 4) : (ny + 1 + 3) / 4, nbatch);
-                const int pe = prof_begin();
-                curl_kernel<T, T, T><<<grd, blk, 0, st>>>(qout + (lev - 1) * nq, qbs, Pl, bs,
-                                                          lev < L ? psi_ + lev * ng : nullptr, bs, g,
-                                                          lev == 1 ? win : nullptr);
-                check_launch();
-                prof_end(pe, IBPM_KCLASS_CURL, 8.0 * (double)(ng + nq) * nbatch);
+                    tc_solve(in_plain(Gl, bs), nbatch, tc_mult[0], Pl, bs, keep);
+            } else {
+                const InBC<T> in{Gl, psi_ + lev * ng, bs, bs, g};
+                if (cen)
+                    tc_solve(centred(in), nbatch, tc_mult[0], Pl, bs, keep);
+                else
+                    tc_solve(in, nbatch, tc_mult[0], Pl, bs, keep);
             }
         }
     }
@@ -784,8 +970,8 @@ struct Engine final : ibpm_handle {
             }
         }
         if (!solved) {
-            xpass(in, out_scratch(t1), nbatch, P.bbox, 1);  // rot of the patch: zero outside its rows
-            ypass(t1, t1, nbatch, ysolve(MULT_AIMPL, 1, 0));
+            xpass(in, out_scratch(t1), nbatch, XOpt{P.bbox, 1, 0, 1});  // rot of the patch: zero outside its rows
+            yimp(t1, nbatch);
             // Gw's levels 2..L hold the level-1 vorticity coarsified and zeros elsewhere:
             // vort2flux's coarsify rewrites their central block, and nothing else ever
             // writes them, so the zeros of the allocation stay
@@ -843,7 +1029,7 @@ struct Engine final : ibpm_handle {
     // psi1, nl1 and FP64 scratch); the float arrays hold levels 2..L
     bool l1d = false;
     double *G1[2] = {nullptr, nullptr}, *nl1[2] = {nullptr, nullptr};
-    double *q1 = nullptr, *psi1 = nullptr, *rest1 = nullptr, *t1d = nullptr;
+    double *q1 = nullptr, *psi1 = nullptr, *rest1 = nullptr, *t1d = nullptr, *t2d = nullptr;
     double *patch_d = nullptr, *q0d = nullptr;
     void step_body_l1d();
     void vort2flux_l1d(const double *G1v, T *Gm, T *qout, double *psi1_out, double *q1_out, bool curl_all);
@@ -941,7 +1127,7 @@ void Engine<T>::setup() {
     {
         std::vector<double> hc(L);
         for (int lev = 1; lev <= L; ++lev) hc[lev - 1] = coef(lev);
-        double *cd = dalloc<double>(L);
+        double *cd = coef_lev = dalloc<double>(L);
         ycols = dalloc<YCol>((size_t)(nx - 1) * (L + 1));
         ydiff = dalloc<double>((size_t)kYDiff * (L + 1));
         yphase = dalloc<double2>((kYChunks + 1) * kYFull);
@@ -949,7 +1135,6 @@ void Engine<T>::setup() {
         CK(launch_ycols(ycols, ydiff, yphase, cx, cy, nx, ny, nullptr, 1, st));
         CK(launch_ycols(ycols + (nx - 1), ydiff + kYDiff, yphase, cx, cy, nx, ny, cd, L, st));
         CK(cudaStreamSynchronize(st));
-        dfree(cd);
     }
     if (!std::is_same<T, double>::value) {
         hi_level1 = true;
@@ -989,6 +1174,7 @@ void Engine<T>::setup() {
             psi1 = dalloc<double>(ng);
             rest1 = dalloc<double>(ng);
             t1d = dalloc<double>(nt);
+            t2d = dalloc<double>(ng);
             q0d = dalloc<double>(nq);
             patch_d = dalloc<double>(2LL * (nx + 1) * (ny + 1));
         }
@@ -1034,6 +1220,9 @@ void Engine<T>::setup() {
     kbatch = std::min(kbatch, 2 * np);
     const int kb = std::max(kbatch, L);
     t1 = dalloc<T>(nt * kb);
+    t1_fields = kb;
+    if (!std::is_same<T, double>::value) t2 = dalloc<T>(ng * L);
+    lines = dalloc<double>(line_len() * kbatch);
     rhs = dalloc<T>(nt);
     rest = dalloc<T>(ng * L);
     qs1 = dalloc<T>(nq);
@@ -1069,6 +1258,27 @@ void Engine<T>::setup() {
     cg_it = dalloc<int>(4);
     CK(cudaStreamCreateWithFlags(&st_side, cudaStreamNonBlocking));
 
+    // 2 sin(pi kx i / nx) of the columns nx/4 and 3 nx/4
+    std::vector<double> hw(2 * (size_t)nx, 0.0);
+    for (int c = 0; c < 2; ++c)
+        for (long long k = 1; k < nx; ++k)
+            hw[c * nx + k - 1] = (double)(2 * sinl(3.14159265358979323846264338327950288L *
+                                                   (long double)(k * ((c ? 3 : 1) * nx / 4) % (2 * nx)) / (long double)nx));
+    ring_q = dalloc<double>((size_t)ring_ld() * (nx - 1));
+    ring_matrix_kernel<<<dim3((ring_ld() + 127) / 128, nx - 1), 128, 0, st>>>(ring_q, ring_ld(), ring_step(), nx,
+                                                                            plan_x<double>().sn);
+    check_launch();
+    line_w = dalloc<double>(2 * (size_t)nx);
+    CK(cudaMemcpyAsync(line_w, hw.data(), sizeof(double) * 2 * nx, cudaMemcpyHostToDevice, st));
+    // a window's rows: what a curl of faces j0 .. j1 reads, j0 - 1 .. j1
+    std::vector<int> hc(4 * (size_t)L, 0);
+    for (int lev = 1; lev <= L; ++lev) {
+        hc[4 * (lev - 1) + 2] = lev == 1 ? 1 : ny / 4 + 2;
+        hc[4 * (lev - 1) + 3] = lev == 1 ? ny : 3 * ny / 4 - 1;
+    }
+    central_win = dalloc<int>(4 * (size_t)L);
+    CK(cudaMemcpyAsync(central_win, hc.data(), sizeof(int) * 4 * L, cudaMemcpyHostToDevice, st));
+
     // _init_body_motion! (src/bodies.jl:33-41): static bodies take their panels now.
     std::vector<double> hxb(2 * (size_t)np, 0.0), hds(np, 0.0);
     for (int b = 0; b < nbody; ++b)
@@ -1084,12 +1294,12 @@ void Engine<T>::setup() {
         if (body_kind[b] == IBPM_BODY_STATIC) update_weights(body_start[b], body_start[b + 1]);
     check_region_error();
     // pass shapes for one level and for all levels at once
-    tune_ypass<T>(t1, t1, 1);
-    if (L > 1) tune_ypass<T>(t1, t1, L);
+    tune_ypass<T>(t1, 1);
+    if (L > 1) tune_ypass<T>(t1, L);
     if (static_bodies) {
         compute_bbox();
         if (std::is_same<T, double>::value) {
-            if (kbatch > L) tune_ypass<T>(t1, t1, kbatch);
+            if (kbatch > L) tune_ypass<T>(t1, kbatch);
             build_Binv();
             shrink_batch_buffers();
         } else {
@@ -1099,6 +1309,7 @@ void Engine<T>::setup() {
             ibpm_options o64 = opt;
             o64.precision = IBPM_FP64;
             e64.init(&problem_copy, o64);
+            e64.by_transforms = true;
             e64.setup();
             const size_t n = 2 * (size_t)np;
             Binv = dalloc<double>(n * n);
@@ -1593,13 +1804,16 @@ void Engine<T>::step_body() {
         check_launch();
         prof_end(pe, IBPM_KCLASS_NONLINEAR, 8.0 * (double)(nq + 4 * ng) * L);
     }
-    trial<T>(rest, Gnew, L, ysolve(MULT_AIMPL, 1, 1), t1);
+    if constexpr (std::is_same<T, double>::value)
+        trial(rest, Gnew, L, ysolve(MULT_AIMPL, 1, 1), t1);
+    else
+        trial_dst(Gold, rest, Gnew, L, coef_lev, t1, t2);
     nc = 1 - nc;  // _cycle!(state.nonlin)
     // couple_surface_rigid (src/coupling.jl:236-250).  The FP32 engine computes the
     // level-1 trial flux that E interpolates in FP64: B^-1 amplifies white noise in
     // E qs by its condition number (1e4..1e5), FP32 rounding would reach the forces.
     if (hi_level1) {
-        vort2flux(psi, qs1, Gnew, 0, 0, 1, false, true);
+        vort2flux(psi, qs1, Gnew, 0, 0, 1, false, true, nullptr, false, P.bbox);
         launch_regT(P, qs1_hi, 0, Ftmp, 0, 1, 1, prm, g, st);
     } else {
         vort2flux(psi, qs1, Gnew, 0, 0, 1, false, false, P.bbox);  // E reads the bbox only
@@ -1697,8 +1911,8 @@ void Engine<T>::step_body() {
     }
     // project_circ (src/coupling.jl:218-230): Gamma = Gamma_s; Gamma_1 -= Ainv_1 rot(E^T F~b)
     reg_patch(Fbt, 1);
-    xpass(InRegRot<T>{Patch<T>{patch, P.bbox, patch_stride}}, out_scratch(t1), 1, P.bbox, 1);
-    ypass(t1, t1, 1, ysolve(MULT_AIMPL, 1, 0));
+    xpass(InRegRot<T>{Patch<T>{patch, P.bbox, patch_stride}}, out_scratch(t1), 1, XOpt{P.bbox, 1, 0, 1});
+    yimp(t1, 1);
     xpass(in_scratch(t1), OutSub<T>{Gnew, ng, nx - 1}, 1);
     // vort2flux!(state.psi, state.q, state.Gamma)
     vort2flux(psi, q, Gnew, 0, 0, 1, true);
@@ -1734,8 +1948,8 @@ void Engine<T>::step_body_l1d() {
         nonlinear_kernel<T, T, true><<<grd, blk, 0, st>>>(a);
         check_launch();
     }
-    trial<double>(rest1, G1n, 1, ysolve(MULT_AIMPL, 1, 0), t1d);
-    if (L > 1) trial<T>(rest + ng, Gnew + ng, L - 1, ysolve(MULT_AIMPL, 2, 1), t1);
+    trial_dst<double>(G1o, rest1, G1n, 1, coef_lev, t1d, t2d);
+    if (L > 1) trial_dst(Gold + ng, rest + ng, Gnew + ng, L - 1, coef_lev + 1, t1, t2);
     nc = 1 - nc;  // _cycle!(state.nonlin)
     // couple_surface_rigid from the FP64 level-1 trial flux
     vort2flux_l1d(G1n, Gnew, nullptr, psi1_hi, qs1_hi, false);
@@ -1751,8 +1965,8 @@ void Engine<T>::step_body_l1d() {
     launch_reg_patch<double>(P, Fbt, 2 * np, patch_d, patch_stride, 1, g, st);
     check_launch();
     xpass<double>(InRegRot<double>{Patch<double>{patch_d, P.bbox, patch_stride}}, OutPlain<double>{t1d, nt, ldt}, 1,
-                  P.bbox, 1);
-    ypass<double>(t1d, t1d, 1, ysolve(MULT_AIMPL, 1, 0));
+                  XOpt{P.bbox, 1, 0, 1});
+    yimp(t1d, 1);
     xpass<double>(InPlain<double>{t1d, nt, ldt}, OutSub<double>{G1n, ng, nx - 1}, 1);
     // vort2flux!(state.psi, state.q, state.Gamma)
     vort2flux_l1d(G1n, Gnew, q, psi1, q1, true);
@@ -1782,20 +1996,21 @@ void Engine<T>::vort2flux_l1d(const double *G1v, T *Gm, T *qout, double *psi1_ou
             xpass(in_plain(Gl, 0), out_scratch(t1), 1);
         else
             xpass(InBC<T>{Gl, psi + lev * ng, 0, 0, g}, out_scratch(t1), 1);
-        ypass(t1, t1, 1, ysolve(MULT_LAPINV, 1, 0));
+        ylap(t1, 1);
         xpass(in_scratch(t1), out_plain(Pl, 0), 1);
-        if (curl_all) {
-            curl_kernel<T, T, T><<<qgrd, qblk, 0, st>>>(qout + (lev - 1) * nq, 0, Pl, 0,
-                                                        lev < L ? psi + lev * ng : nullptr, 0, g);
-            check_launch();
-        }
+    }
+    if (curl_all && L > 1) {
+        curl_kernel<T, T, T><<<dim3(qgrd.x, qgrd.y, L - 1), qblk, 0, st>>>(qout + nq, nq, psi + ng, ng,
+                                                                          L > 2 ? psi + 2 * ng : nullptr, ng, g, nullptr,
+                                                                          L - 1);
+        check_launch();
     }
     const T *coarse = L > 1 ? psi + ng : nullptr;
     if (coarse)
         xpass<double>(InBC<double, T>{G1v, coarse, 0, 0, g}, OutPlain<double>{t1d, nt, ldt}, 1);
     else
         xpass<double>(InPlain<double>{G1v, 0, nx - 1}, OutPlain<double>{t1d, nt, ldt}, 1);
-    ypass<double>(t1d, t1d, 1, ysolve(MULT_LAPINV, 1, 0));
+    ylap(t1d, 1);
     xpass<double>(InPlain<double>{t1d, nt, ldt}, OutPlain<double>{psi1_out, ng, nx - 1}, 1);
     curl_kernel<double, double, T><<<qgrd, qblk, 0, st>>>(q1_out, 0, psi1_out, 0, coarse, 0, g);
     check_launch();
@@ -2253,7 +2468,10 @@ void Engine<T>::diag_solve(int op, int level, const double *b, double *x) {
         yexpl_kernel<T><<<dim3((nx + 30) / 32, (ny + 6) / 8), dim3(32, 8), 0, st>>>(t1, y, ldt, nx, ny, coef(level), cx);
         check_launch();
     } else {
-        ypass(t1, y, 1, ysolve(mode, level, 0));
+        if (mode == MULT_LAPINV)
+            ylap(t1, 1);
+        else
+            yimp(t1, 1, level);
     }
     xpass(in_scratch(y), out_plain(sol, ng), 1);
     download(x, sol, (size_t)ng);
@@ -2343,9 +2561,9 @@ struct CaseGroup {
     int device = 0;
     cudaStream_t st = nullptr;
     T *q = nullptr, *psi = nullptr, *G[2] = {nullptr, nullptr}, *nl[2] = {nullptr, nullptr};
-    T *t1 = nullptr, *rest = nullptr, *qs1 = nullptr;
+    T *t1 = nullptr, *t2 = nullptr, *rest = nullptr, *qs1 = nullptr;
     double *t1_hi = nullptr, *psi1_hi = nullptr, *qs1_hi = nullptr;
-    double *re_tab = nullptr;
+    double *re_tab = nullptr, *lines = nullptr, *coef_all = nullptr;
     // the implicit diffusion's y-solve tables, case-major (batch b = case L + level - 1)
     YCol *ycols = nullptr;
     double *ydiff = nullptr;
@@ -2409,6 +2627,8 @@ struct CaseGroup {
         nl[0] = alloc<T>(ngL * C);
         nl[1] = alloc<T>(ngL * C);
         t1 = alloc<T>((size_t)(e0->nt * L) * C);
+        lines = alloc<double>((size_t)e0->line_len() * C);
+        if (!std::is_same<T, double>::value) t2 = alloc<T>(ngL * C);
         rest = alloc<T>(ngL * C);
         qs1 = alloc<T>((size_t)nq * C);
         if (e0->hi_level1) {
@@ -2423,7 +2643,7 @@ struct CaseGroup {
             re[c] = cs[c]->g.Re;
             for (int lev = 1; lev <= L; ++lev) ca[(size_t)c * L + lev - 1] = cs[c]->coef(lev);
         }
-        double *coef_all = alloc<double>(ca.size());
+        coef_all = alloc<double>(ca.size());
         re_tab = alloc<double>(C);
         ycols = alloc<YCol>((size_t)(e0->nx - 1) * C * L);
         ydiff = alloc<double>((size_t)kYDiff * C * L);
@@ -2442,7 +2662,7 @@ struct CaseGroup {
         }
         CK(cudaMemcpyAsync(views, hv.data(), sizeof(CaseView) * C, cudaMemcpyHostToDevice, st));
         CK(cudaStreamSynchronize(st));
-        e0->template tune_ypass<T>(t1, t1, C);  // the group's Y passes cover C fields
+        e0->template tune_ypass<T>(t1, C);  // the group's Y passes cover C fields
         // move every case's state into its slot and point the case there
         for (int c = 0; c < C; ++c) {
             Engine<T> &e = *cs[c];
@@ -2534,15 +2754,20 @@ struct CaseGroup {
         Engine<T> &e;
         cudaStream_t st;
         T *t1;
-        double *t1_hi, *psi1_hi, *qs1_hi;
+        int t1_fields;
+        double *lines, *t1_hi, *psi1_hi, *qs1_hi;
         Borrow(Engine<T> &e_, CaseGroup &gr) : e(e_) {
             st = e.st;
             t1 = e.t1;
+            t1_fields = e.t1_fields;
+            lines = e.lines;
             t1_hi = e.t1_hi;
             psi1_hi = e.psi1_hi;
             qs1_hi = e.qs1_hi;
             e.st = gr.st;
             e.t1 = gr.t1;
+            e.t1_fields = gr.L * gr.C;
+            e.lines = gr.lines;
             e.t1_hi = gr.t1_hi;
             e.psi1_hi = gr.psi1_hi;
             e.qs1_hi = gr.qs1_hi;
@@ -2550,6 +2775,8 @@ struct CaseGroup {
         ~Borrow() {
             e.st = st;
             e.t1 = t1;
+            e.t1_fields = t1_fields;
+            e.lines = lines;
             e.t1_hi = t1_hi;
             e.psi1_hi = psi1_hi;
             e.qs1_hi = qs1_hi;
@@ -2570,9 +2797,12 @@ struct CaseGroup {
             nonlinear_kernel<T, T, true><<<grd, blk, 0, st>>>(a);
             e.check_launch();
         }
-        e.template trial<T>(rest, Gnew, C * L, ysolve(1), t1);
+        if constexpr (std::is_same<T, double>::value)
+            e.trial(rest, Gnew, C * L, ysolve(1), t1);
+        else
+            e.trial_dst(Gold, rest, Gnew, C * L, coef_all, t1, t2);
         nc = 1 - nc;
-        e.vort2flux(psi, e.hi_level1 ? nullptr : qs1, Gnew, bsG, nq, C, false, e.hi_level1, nullptr);
+        e.vort2flux(psi, e.hi_level1 ? nullptr : qs1, Gnew, bsG, nq, C, false, e.hi_level1, nullptr, false, bbox_tab, 4);
         // per case, one launch over all cases each: E qs, F~b = B^-1 Ftmp,
         // update_vars!, E^T F~b and the X pass of its rot (zero outside each case's window)
         if (e.hi_level1)
@@ -2587,9 +2817,13 @@ struct CaseGroup {
         e.check_launch();
         launch_reg_patch_multi<T>(views, C, e.g, st);
         e.check_launch();
-        e.xpass(InRegRotTab<T>{views}, e.out_scratch(t1), C, bbox_tab, 1, 4);
+        e.xpass(InRegRotTab<T>{views}, e.out_scratch(t1), C,
+                typename Engine<T>::XOpt{bbox_tab, 1, 4, C});
         // project_circ's solve at level 1 of every case, then vort2flux!
-        e.ypass(t1, t1, C, ysolve(L));
+        if constexpr (std::is_same<T, double>::value)
+            e.ypass(t1, C, ysolve(L));
+        else
+            e.ypass_dst(t1, C, coef_all, L);
         e.xpass(e.in_scratch(t1), OutSub<T>{Gnew, bsG, e.nx - 1}, C);
         e.vort2flux(psi, q, Gnew, bsG, bsQ, C, true);
         gc = 1 - gc;

@@ -6,6 +6,7 @@
 #include <type_traits>
 #include "common.cuh"
 #include "fft_pow2.cuh"
+#include "tc_dst.h"
 #include "ytri.cuh"
 
 namespace ibpm {
@@ -36,7 +37,24 @@ struct InPlain {
     }
 };
 
-// Prologue of vort2flux's telescoping solve (src/fluid.jl:194-197):
+// Prologue: levels of several fields, batch b level b % nl (ls apart) of field b / nl.
+// at(b) is the one level as a plain field: the X pass resolves it once per block
+// (the division, left in the load, cost a 1024^2 pass 4 of its 12.7 us).
+template <class T>
+struct InLevels {
+    const T *p;
+    long long bs;
+    int ld, nl;
+    long long ls;
+    __device__ __forceinline__ InPlain<T> at(int b) const { return InPlain<T>{p + (b / nl) * bs + (b % nl) * ls, 0, ld}; }
+};
+template <class In>
+__device__ __forceinline__ const In &resolve(const In &in, int) { return in; }
+template <class T>
+__device__ __forceinline__ InPlain<T> resolve(const InLevels<T> &in, int b) { return in.at(b); }
+
+// Prologue of the telescoping solves that add the boundary values to the field
+// (FP32 levels, tensor-core transforms; src/fluid.jl:194-197):
 // Gamma_tmp = Gamma[:, lev]; apply_bc!(Gamma_tmp, get_bc(psi[:, lev+1]); fac=1)
 // (the coarser level's psi may be of another element type TC)
 template <class T, class TC = T>
@@ -139,21 +157,181 @@ struct OutSub {
     }
 };
 
+// Boundary values of the next finer level (get_bc! of a solved level's psi,
+// src/fluid.jl:278-306) as the finer level's Y solve takes them.  Per batch:
+// 2 nx doubles, the DST along x of the interpolated rows ny/4 and 3 ny/4 (at
+// their kx - 1), then 2 ny doubles, the columns nx/4 and 3 nx/4 by row.
+// A source on the field's outer rows enters its column systems as those two
+// transformed rows, one on its outer columns as two sine-weighted vectors, so
+// the X passes need no boundary values and run for all levels at once.
+//
+// The rows' way from the solved scratch field (kx, y) to there is linear:
+// back along x, the centre part interpolated, and along x again.  Q is that
+// operator as a matrix (ring_matrix_kernel), so a few warps form both rows as dot
+// products.  As two transforms in one block, one after the other, they were the
+// length of every kernel that held them: 11 us of a 17 us one at 1024 points.
+struct RingOut {
+    double *lines = nullptr;
+    long long stride = 0;
+    int nx = 0, ny = 0;
+    const double *Q = nullptr;  // row kx - 1, qld entries
+    int qld = 0, step = 1;      // step 2: only modes of kx's parity couple (nx a multiple of 4)
+};
+
+// One output mode per call: kx - 1 = k of both rows of batches b .. b + F - 1, by
+// the calling warp: an entry of Q is read once for all of them.
+template <int F, class In>
+__device__ __forceinline__ void ring_mode_f(const In &in, int b, const RingOut &ro, int k) {
+    const int lane = threadIdx.x & 31, jb = ro.ny / 4, jt = 3 * ro.ny / 4;
+    const int m0 = ro.step == 2 ? (k & 1) + 1 : 1;  // first input mode
+    const int nm = ro.step == 2 ? (ro.nx - m0 + 1) / 2 : ro.nx - 1;
+    const double *__restrict__ row = ro.Q + (long long)ro.qld * k;
+    double sb[F] = {}, st[F] = {};
+#pragma unroll(8 / F)
+    for (int q = lane; q < nm; q += 32) {
+        const int m = m0 + q * ro.step;
+        const double w = __ldg(&row[q]);
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+            sb[f] = fma(w, in(b + f, m, jb), sb[f]);
+            st[f] = fma(w, in(b + f, m, jt), st[f]);
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            sb[f] += __shfl_xor_sync(0xffffffffu, sb[f], o);
+            st[f] += __shfl_xor_sync(0xffffffffu, st[f], o);
+        }
+        if (lane == 0) {
+            double *dst = ro.lines + (b + f) * ro.stride + k;
+            dst[0] = sb[f];
+            dst[ro.nx] = st[f];
+        }
+    }
+}
+// the batches b .. b + kRingF - 1 of nb, for b a multiple of kRingF
+constexpr int kRingF = 4;
+template <class In>
+__device__ __forceinline__ void ring_mode(const In &in, int b, int nb, const RingOut &ro, int k) {
+    if (b % kRingF != 0) return;
+    if (b + kRingF <= nb) {
+        ring_mode_f<kRingF>(in, b, ro, k);
+    } else {
+        for (; b < nb; ++b) ring_mode_f<1>(in, b, ro, k);
+    }
+}
+// Q[k][q] = sum_i 2 sin(pi kx i / nx) ring_i(m), ring_i(m) the mode m interpolated
+// to the finer level's boundary point i (sn: sin(pi j / nx), j <= nx).
+static __global__ void ring_matrix_kernel(double *Q, int qld, int step, int nx, const double *__restrict__ sn) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y, kx = k + 1;
+    const int m = step == 2 ? (k & 1) + 1 + 2 * q : q + 1;
+    if (q >= qld) return;
+    double acc = 0.0;
+    if (m < nx) {
+        auto sine = [&](int a) {  // sin(pi a / nx), a >= 0
+            a %= 2 * nx;
+            return a <= nx ? __ldg(&sn[a]) : -__ldg(&sn[2 * nx - a]);
+        };
+        double lo = 2 * sine(m * (nx / 4));
+        for (int c = 1; c <= nx / 2; ++c) {  // coarse point nx/4 + c: boundary points 2c - 1 and 2c
+            const double hi = 2 * sine(m * (nx / 4 + c));
+            acc = fma(2 * sine(kx * (2 * c - 1)), 0.5 * (hi + lo), acc);
+            if (2 * c < nx) acc = fma(2 * sine(kx * (2 * c)), hi, acc);
+            lo = hi;
+        }
+    }
+    Q[(long long)qld * k + q] = acc;
+}
+
+// A solved coarse level reduced to what the finer level reads: one warp per row j
+// in ny/4 .. ny/4 + ny/2 for the columns psi(nx/4, j) and psi(3 nx/4, j) as
+// weighted sums over kx (wl, wr: 2 sin(pi kx i / nx), RODFT00's factor), one per
+// mode of the rows.  The chain from level to level waits for this (4.5 us for one
+// 1024^2 FP64 level) and not for the level's last X pass (8.7 us), which runs for
+// all levels at once after it, or not at all where only the level-1 flux is
+// wanted.  psi (may be null; batch stride pbs): where a window
+// (win + win_stride b, or everywhere if null) reaches the domain's boundary, whose
+// faces a curl takes from the coarser level, the first block also stores those two
+// rows and the others the two columns of psi.
+template <class D>
+__global__ void __launch_bounds__(64)
+    xlines_kernel(InPlain<typename D::Real> in, RingOut ro, PlanT<typename D::Real> pl, const double *__restrict__ wl,
+                  const double *__restrict__ wr, typename D::Real *psi, long long pbs, const int *__restrict__ win,
+                  int win_stride) {
+    using T = typename D::Real;
+    using C = typename D::C;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int b = blockIdx.y, t = threadIdx.x, bx = (int)blockIdx.x - 1;
+    if (psi != nullptr && win != nullptr) {
+        const int *w = win + b * win_stride;
+        if (w[0] > 1 && w[1] < ro.nx && w[2] > 1 && w[3] < ro.ny) psi = nullptr;
+    }
+    if (bx < 0) {
+        if (psi == nullptr) return;
+        psi += b * pbs;
+        C *buf = reinterpret_cast<C *>(smem_raw) + (t / D::TPF) * D::smem_len(pl.M);
+        double2 *wt = reinterpret_cast<double2 *>(smem_raw + scratch_offset<D>(pl.M, 64 / D::TPF)) + D::NWARP * (t / D::TPF);
+        const int jb = ro.ny / 4, jt = 3 * ro.ny / 4, tt = t % D::TPF;  // every group holds the same line
+        for (int i = tt; i <= pl.M; i += D::TPF)
+            buf[D::idx(i)] = i >= 1 && i < pl.M ? Cx<T>::make((T)in(b, i, jb), (T)in(b, i, jt)) : Cx<T>::make(0, 0);
+        __syncthreads();
+        D::dst(buf, pl, tt, wt);
+        if (t < D::TPF)
+            for (int i = 1 + tt; i < pl.M; i += D::TPF) {
+                const C y = buf[D::idx(i)];
+                psi[(i - 1) + (long long)(pl.M - 1) * (jb - 1)] = y.x;
+                psi[(i - 1) + (long long)(pl.M - 1) * (jt - 1)] = y.y;
+            }
+        return;
+    }
+    const int task = bx * 2 + (t >> 5), ncol = ro.ny / 2 + 1;
+    if (task >= ncol) {
+        if (task - ncol < ro.nx - 1) ring_mode(in, b, (int)gridDim.y, ro, task - ncol);
+        return;
+    }
+    const int j = ro.ny / 4 + task;
+    double sl = 0.0, sr = 0.0;
+#pragma unroll 8
+    for (int i = 1 + (t & 31); i < ro.nx; i += 32) {
+        const double v = in(b, i, j);
+        sl = fma(v, __ldg(&wl[i - 1]), sl);
+        sr = fma(v, __ldg(&wr[i - 1]), sr);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        sl += __shfl_xor_sync(0xffffffffu, sl, o);
+        sr += __shfl_xor_sync(0xffffffffu, sr, o);
+    }
+    if ((t & 31) == 0) {
+        double *col = ro.lines + b * ro.stride + 2 * ro.nx + (j - 1);
+        col[0] = (double)(T)sl;
+        col[ro.ny] = (double)(T)sr;
+        if (psi != nullptr && j != ro.ny / 4 && j != 3 * ro.ny / 4) {  // those rows are the first block's
+            T *row = psi + b * pbs + (long long)(ro.nx - 1) * (j - 1) - 1;
+            row[ro.nx / 4] = (T)sl;
+            row[3 * ro.nx / 4] = (T)sr;
+        }
+    }
+}
+
 // X pass: DST along x of rows (ja, jb) = (2p+1, 2p+2) of each batch field.
 // D is the line transform (Pow2Dst<M> or GenericDst); NG line pairs per block.
-// rows (device, may be null): the body's face window i0, i1, j0, j1 (batch b's
-// at rows + b rows_stride).  A block
+// rows (device, may be null): a face window i0, i1, j0, j1 (batch b's at rows +
+// (b % rows_mod) rows_stride).  A block
 // none of whose rows lies in j0-1 .. j1 returns at once: with zero_outside = 0
 // its output rows stay unwritten (the rows a curl of those faces reads lie
 // inside), with zero_outside = 1 it writes them as zeros (the transform of the
 // input's zero rows: rot of a patch inside the window is zero outside them).
 template <class D, int NG, class In, class Out>
 __global__ void __launch_bounds__(D::TPF *NG, D::OCC / (D::TPF * NG))
-    xpass_kernel(In in, Out out, PlanT<typename D::Real> pl, int nrows, const int *__restrict__ rows = nullptr,
-                 int zero_outside = 0, int rows_stride = 0) {
+    xpass_kernel(In inp, Out out, PlanT<typename D::Real> pl, int nrows, const int *__restrict__ rows = nullptr,
+                 int zero_outside = 0, int rows_stride = 0, int rows_mod = 1) {
+    const int bx = blockIdx.x;
     if (rows != nullptr) {  // uniform over the block: before any barrier
-        rows += (long long)rows_stride * blockIdx.y;
-        const int r0 = 2 * NG * (int)blockIdx.x + 1, r1 = r0 + 2 * NG - 1;
+        rows += (long long)rows_stride * (blockIdx.y % rows_mod);
+        const int r0 = 2 * NG * bx + 1, r1 = r0 + 2 * NG - 1;
         if (r1 < rows[2] - 1 || r0 > rows[3]) {
             if (zero_outside) {
                 const int t = threadIdx.x % D::TPF, ja = r0 + 2 * (int)(threadIdx.x / D::TPF);
@@ -174,7 +352,8 @@ __global__ void __launch_bounds__(D::TPF *NG, D::OCC / (D::TPF * NG))
     C *buf = smem + g * G;
     double2 *wt = reinterpret_cast<double2 *>(smem_raw + scratch_offset<D>(M, NG)) + D::NWARP * g;
     const int b = blockIdx.y;
-    const int pair = blockIdx.x * NG + g;
+    const auto in = resolve(inp, b);
+    const int pair = bx * NG + g;
     const int ja = 2 * pair + 1, jb = 2 * pair + 2;
     const bool va = ja <= nrows, vb = jb <= nrows;
     if constexpr (D::MC > 0) {
@@ -234,6 +413,300 @@ __global__ void __launch_bounds__(D::TPF *NG, D::OCC / (D::TPF * NG))
     }
 }
 
+// Y pass by transforms: for each column i, x[i, :] = DST_y(mult(i, :) * DST_y(in[i, :])),
+// Laplacian inverse (coef null) or implicit diffusion of coefficients coef[b coef_stride].
+// A block owns 2*NG adjacent columns; loads and stores are row-coalesced; in
+// place or not.  The FP32 engine's solves: the direct solve (ytri.cuh) is faster
+// and closer to 64 bits for them too, but an FP32 run is reproducible only bit for
+// bit (one changed rounding draws the transforms' noise anew, 1e-5 of the
+// vorticity in ten steps and 1e-4..1e-3 of the forces), so that engine keeps its
+// order of operations, its FP64 level-1 solves and B^-1 included.
+template <class D, int NG>
+__global__ void __launch_bounds__(D::TPF *NG, D::OCC / (D::TPF * NG))
+    ypass_kernel(const typename D::Real *in, typename D::Real *out, long long bs, int ld, int ncols,
+                 PlanT<typename D::Real> pl, const double *__restrict__ coef, int coef_stride,
+                 const double *__restrict__ cx, const double *__restrict__ cy, double scale) {
+    using T = typename D::Real;
+    using C = typename D::C;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *smem = reinterpret_cast<C *>(smem_raw);
+    constexpr int TPF = D::TPF;
+    const int M = pl.M;
+    const int G = D::smem_len(M);
+    const int g = threadIdx.x / TPF, t = threadIdx.x % TPF;
+    C *buf = smem + g * G;
+    double2 *wt = reinterpret_cast<double2 *>(smem_raw + scratch_offset<D>(M, NG)) + D::NWARP * g;
+    const int b = blockIdx.y;
+    const int c0 = blockIdx.x * 2 * NG;  // 0-based first column of the block
+    const T *src = in + b * bs;
+    T *dst = out + b * bs;
+    constexpr int W = 2 * NG;
+    if constexpr (D::MC > 0) {
+        // compile-time trip count, loads issued in chunks of CH before their stores
+        constexpr int NT = NG * TPF;
+        constexpr int NIT = (W * (D::MC + 1) + NT - 1) / NT;
+        constexpr int CH = 12;
+#pragma unroll
+        for (int k0 = 0; k0 < NIT; k0 += CH) {
+            T v[CH];
+#pragma unroll
+            for (int k = 0; k < CH; ++k) {
+                const int e = threadIdx.x + (k0 + k) * NT;
+                const int c = e % W, jj = e / W;
+                const int col = c0 + c;
+                v[k] = (k0 + k < NIT && jj >= 1 && jj < D::MC && col < ncols) ? src[col + (long long)ld * (jj - 1)]
+                                                                               : (T)0;
+            }
+#pragma unroll
+            for (int k = 0; k < CH; ++k) {
+                const int e = threadIdx.x + (k0 + k) * NT;
+                const int c = e % W, jj = e / W;
+                if (k0 + k < NIT && jj <= D::MC) *(reinterpret_cast<T *>(smem + (c >> 1) * G + D::idx(jj)) + (c & 1)) = v[k];
+            }
+        }
+    } else {
+        for (int e = threadIdx.x; e < W * (M + 1); e += blockDim.x) {
+            const int c = e % W, jj = e / W;
+            const int col = c0 + c;
+            T v = 0;
+            if (jj >= 1 && jj < M && col < ncols) v = src[col + (long long)ld * (jj - 1)];
+            T *slot = reinterpret_cast<T *>(smem + (c >> 1) * G + D::idx(jj)) + (c & 1);
+            *slot = v;
+        }
+    }
+    __syncthreads();
+    // DST, spectral multiply, DST; one loop body so the transform is emitted once
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+        D::dst(buf, pl, t, wt);
+        if (pass == 1) break;
+        const int ia = c0 + 2 * g + 1, ib = c0 + 2 * g + 2;  // 1-based columns
+        const double cb = coef ? coef[b * coef_stride] : 0.0;
+        auto factor = [&](double cxi, double cyj) -> double {
+            const double lam = -2 * ((cxi + cyj) - 2);
+            return scale * recip(coef ? 1 + lam * cb : lam);
+        };
+        if constexpr (D::MC > 0) {
+            constexpr int NIT = (D::MC - 1 + TPF - 1) / TPF;
+            const double cxa = ia <= ncols ? __ldg(&cx[ia]) : 0.0, cxb = ib <= ncols ? __ldg(&cx[ib]) : 0.0;
+            double cyv[NIT];
+#pragma unroll
+            for (int k = 0; k < NIT; ++k) {
+                const int jj = 1 + t + k * TPF;
+                cyv[k] = jj < D::MC ? __ldg(&cy[jj]) : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < NIT; ++k) {
+                const int jj = 1 + t + k * TPF;
+                if (jj >= D::MC) break;
+                C y = buf[D::idx(jj)];
+                y.x = (T)(y.x * ((ia <= ncols) ? factor(cxa, cyv[k]) : 0.0));
+                y.y = (T)(y.y * ((ib <= ncols) ? factor(cxb, cyv[k]) : 0.0));
+                buf[D::idx(jj)] = y;
+            }
+        } else {
+            for (int jj = 1 + t; jj < M; jj += TPF) {
+                C y = buf[D::idx(jj)];
+                y.x = (T)(y.x * ((ia <= ncols) ? factor(__ldg(&cx[ia]), __ldg(&cy[jj])) : 0.0));
+                y.y = (T)(y.y * ((ib <= ncols) ? factor(__ldg(&cx[ib]), __ldg(&cy[jj])) : 0.0));
+                buf[D::idx(jj)] = y;
+            }
+        }
+        __syncthreads();
+    }
+    for (int e = threadIdx.x; e < W * (M + 1); e += blockDim.x) {
+        const int c = e % W, jj = e / W;
+        const int col = c0 + c;
+        if (jj >= 1 && jj < M && col < ncols) {
+            const T *slot = reinterpret_cast<const T *>(smem + (c >> 1) * G + D::idx(jj)) + (c & 1);
+            dst[col + (long long)ld * (jj - 1)] = *slot;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Merged trial solve of get_trial_state (src/fluid.jl:485-496) by transforms:
+//   Gamma_s = Ainv (A Gamma + rest),  rest = dt (1.5 N1 - 0.5 N2) + rhsbc.
+// With S the 2D DST-I and S S = 1/scale:  S(A Gamma) = S(Gamma) / Lambda_e, so
+//   Gamma_s = S( scale / Lambda_i * ( S(Gamma) / Lambda_e + S(rest) ) ),
+// three passes instead of the reference's four transforms in six passes.  The FP32
+// engine's; the FP64 engine takes A Gamma from the nonlinear kernel's stencil and
+// one field through the general passes (84 against 220 us at 1024^2 x 5).
+// ---------------------------------------------------------------------------
+
+// X pass: row j of level b as one complex line z = Gamma + i rest.
+template <class D, int NG>
+__global__ void __launch_bounds__(D::TPF *NG, D::OCC / (D::TPF * NG))
+    xpass_trial_kernel(const typename D::Real *__restrict__ gam, const typename D::Real *__restrict__ rest,
+                       typename D::Real *__restrict__ t1, typename D::Real *__restrict__ t2, long long bs, int ld,
+                       PlanT<typename D::Real> pl, int nrows) {
+    using T = typename D::Real;
+    using C = typename D::C;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *smem = reinterpret_cast<C *>(smem_raw);
+    constexpr int TPF = D::TPF;
+    const int M = pl.M;
+    const int G = D::smem_len(M);
+    const int g = threadIdx.x / TPF, t = threadIdx.x % TPF;
+    C *buf = smem + g * G;
+    double2 *wt = reinterpret_cast<double2 *>(smem_raw + scratch_offset<D>(M, NG)) + D::NWARP * g;
+    const int b = blockIdx.y;
+    const int j = blockIdx.x * NG + g + 1;
+    const bool valid = j <= nrows;
+    const long long row = b * bs + (long long)ld * (j - 1);
+    if constexpr (D::MC > 0) {
+        constexpr int NIT = (D::MC + 1 + TPF - 1) / TPF;
+        T za[NIT], zb[NIT];
+#pragma unroll
+        for (int k = 0; k < NIT; ++k) {
+            const int i = t + k * TPF;
+            const bool ok = valid && i >= 1 && i < D::MC;
+            za[k] = ok ? gam[row + i - 1] : (T)0;
+            zb[k] = ok ? rest[row + i - 1] : (T)0;
+        }
+#pragma unroll
+        for (int k = 0; k < NIT; ++k) {
+            const int i = t + k * TPF;
+            if (i <= D::MC) buf[D::idx(i)] = Cx<T>::make(za[k], zb[k]);
+        }
+    } else {
+        for (int i = t; i <= M; i += TPF) {
+            C z = Cx<T>::make(0, 0);
+            if (valid && i >= 1 && i < M) z = Cx<T>::make(gam[row + i - 1], rest[row + i - 1]);
+            buf[D::idx(i)] = z;
+        }
+    }
+    __syncthreads();
+    D::dst(buf, pl, t, wt);
+    if (valid)
+        for (int i = 1 + t; i < M; i += TPF) {
+            const C y = buf[D::idx(i)];
+            t1[row + i - 1] = y.x;
+            t2[row + i - 1] = y.y;
+        }
+}
+
+// Y pass: a block owns 2NG adjacent columns.  Phase 1 transforms each column's
+// (S_x Gamma, S_x rest) pair as one complex line and combines
+//   v = scale / Lambda_i * (S Gamma / Lambda_e + S rest)
+//     = (S Gamma (1 - lam c) + S rest) * scale / (1 + lam c),   c = dt / (2 Re hc^2);
+// phase 2 transforms the real v of two columns packed as one complex line (out may
+// be t1: a block reads its columns whole before it stores them).
+// Resident threads per SM the kernel is compiled for: 512 for FP32 lines of up to
+// 512 points (at most 128 registers a thread), 256 otherwise.
+template <class D>
+constexpr int trial_occ() {
+    return (sizeof(typename D::Real) == 4 && D::MC > 0 && D::MC <= 512) ? 512 : 256;
+}
+template <class D, int NG>
+__global__ void __launch_bounds__(D::TPF *NG, trial_occ<D>() / (D::TPF * NG))
+    ypass_trial_kernel(const typename D::Real *t1, const typename D::Real *__restrict__ t2, typename D::Real *out,
+                       long long bs, int ncols, PlanT<typename D::Real> pl, const double *__restrict__ coef,
+                       const double *__restrict__ cx, const double *__restrict__ cy, double scale) {
+    using T = typename D::Real;
+    using C = typename D::C;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *smem = reinterpret_cast<C *>(smem_raw);
+    constexpr int TPF = D::TPF;
+    constexpr int W = 2 * NG;
+    const int M = pl.M;
+    const int G = D::smem_len(M);
+    const int g = threadIdx.x / TPF, t = threadIdx.x % TPF;
+    double2 *wt = reinterpret_cast<double2 *>(smem_raw + scratch_offset<D>(M, W)) + D::NWARP * g;
+    const int b = blockIdx.y;
+    const int c0 = blockIdx.x * W;  // 0-based first column
+    const T *s1 = t1 + b * bs, *s2 = t2 + b * bs;
+    T *dst = out + b * bs;
+    if constexpr (D::MC > 0) {
+        constexpr int NT = NG * TPF;
+        constexpr int NIT = (W * (D::MC + 1) + NT - 1) / NT;
+        constexpr int CH = 8;
+#pragma unroll
+        for (int k0 = 0; k0 < NIT; k0 += CH) {
+            T va[CH], vb[CH];
+#pragma unroll
+            for (int k = 0; k < CH; ++k) {
+                const int e = threadIdx.x + (k0 + k) * NT;
+                const int c = e % W, jj = e / W;
+                const int col = c0 + c;
+                const bool ok = k0 + k < NIT && jj >= 1 && jj < D::MC && col < ncols;
+                const long long o = col + (long long)ncols * (jj - 1);
+                va[k] = ok ? s1[o] : (T)0;
+                vb[k] = ok ? s2[o] : (T)0;
+            }
+#pragma unroll
+            for (int k = 0; k < CH; ++k) {
+                const int e = threadIdx.x + (k0 + k) * NT;
+                const int c = e % W, jj = e / W;
+                if (k0 + k < NIT && jj <= D::MC) smem[c * G + D::idx(jj)] = Cx<T>::make(va[k], vb[k]);
+            }
+        }
+    } else
+    for (int e = threadIdx.x; e < W * (M + 1); e += blockDim.x) {
+        const int c = e % W, jj = e / W;
+        const int col = c0 + c;
+        C z = Cx<T>::make(0, 0);
+        if (jj >= 1 && jj < M && col < ncols) {
+            const long long o = col + (long long)ncols * (jj - 1);
+            z = Cx<T>::make(s1[o], s2[o]);
+        }
+        smem[c * G + D::idx(jj)] = z;
+    }
+    __syncthreads();
+    const double cb = coef[b];
+#pragma unroll 1
+    for (int r = 0; r < 2; ++r) {
+        const int c = r * NG + g;
+        C *buf = smem + c * G;
+        D::dst(buf, pl, t, wt);
+        const int col1 = c0 + c + 1;  // 1-based column
+        const bool ok = col1 <= ncols;
+        const double cxv = ok ? __ldg(&cx[col1]) : 0.0;
+        auto combine = [&](int jj, double cyj) {
+            const C y = buf[D::idx(jj)];
+            double v = 0.0;
+            if (ok) {
+                const double lam = -2 * ((cxv + cyj) - 2);
+                v = ((double)y.x * (1 - lam * cb) + (double)y.y) * (scale * recip(1 + lam * cb));
+            }
+            buf[D::idx(jj)] = Cx<T>::make((T)v, 0);
+        };
+        if constexpr (D::MC > 0) {
+            constexpr int NIT = (D::MC - 1 + TPF - 1) / TPF;
+            double cyv[NIT];
+#pragma unroll
+            for (int k = 0; k < NIT; ++k) {
+                const int jj = 1 + t + k * TPF;
+                cyv[k] = jj < D::MC ? __ldg(&cy[jj]) : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < NIT; ++k) {
+                const int jj = 1 + t + k * TPF;
+                if (jj < D::MC) combine(jj, cyv[k]);
+            }
+        } else {
+            for (int jj = 1 + t; jj < M; jj += TPF) combine(jj, __ldg(&cy[jj]));
+        }
+        __syncthreads();
+    }
+    // phase 2: pack columns (2g, 2g+1) into buffer 2g
+    {
+        C *ba = smem + (2 * g) * G;
+        const C *bb = smem + (2 * g + 1) * G;
+        for (int jj = 1 + t; jj < M; jj += TPF) ba[D::idx(jj)].y = bb[D::idx(jj)].x;
+        __syncthreads();
+        D::dst(ba, pl, t, wt);
+    }
+    for (int e = threadIdx.x; e < W * (M + 1); e += blockDim.x) {
+        const int c = e % W, jj = e / W;
+        const int col = c0 + c;
+        if (jj >= 1 && jj < M && col < ncols) {
+            const C y = smem[(c & ~1) * G + D::idx(jj)];
+            dst[col + (long long)ncols * (jj - 1)] = (c & 1) ? y.y : y.x;
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Stencil kernels
 // ---------------------------------------------------------------------------
@@ -246,7 +719,7 @@ struct NonlinArgs {
     const T *gam;         // ng x L
     T *out;               // ng x L (state.nonlin[1])
     const T *n2;          // ng x L (state.nonlin[2]); with rest != nullptr
-    T *rest;              // ng x L: A Gamma + dt (1.5 N1 - 0.5 N2) + rhsbc, or nullptr
+    T *rest;              // ng x L: dt (1.5 N1 - 0.5 N2) + rhsbc, in the FP64 engine plus A Gamma, or nullptr
     const StepDev *prm;
     Grid g;
     // Ensembles of cases of one shape, stacked case-major (batch b = case L + level - 1):
@@ -412,17 +885,18 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
         const double n1 = r * (1 / (hc * hc));
         a.out[b * ng + GI(I, J)] = (T)n1;
         if (a.rest) {
-            // rest = A Gamma + dt b1 N1 + dt b2 N2 + rhsbc (fluid.jl:487-493), rhsbc =
-            // apply_bc!(0, get_bc(..); fac).  A = 1 - c (-Laplacian), diagonal under the
-            // 2D DST, is this five-point stencil with zeros beyond the field: taking it
-            // here spares the trial solve a second field through its passes
-            const double rc = g.dt / (re_of() * (hc * hc));
-            const double gc = (double)gm[y + 1][x + 1];
-            const double lap = ((double)gm[y + 1][x] + (double)gm[y + 1][x + 2] - 2 * gc) +
-                               ((double)gm[y][x + 1] + (double)gm[y + 2][x + 1] - 2 * gc);
-            double v = (g.dt * 1.5) * n1 + (g.dt * -0.5) * (double)rn[y][x] + (gc + 0.5 * rc * lap);
+            // rest = dt b1 N1 + dt b2 N2 + rhsbc (fluid.jl:487-493), rhsbc = apply_bc!(0, get_bc(..); fac)
+            double v = (g.dt * 1.5) * n1 + (g.dt * -0.5) * (double)rn[y][x];
+            if constexpr (sizeof(T) == 8 && std::is_same<T, TC>::value) {
+                // + A Gamma.  A = 1 - c (-Laplacian), diagonal under the 2D DST, is this
+                // five-point stencil with zeros beyond the field: taking it here spares
+                // the trial solve a second field through its passes
+                const double gc = gm[y + 1][x + 1];
+                const double lap = (gm[y + 1][x] + gm[y + 1][x + 2] - 2 * gc) + (gm[y][x + 1] + gm[y + 2][x + 1] - 2 * gc);
+                v += gc + 0.5 * (g.dt / (re_of() * (hc * hc))) * lap;
+            }
             if (lev < g.L && on_ring(g, I, J)) {
-                const double fac = 0.25 * rc;
+                const double fac = 0.25 * g.dt / (re_of() * (hc * hc));
                 v = v + apply_bc_at(0.0, C, g, I, J, fac);
             }
             a.rest[b * ng + GI(I, J)] = (T)v;
@@ -433,17 +907,20 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
 // 4-argument curl! (src/fluid.jl:230-276) with psi_bc = get_bc(psi_coarse) (zero if null).
 // One thread per (i, j) writes both faces there: the x face u(i, j) (i <= nx+1,
 // j <= ny) and the y face v(i, j) (i <= nx, j <= ny+1); inside the ring they share
-// psi(i-1, j-1).  Batch b (blockIdx.z) uses psi + b*bs, q + b*qbs, coarse + b*cbs.
+// psi(i-1, j-1).  Batch b (blockIdx.z) uses psi + b*bs, q + b*qbs, coarse + b*cbs;
+// with nl > 1 batch b is level b % nl + 1 of nl levels, whose coarsest has no
+// coarser field.
 // win (device, may be null): only the faces in i0..i1 x j0..j1 are written, by a
 // grid of any size sweeping the window.
 template <class T, class TP, class TC>
 __global__ void curl_kernel(T *__restrict__ qout, long long qbs, const TP *__restrict__ psi, long long bs,
-                            const TC *__restrict__ coarse, long long cbs, Grid g, const int *__restrict__ win = nullptr) {
+                            const TC *__restrict__ coarse, long long cbs, Grid g, const int *__restrict__ win = nullptr,
+                            int nl = 1) {
     const int nx = g.nx, ny = g.ny;
     const long long nu = (long long)(nx + 1) * ny;
     const int b = blockIdx.z;
     const TP *Pt = psi + b * bs;
-    const TC *C = coarse ? coarse + b * cbs : nullptr;
+    const TC *C = coarse && (nl == 1 || (b + 1) % nl != 0) ? coarse + b * cbs : nullptr;
     T *q = qout + b * qbs;
     auto P = [&](long long k) -> double { return (double)Pt[k]; };
     auto face = [&](int i, int j) {

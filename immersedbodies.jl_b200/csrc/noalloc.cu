@@ -45,8 +45,9 @@ constexpr int kNoAllocMaxM = 1024;
 constexpr size_t kScratchField = kNoAllocMaxCells + 4 * kNoAllocMaxM;
 // offset of the y solve's tables after the transforms' (a multiple of 16 bytes)
 constexpr size_t kYTables = 2 * (2 * kNoAllocMaxM) + 4 * (kNoAllocMaxM + 1);
-static_assert(sizeof(YCol) == 8 * sizeof(double) && kYTables % 2 == 0 && kYDiff % 2 == 0, "table alignment");
-constexpr size_t kScratchDoubles = kScratchField + kYTables + 8 * kNoAllocMaxM + kYDiff + 2 * (kYChunks + 1) * kYFull;
+constexpr size_t kYColD = sizeof(YCol) / sizeof(double);
+static_assert(sizeof(YCol) == kYColD * sizeof(double) && kYTables % 2 == 0 && kYDiff % 2 == 0, "table alignment");
+constexpr size_t kScratchDoubles = kScratchField + kYTables + kYColD * kNoAllocMaxM + kYDiff + 2 * (kYChunks + 1) * kYFull;
 
 static __device__ __align__(256) double g_scratch[kScratchDoubles];
 
@@ -115,7 +116,7 @@ cudaError_t xpass_na(const PlanT<double> &pl, In in, Out out, int nrows, cudaStr
     constexpr int NG = 2;
     const cudaLaunchConfig_t c =
         launch_cfg(dim3(((nrows + 1) / 2 + NG - 1) / NG, 1), dim3(NG * D::TPF), pass_smem<D>(pl.M, NG, NG), st);
-    return cudaLaunchKernelEx(&c, xpass_kernel<D, NG, In, Out>, in, out, pl, nrows, (const int *)nullptr, 0, 0);
+    return cudaLaunchKernelEx(&c, xpass_kernel<D, NG, In, Out>, in, out, pl, nrows, (const int *)nullptr, 0, 0, 1);
 }
 
 cudaError_t tables_na(double2 *tw, double *sn, double *cs, int M, cudaStream_t st) {
@@ -164,8 +165,8 @@ int ibpm_lap_inv_noalloc(int nx, int ny, const double *b, double *x, void *strea
             e = tables_na(twx, snx, csx, nx, st);
             if (e == cudaSuccess) e = tables_na(twy, sny, csy, ny, st);
             if (e == cudaSuccess)
-                e = launch_ycols(reinterpret_cast<YCol *>(tab + kYTables), tab + kYTables + 8 * kNoAllocMaxM,
-                                 reinterpret_cast<double2 *>(tab + kYTables + 8 * kNoAllocMaxM + kYDiff), csx, csy, nx, ny,
+                e = launch_ycols(reinterpret_cast<YCol *>(tab + kYTables), tab + kYTables + kYColD * kNoAllocMaxM,
+                                 reinterpret_cast<double2 *>(tab + kYTables + kYColD * kNoAllocMaxM + kYDiff), csx, csy, nx, ny,
                                  nullptr, 1, st);
             if (e != cudaSuccess) return fail(IBPM_ERR_CUDA, cudaGetErrorString(e));
             slot.nx = nx;
@@ -179,12 +180,12 @@ int ibpm_lap_inv_noalloc(int nx, int ny, const double *b, double *x, void *strea
     plx.sn = tab + 4 * kNoAllocMaxM;
     ply.sn = plx.sn + (kNoAllocMaxM + 1);
     const YSolve m{reinterpret_cast<const YCol *>(tab + kYTables),
-                   tab + kYTables + 8 * kNoAllocMaxM,
-                   reinterpret_cast<const double2 *>(tab + kYTables + 8 * kNoAllocMaxM + kYDiff), 0, 0};
+                   tab + kYTables + kYColD * kNoAllocMaxM,
+                   reinterpret_cast<const double2 *>(tab + kYTables + kYColD * kNoAllocMaxM + kYDiff), 0, 0};
     using D = GenericDst<double>;
     const int ld = (nx + 3) / 4 * 4;
     cudaError_t e = xpass_na<D>(plx, InPlain<double>{b, 0, nx - 1}, OutPlain<double>{t1, 0, ld}, ny - 1, st);
-    if (e == cudaSuccess) e = launch_ytri<double>(t1, t1, 0, ld, nx - 1, ny, 1, ytri_wshift<double>(nx - 1, ny, 1), m, st);
+    if (e == cudaSuccess) e = launch_ytri(t1, 0, ld, nx - 1, ny, 1, ytri_wshift(nx - 1, 1), m, st);
     if (e == cudaSuccess)
         e = xpass_na<D>(plx, InPlain<double>{t1, 0, ld}, OutPlain<double>{x, 0, nx - 1}, ny - 1, st);
     if (e != cudaSuccess) return fail(IBPM_ERR_CUDA, cudaGetErrorString(e));

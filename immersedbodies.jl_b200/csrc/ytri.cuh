@@ -84,6 +84,15 @@ struct __align__(16) YCol {
     double det;     // 1 / (1 - r^2M)
     double ek;      // r^k, k = rows up to M in the chunk that holds row M
     double ek1;     // r^(k - 1)
+    double sx;      // 2 sin(pi kx / nx): what a unit source on the first column adds
+    double pad;
+};
+// Boundary values from the coarser level (RingOut in kernels.cuh): batch b at
+// lines + b stride
+struct YRing {
+    const double *lines = nullptr;
+    long long stride = 0;
+    int nx = 0, ny = 0;
 };
 // The y solve of one launch: batch b takes cols + b cstride and diff + b dstride.
 struct YSolve {
@@ -94,29 +103,29 @@ struct YSolve {
     long long cstride, dstride;
 };
 
-// In place (out == in) or not; both with leading dimension ld and batch stride
-// bs.  blockDim.x = 64 << wshift, 64 MR >= M.
-template <class T, int MR>
+// In place; leading dimension ld, batch stride bs.  blockDim.x = 64 << wshift,
+// 64 MR >= M.
+// RING: the field's sources on its outer rows and columns are added to b.
+template <int MR, bool RING>
 __global__ void __launch_bounds__(kYChunks *kYMaxW)
-    ytri_kernel(const T *in, T *out, long long bs, int ld, int ncols, int M, int wshift, YSolve ys) {
-    constexpr bool kCorrect = sizeof(T) == 8;  // below FP32 rounding otherwise
+    ytri_kernel(double *f, long long bs, int ld, int ncols, int M, int wshift, YSolve ys, YRing yr) {
     constexpr int kPad = kYMaxW * (kYChunks + 2);
     // chunk totals, then starts of P and Q; r^(row) of the homogeneous terms.  Row
     // stride 64 + 16 / W: the threads' stores and the scan's 16-byte loads are free
     // of bank conflicts
     __shared__ __align__(16) double sP[kPad], sQ[kPad], sA[kPad], sB[kPad];
     __shared__ double sPM[kYMaxW], sQ1[kYMaxW];
-    __shared__ double2 mom[kCorrect ? kYMaxW * kYChunks : 1];
-    __shared__ double modes[kCorrect ? kYMaxW : 1][kYFull];
+    __shared__ double2 mom[kYMaxW * kYChunks];
+    __shared__ double modes[kYMaxW][kYFull];
     const int W = 1 << wshift, tid = threadIdx.x, S = kYChunks + (16 >> wshift);
     const int w = tid & (W - 1), p = tid >> wshift;
     const int c0 = blockIdx.x << wshift, col = c0 + w;  // 0-based column: kx = col + 1
     const int b = blockIdx.y, n = M - 1, j0 = p * MR;   // rows j0+1 .. j0+MR
     const bool valid = col < ncols;
-    const T *src = in + b * bs + col + (long long)ld * j0;
-    T raw[MR];
+    double *src = f + b * bs + col + (long long)ld * j0;
+    double v[MR];
 #pragma unroll
-    for (int k = 0; k < MR; ++k) raw[k] = valid && j0 + k < n ? src[ld * k] : (T)0;
+    for (int k = 0; k < MR; ++k) v[k] = valid && j0 + k < n ? src[ld * k] : 0.0;
     const YCol *cols = ys.cols + b * ys.cstride;
     const double2 rr = *reinterpret_cast<const double2 *>(&cols[valid ? col : 0].rh);
     const double rh = rr.x, rl = rr.y;
@@ -126,24 +135,47 @@ __global__ void __launch_bounds__(kYChunks *kYMaxW)
     const double R = yc.R, ekx = (tid & 32) ? yc.ek1 : yc.ek;
     const double2 ce = *reinterpret_cast<const double2 *>(&cols[valid ? col : 0].eM);
     const double kap = cols[valid ? col : 0].kap;
-    bool correct = false;
     const bool full = n <= kYFull;
     const int nmode = full ? n : min(kYModes, n);
     double2 ph_p = make_double2(0.0, 0.0), ph_t = ph_p, ph_r = ph_p;
-    if constexpr (kCorrect) {
-        correct = c0 < kYModes && __ldg(ys.diff + b * ys.dstride + kYDiff - 1) != 0.0;
-        if (correct) {
-            const int ky = min(tid >> (2 + wshift), kYFull - 1);
-            ph_p = __ldg(&ys.phase[p * kYFull]);
-            ph_t = __ldg(&ys.phase[(tid & 3) * kYFull + ky]);
-            ph_r = __ldg(&ys.phase[kYChunks * kYFull + ky]);
-        }
+    const bool correct = c0 < kYModes && __ldg(ys.diff + b * ys.dstride + kYDiff - 1) != 0.0;
+    if (correct) {
+        const int ky = min(tid >> (2 + wshift), kYFull - 1);
+        ph_p = __ldg(&ys.phase[p * kYFull]);
+        ph_t = __ldg(&ys.phase[(tid & 3) * kYFull + ky]);
+        ph_r = __ldg(&ys.phase[kYChunks * kYFull + ky]);
     }
-    double v[MR];
+    if constexpr (RING) {
+        // the coarse columns' values, interpolated to this chunk's rows: the odd rows
+        // are means of two; the last column's sign alternates with kx
+        const double *hat = yr.lines + b * yr.stride;
+        const double *cl = hat + 2 * yr.nx + M / 4 - 1, *cr = cl + yr.ny;
+        const double sx = cols[valid ? col : 0].sx, sg = (col & 1) ? -sx : sx;
+        if constexpr (MR % 2 == 0) {
+            double q[MR / 2 + 1];
 #pragma unroll
-    for (int k = 0; k < MR; ++k) {
-        v[k] = widen(raw[k]);
-        if constexpr (sizeof(T) == 4) asm("" : "+d"(v[k]));  // converted once: the compiler would repeat it at every use
+            for (int m = 0; m <= MR / 2; ++m) {
+                const int at = j0 / 2 + m;
+                q[m] = at <= M / 2 ? fma(sx, cl[at], sg * cr[at]) : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < MR; ++k)
+                if (j0 + k < n) v[k] += (k & 1) ? q[(k + 1) / 2] : 0.5 * (q[k / 2] + q[k / 2 + 1]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < MR; ++k) {
+                const int j = j0 + k + 1;
+                if (j > n) continue;
+                const double hi = fma(sx, cl[(j + 1) / 2], sg * cr[(j + 1) / 2]);
+                v[k] += (j & 1) ? 0.5 * (hi + fma(sx, cl[j / 2], sg * cr[j / 2])) : hi;
+            }
+        }
+        if (valid) {
+            if (p == 0) v[0] += hat[col];
+#pragma unroll
+            for (int k = 0; k < MR; ++k)
+                if (j0 + k == n - 1) v[k] += hat[yr.nx + col];
+        }
     }
 
     // local recurrences; the owner of row M stops there
@@ -163,7 +195,7 @@ __global__ void __launch_bounds__(kYChunks *kYMaxW)
             m0 += v[k];
             m1 = fma((double)(k - KC), v[k], m1);
         }
-        mom[kCorrect ? p * W + w : 0] = make_double2(m0, m1);
+        mom[p * W + w] = make_double2(m0, m1);
     }
     __syncthreads();
 
@@ -225,7 +257,7 @@ __global__ void __launch_bounds__(kYChunks *kYMaxW)
             double s0 = 0.0, s1 = 0.0;
 #pragma unroll
             for (int q = 0; q < kYChunks / 4; ++q) {
-                const double2 mm = mom[kCorrect ? (q * 4 + part) * W + mw : 0];
+                const double2 mm = mom[(q * 4 + part) * W + mw];
                 s0 = fma(mm.x, ph.x, s0);
                 s1 = fma(mm.y, ph.y, s1);
                 ph = make_double2(fma(ph.x, ph_r.y, ph.y * ph_r.x), fma(ph.y, ph_r.y, -ph.x * ph_r.x));  // 4 chunks on
@@ -261,7 +293,7 @@ __global__ void __launch_bounds__(kYChunks *kYMaxW)
         double e0 = 0.0, e1 = 0.0;
         double2 ph = ph_p;
         for (int ky = 0; ky < nmode; ++ky) {
-            const double a = modes[kCorrect ? w : 0][ky];
+            const double a = modes[w][ky];
             e0 = fma(a, ph.x, e0);
             e1 = fma(a * (ky + 1), ph.y, e1);
             ph = make_double2(fma(ph.x, ph_p.y, ph.y * ph_p.x), fma(ph.y, ph_p.y, -ph.x * ph_p.x));  // next mode
@@ -271,10 +303,9 @@ __global__ void __launch_bounds__(kYChunks *kYMaxW)
         for (int k = 0; k < MR; ++k) x[k] = full ? e0 : x[k] + fma((double)(k - KC), e1, e0);
     }
     if (valid) {
-        T *dst = out + b * bs + col + (long long)ld * j0;
 #pragma unroll
         for (int k = 0; k < MR; ++k)
-            if (j0 + k < n) dst[ld * k] = (T)x[k];
+            if (j0 + k < n) src[ld * k] = x[k];
     }
 }
 
@@ -301,6 +332,8 @@ static __global__ void ycols_kernel(YCol *cols, double *diff, double2 *phase, co
         y.det = -1 / expm1(2 * M * lr);
         y.ek = exp(k * lr);
         y.ek1 = exp((k - 1) * lr);
+        y.sx = 2 * sinpi((double)(q + 1) / nx);
+        y.pad = 0.0;
         cols[(long long)b * (nx - 1) + q] = y;
     }
     const bool full = n <= kYFull;
@@ -351,15 +384,10 @@ __global__ void yexpl_kernel(const T *__restrict__ in, T *__restrict__ out, int 
 }
 
 // Columns per block, as log2, for nbatch fields of ncols columns (measured,
-// 2 / 4 / 8 columns: one 1024^2 FP64 field 8.3 / 6.5 / 10.0 us, five 31.8 /
-// 20.3 / 22.7 us; one 256^2 field 3.7 / 4.3 / 8.0 us, where few blocks leave the
-// correcting ones as the kernel's length; five 1024^2 FP32 fields, whose sectors
-// hold eight columns, 35.5 / 26.2 / 22.7 us).
-template <class T>
-int ytri_wshift(int ncols, int M, int nbatch) {
-    if ((long long)ncols * nbatch < 300) return 1;
-    return sizeof(T) == 4 && M > 512 ? 3 : 2;
-}
+// 2 / 4 / 8 columns: one 1024^2 field 8.3 / 6.5 / 10.0 us, five 31.8 / 20.3 /
+// 22.7 us; one 256^2 field 3.7 / 4.3 / 8.0 us, where few blocks leave the
+// correcting ones as the kernel's length).
+inline int ytri_wshift(int ncols, int nbatch) { return (long long)ncols * nbatch < 300 ? 1 : 2; }
 
 // Rows per thread of a transform length M: the smallest compiled chunk that covers it.
 inline int ytri_rows(int M) {
@@ -380,28 +408,27 @@ inline cudaError_t launch_ycols(YCol *cols, double *diff, double2 *phase, const 
     return cudaLaunchKernelEx(&cfg, ycols_kernel, cols, diff, phase, cx, cy, nx, M, ytri_rows(M), coef);
 }
 
-// Enqueues the Y solve of nbatch fields with 1 << wshift columns a block; the
+// Enqueues the Y solve, in place, of nbatch fields with 1 << wshift columns a block; the
 // return code is the launch's own.
-template <class T>
-cudaError_t launch_ytri(const T *in, T *out, long long bs, int ld, int ncols, int M, int nbatch, int wshift,
-                        const YSolve &ys, cudaStream_t st) {
+inline cudaError_t launch_ytri(double *f, long long bs, int ld, int ncols, int M, int nbatch, int wshift,
+                               const YSolve &ys, cudaStream_t st, const YRing &yr = {}) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((ncols + (1 << wshift) - 1) >> wshift, nbatch);
     cfg.blockDim = dim3(kYChunks << wshift);
     cfg.stream = st;
-    auto go = [&](auto *k) { return cudaLaunchKernelEx(&cfg, k, in, out, bs, ld, ncols, M, wshift, ys); };
+    auto go = [&](auto *k) { return cudaLaunchKernelEx(&cfg, k, f, bs, ld, ncols, M, wshift, ys, yr); };
     switch (ytri_rows(M)) {
-        case 1: return go(ytri_kernel<T, 1>);
-        case 2: return go(ytri_kernel<T, 2>);
-        case 3: return go(ytri_kernel<T, 3>);
-        case 4: return go(ytri_kernel<T, 4>);
-        case 5: return go(ytri_kernel<T, 5>);
-        case 6: return go(ytri_kernel<T, 6>);
-        case 8: return go(ytri_kernel<T, 8>);
-        case 10: return go(ytri_kernel<T, 10>);
-        case 12: return go(ytri_kernel<T, 12>);
-        case 14: return go(ytri_kernel<T, 14>);
-        case 16: return go(ytri_kernel<T, 16>);
+        case 1: return yr.lines ? go(ytri_kernel<1, true>) : go(ytri_kernel<1, false>);
+        case 2: return yr.lines ? go(ytri_kernel<2, true>) : go(ytri_kernel<2, false>);
+        case 3: return yr.lines ? go(ytri_kernel<3, true>) : go(ytri_kernel<3, false>);
+        case 4: return yr.lines ? go(ytri_kernel<4, true>) : go(ytri_kernel<4, false>);
+        case 5: return yr.lines ? go(ytri_kernel<5, true>) : go(ytri_kernel<5, false>);
+        case 6: return yr.lines ? go(ytri_kernel<6, true>) : go(ytri_kernel<6, false>);
+        case 8: return yr.lines ? go(ytri_kernel<8, true>) : go(ytri_kernel<8, false>);
+        case 10: return yr.lines ? go(ytri_kernel<10, true>) : go(ytri_kernel<10, false>);
+        case 12: return yr.lines ? go(ytri_kernel<12, true>) : go(ytri_kernel<12, false>);
+        case 14: return yr.lines ? go(ytri_kernel<14, true>) : go(ytri_kernel<14, false>);
+        case 16: return yr.lines ? go(ytri_kernel<16, true>) : go(ytri_kernel<16, false>);
         default: return cudaErrorInvalidValue;
     }
 }
