@@ -11,6 +11,7 @@
 //   ibpm_get_state.
 // One step (advance!, src/solver.jl:155-190) is ~60 kernels on one stream;
 // each 2D DST solve is three line passes (see fft_dst.cuh).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -48,6 +49,23 @@ __global__ void tc_mult_kernel(Mult m, int P, float *tab) {
     if (r >= P) return;
     const int kx = tc_blk(c, P), ky = tc_blk(r, P);
     tab[(size_t)c * P + r] = (kx != 0 && ky != 0) ? (float)m(kx, ky) : 0.0f;
+}
+
+// Plain CG with B as a matrix.  An application of B is some twenty dependent
+// launches (about 90 us at 512^2 x 4, however small the body), while its n = 2 np
+// columns in batches cost about 0.2 n of them and CG takes about 0.3 n iterations
+// per decade of residual.  So where the first residual is more than kDenseGain
+// above the tolerance, B is assembled once for the step and the iterations run in
+// one cluster: at most kDenseN rows, those of each of kDenseCtas blocks in its
+// shared memory.  512^2 x 4, 101 points, reltol 1e-12, 530 iterations: a step took
+// 49.7 ms with B applied each time, 6.3 so.  The iteration is the same; only the
+// rounding of B u differs.
+constexpr double kDenseGain = 30.0;
+constexpr int kDenseCtas = 8, kDenseN = 448, kDenseThreads = 256;
+constexpr size_t dense_smem(int n) {
+    const int rows = (n + kDenseCtas - 1) / kDenseCtas;
+    // the block's rows of B; u and r whole; the blocks' partial sums, two kinds
+    return sizeof(double) * ((size_t)rows * n + 2 * (size_t)n + 2 * kDenseCtas);
 }
 
 thread_local std::string g_create_error;
@@ -334,6 +352,7 @@ struct Engine final : ibpm_handle {
     T *Gw = nullptr, *psiw = nullptr, *qw = nullptr;  // batch work (K columns)
     double *fcol = nullptr;
     double *Binv = nullptr, *Bwork = nullptr;  // B^-1 and the Gauss-Jordan ping-pong buffer
+    double *Bd = nullptr;  // B of the step, for the assembled CG (moving bodies, FP64, 2 np <= kDenseN)
     double *cg_u = nullptr, *cg_r = nullptr, *cg_c = nullptr, *cg_z = nullptr, *cg_s = nullptr, *cg_s_h = nullptr;
     int *err = nullptr, *err_h = nullptr;
     int last_cg_iters = 0;
@@ -1069,9 +1088,11 @@ struct Engine final : ibpm_handle {
     void diag_reg(const double *f, double *gamma1, const double *q1, double *fout) override;
     void setup();
     void build_Binv();
+    void assemble_B(double *B);
     void assemble_invert_B();
     void direct_rebuild();
     int batch_width() const;
+    int moving_batch() const;
     void cg(double *x, const double *b, bool have_bx = false, bool precond = false, const double *rref = nullptr);
     void cg_collect();
     int *cg_it = nullptr;
@@ -1216,7 +1237,7 @@ void Engine<T>::setup() {
 
     kbatch = batch_width();
     if (!std::is_same<T, double>::value) kbatch = 1;  // FP32 builds B^-1 with an FP64 engine
-    if (!static_bodies) kbatch = 2;  // the warm start applies B to two vectors at once
+    if (!static_bodies) kbatch = moving_batch();
     kbatch = std::min(kbatch, 2 * np);
     const int kb = std::max(kbatch, L);
     t1 = dalloc<T>(nt * kb);
@@ -1250,6 +1271,7 @@ void Engine<T>::setup() {
     psiw = dalloc<T>(ng * L * kbatch);
     qw = dalloc<T>(nq * kbatch);
     fcol = dalloc<double>(2 * (size_t)np * kbatch);
+    if (!static_bodies && std::is_same<T, double>::value && 2 * np <= kDenseN) Bd = dalloc<double>(4 * (size_t)np * np);
     cg_u = dalloc<double>(2 * np);
     cg_z = dalloc<double>(2 * np);
     cg_r = dalloc<double>(2 * np);
@@ -1327,6 +1349,15 @@ int Engine<T>::batch_width() const {
     return (int)std::min<long long>(2 * np, std::max(1LL, std::min<long long>(64, (4LL << 30) / per_col)));
 }
 
+// Columns of B a moving-body handle applies at once: the warm start two vectors,
+// the assembled CG up to sixteen within about 1 GB of column work.
+template <class T>
+int Engine<T>::moving_batch() const {
+    if (!std::is_same<T, double>::value || 2 * np > kDenseN) return 2;
+    const long long per_col = (2 * ng * L + nq + 2 * ng) * (long long)sizeof(T);
+    return (int)std::max(2LL, std::min<long long>(16, (1LL << 30) / per_col));
+}
+
 // _Binv_precomputed (src/coupling.jl:187-192): B column by column, then its inverse.
 template <class T>
 void Engine<T>::build_Binv() {
@@ -1341,8 +1372,19 @@ void Engine<T>::build_Binv() {
     if (err_h[1] != 0) throw ApiError{IBPM_ERR_INVALID, "B is not positive definite (pivot " + std::to_string(err_h[1]) + ")"};
 }
 
-// B of the current body position into Binv, kbatch columns per batched
-// application, then inverted by Gauss-Jordan elimination without pivoting
+// B of the current body position, kbatch columns per batched application.
+template <class T>
+void Engine<T>::assemble_B(double *B) {
+    const int n = 2 * np;
+    for (int c0 = 0; c0 < n; c0 += kbatch) {
+        const int nb = std::min(kbatch, n - c0);
+        unit_columns_kernel<<<(n * nb + 255) / 256, 256, 0, st>>>(fcol, n, c0, nb);
+        check_launch();
+        apply_B(fcol, B + (size_t)c0 * n, n, nb);
+    }
+}
+
+// B of the current body position into Binv, then inverted by Gauss-Jordan elimination without pivoting
 // between Binv and Bwork (the symmetric part of B is positive definite; with
 // nested levels B itself is not exactly symmetric); a pivot <= 0 sets err[1].
 template <class T>
@@ -1353,12 +1395,7 @@ void Engine<T>::assemble_invert_B() {
     tc_on = tc_prod > 0 && preconditioned() && tc != nullptr;
     const bool assembled_tc = tc_on;
     try {
-        for (int c0 = 0; c0 < n; c0 += kbatch) {
-            const int nb = std::min(kbatch, n - c0);
-            unit_columns_kernel<<<(n * nb + 255) / 256, 256, 0, st>>>(fcol, n, c0, nb);
-            check_launch();
-            apply_B(fcol, Binv + (size_t)c0 * n, n, nb);
-        }
+        assemble_B(Binv);
     } catch (...) {
         tc_on = false;
         throw;
@@ -1436,6 +1473,7 @@ struct CgArgs {
     int pre;
     double *z;
     const double *rref;
+    int dense;  // the assembled form may take over (kDenseGain)
 };
 
 __device__ __forceinline__ double cg_block_sum(double v, double *red) {
@@ -1450,7 +1488,7 @@ __device__ __forceinline__ double cg_block_sum(double v, double *red) {
 
 // r = b - c (c = B x0); u = 0; residual, tol = max(reltol ||r0||, abstol), and the
 // loop condition of IterativeSolvers' done(): !(it >= maxiter || ||r|| <= tol).
-__global__ void cg_init_kernel(CgArgs a, cudaGraphConditionalHandle h, int use_h) {
+__global__ void cg_init_kernel(CgArgs a, cudaGraphConditionalHandle h, cudaGraphConditionalHandle h_dense, int use_h) {
     __shared__ double red[32];
     double acc = 0.0;
     for (int k = threadIdx.x; k < a.n; k += blockDim.x) {
@@ -1475,8 +1513,99 @@ __global__ void cg_init_kernel(CgArgs a, cudaGraphConditionalHandle h, int use_h
         a.s[4] = res;  // initial residual, for reports
         a.s[8] = 1.0;  // rho before the first direction (u = 0 makes it immaterial)
         a.it[0] = 0;
-        if (use_h) cudaGraphSetConditional(h, cont ? 1u : 0u);
+        const bool dense = a.dense && cont && res > kDenseGain * tol;
+        if (use_h) cudaGraphSetConditional(h, cont && !dense ? 1u : 0u);
+        if (use_h && a.dense) cudaGraphSetConditional(h_dense, dense ? 1u : 0u);
     }
+}
+
+// cg_init_kernel's iteration to its end with the matrix B (n x n, column-major):
+// one cluster; block k owns rows k rows .. (k + 1) rows - 1 of B, x, r and c, and
+// every block holds u and r whole.  Two cluster barriers an iteration: one for
+// u . c, one for the new residual's rows and norm.  The blocks add the partial
+// sums in one order, so all of them take the same branch.
+__global__ void __cluster_dims__(kDenseCtas, 1, 1) __launch_bounds__(kDenseThreads)
+    cg_dense_kernel(CgArgs a, const double *__restrict__ B) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ double dsm[];
+    __shared__ double red[32];
+    const int n = a.n, rows = (n + kDenseCtas - 1) / kDenseCtas, rank = (int)cl.block_rank();
+    const int row0 = rank * rows, nr = max(0, min(rows, n - row0));
+    double *Bs = dsm, *u = Bs + (size_t)rows * n, *rv = u + n, *sums = rv + n;  // sums[kind][block]
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    for (int e = tid; e < nr * n; e += kDenseThreads) {
+        const int rr = e % nr, c = e / nr;
+        Bs[(size_t)rr * n + c] = B[(row0 + rr) + (size_t)n * c];
+    }
+    for (int k = tid; k < n; k += kDenseThreads) {
+        u[k] = 0.0;
+        rv[k] = a.r[k];
+    }
+    // thread q < nr owns row row0 + q
+    double x = tid < nr ? a.x[row0 + tid] : 0.0, c = 0.0;
+    __shared__ double cs[kDenseThreads];
+    double res = a.s[0], prev = a.s[1];
+    const double tol = a.s[2];
+    int it = 0, bad = 0;
+    bool cont = a.s[3] != 0.0;
+    cl.sync();
+    // the block's sum of v into every block's slot
+    auto publish = [&](double v, int kind) {
+        v = cg_block_sum(v, red);
+        if (tid < kDenseCtas) cl.map_shared_rank(sums, tid)[kind * kDenseCtas + rank] = v;
+    };
+    auto total = [&](int kind) {
+        double t = 0.0;
+        for (int k = 0; k < kDenseCtas; ++k) t += sums[kind * kDenseCtas + k];
+        return t;
+    };
+    while (cont) {
+        const double beta = res * res / (prev * prev);
+        for (int k = tid; k < n; k += kDenseThreads) u[k] = rv[k] + beta * u[k];
+        __syncthreads();
+        for (int q = w; q < nr; q += kDenseThreads / 32) {
+            const double *row = Bs + (size_t)q * n;
+            double acc = 0.0;
+            for (int k = lane; k < n; k += 32) acc = fma(row[k], u[k], acc);
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane == 0) cs[q] = acc;
+        }
+        __syncthreads();
+        c = tid < nr ? cs[tid] : 0.0;
+        const double um = tid < nr ? u[row0 + tid] : 0.0;
+        publish(um * c, 0);
+        cl.sync();
+        const double alpha = res * res / total(0);
+        double rn = 0.0;
+        if (tid < nr) {
+            x += alpha * um;
+            rn = rv[row0 + tid] - alpha * c;
+            for (int k = 0; k < kDenseCtas; ++k) cl.map_shared_rank(rv, k)[row0 + tid] = rn;
+        }
+        publish(rn * rn, 1);
+        cl.sync();
+        prev = res;
+        res = sqrt(total(1));
+        ++it;
+        cont = !(it >= a.maxiter || res <= tol);
+        if (!isfinite(res)) {
+            bad = 1;
+            cont = false;
+        }
+    }
+    if (tid < nr) {
+        a.x[row0 + tid] = x;
+        a.r[row0 + tid] = rv[row0 + tid];
+    }
+    if (rank == 0 && tid == 0) {
+        a.s[0] = res;
+        a.s[1] = prev;
+        a.s[3] = 0.0;
+        a.it[0] = it;
+        if (bad) a.err[2] = 1;
+    }
+    cl.sync();  // no block leaves while another may still write to its shared memory
 }
 
 // IBPM_WS_PRECOND_EXTRAP's start: x0 = Binv b (in x) is kept, and x gets the
@@ -1604,8 +1733,9 @@ template <class T>
 void Engine<T>::cg(double *x, const double *b, bool have_bx, bool precond, const double *rref) {
     const int n = 2 * np;
     const int nchunk = (n + 63) / 64;
+    const bool dense = !precond && Bd != nullptr;
     CgArgs a{n, x, cg_r, cg_u, cg_c, b, cg_s, cg_it, err, opt.cg_maxiter, opt.cg_reltol, opt.cg_abstol, precond ? 1 : 0,
-             cg_z, rref};
+             cg_z, rref, dense ? 1 : 0};
     // the direction: plain, or preconditioned by Binv (z = Binv r)
     auto direction = [&]() {
         if (precond) {
@@ -1617,6 +1747,18 @@ void Engine<T>::cg(double *x, const double *b, bool have_bx, bool precond, const
         }
         check_launch();
     };
+    auto assembled = [&]() {
+        assemble_B(Bd);
+        cg_dense_kernel<<<kDenseCtas, kDenseThreads, dense_smem(n), st>>>(a, Bd);
+        check_launch();
+    };
+    if (dense) {
+        static std::atomic<unsigned long long> attr_devices{0};
+        if (need_attr(attr_devices)) {
+            CK(cudaFuncSetAttribute(cg_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dense_smem(kDenseN)));
+            attr_devices.fetch_or(device_bit());
+        }
+    }
     if (!have_bx) apply_B(x, cg_c, n, 1);  // else cg_c already holds B x
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(st, &cs));
@@ -1625,46 +1767,58 @@ void Engine<T>::cg(double *x, const double *b, bool have_bx, bool precond, const
         const cudaGraphNode_t *deps = nullptr;
         size_t ndeps = 0;
         CK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &gr, &deps, &ndeps));
-        cudaGraphConditionalHandle hnd;
+        cudaGraphConditionalHandle hnd, hnd_dense = 0;
         CK(cudaGraphConditionalHandleCreate(&hnd, gr, 0, 0));
-        cg_init_kernel<<<1, 256, 0, st>>>(a, hnd, 1);
+        if (dense) CK(cudaGraphConditionalHandleCreate(&hnd_dense, gr, 0, 0));
+        cg_init_kernel<<<1, 256, 0, st>>>(a, hnd, hnd_dense, 1);
         check_launch();
-        CK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &gr, &deps, &ndeps));
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = hnd;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        cudaGraphNode_t node;
-        CK(cudaGraphAddNode(&node, gr, deps, ndeps, &cp));
-        CK(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
-        // capture the loop body into the WHILE node's graph on the side stream
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        cudaStream_t main = st;
-        st = st_side;
-        try {
-            CK(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+        // a conditional node after the stream's last one; its body is captured on
+        // the side stream
+        auto conditional = [&](cudaGraphConditionalNodeType type, cudaGraphConditionalHandle h, auto &&body_fn) {
+            CK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &gr, &deps, &ndeps));
+            cudaGraphNodeParams cp = {};
+            cp.type = cudaGraphNodeTypeConditional;
+            cp.conditional.handle = h;
+            cp.conditional.type = type;
+            cp.conditional.size = 1;
+            cudaGraphNode_t node;
+            CK(cudaGraphAddNode(&node, gr, deps, ndeps, &cp));
+            CK(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
+            cudaGraph_t body = cp.conditional.phGraph_out[0];
+            cudaStream_t main = st;
+            st = st_side;
+            try {
+                CK(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+                body_fn();
+                cudaGraph_t out = nullptr;
+                CK(cudaStreamEndCapture(st, &out));
+            } catch (...) {
+                cudaGraph_t out = nullptr;
+                cudaStreamEndCapture(st, &out);
+                st = main;
+                throw;
+            }
+            st = main;
+        };
+        if (dense) conditional(cudaGraphCondTypeIf, hnd_dense, assembled);
+        conditional(cudaGraphCondTypeWhile, hnd, [&] {
             direction();
             apply_B(cg_u, cg_c, n, 1);
             cg_update_kernel<<<1, 256, 0, st>>>(a, hnd, 1);
             check_launch();
-            cudaGraph_t out = nullptr;
-            CK(cudaStreamEndCapture(st, &out));
-        } catch (...) {
-            cudaGraph_t out = nullptr;
-            cudaStreamEndCapture(st, &out);
-            st = main;
-            throw;
-        }
-        st = main;
+        });
         return;
     }
-    cg_init_kernel<<<1, 256, 0, st>>>(a, 0, 0);
+    cg_init_kernel<<<1, 256, 0, st>>>(a, 0, 0, 0);
     check_launch();
-    for (;;) {
+    for (bool first = true;; first = false) {
         CK(cudaMemcpyAsync(cg_s_h, cg_s, sizeof(double) * 4, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         if (cg_s_h[3] == 0.0) break;
+        if (first && dense && cg_s_h[0] > kDenseGain * cg_s_h[2]) {
+            assembled();
+            break;
+        }
         direction();
         apply_B(cg_u, cg_c, n, 1);
         cg_update_kernel<<<1, 256, 0, st>>>(a, 0, 0);
