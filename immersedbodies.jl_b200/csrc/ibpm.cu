@@ -461,10 +461,12 @@ struct Engine final : ibpm_handle {
     // drops the captured step graphs (re-captured on the next step)
     void drop_graphs() {
         for (int p = 0; p < 2; ++p) {
-            if (graph_exec[p]) cudaGraphExecDestroy(graph_exec[p]);
-            if (graph[p]) cudaGraphDestroy(graph[p]);
-            graph_exec[p] = nullptr;
-            graph[p] = nullptr;
+            for (int v = 0; v < 2; ++v) {
+                if (graph_exec[p][v]) cudaGraphExecDestroy(graph_exec[p][v]);
+                if (graph[p][v]) cudaGraphDestroy(graph[p][v]);
+                graph_exec[p][v] = nullptr;
+                graph[p][v] = nullptr;
+            }
         }
         if (binv_exec) cudaGraphExecDestroy(binv_exec);
         if (binv_graph) cudaGraphDestroy(binv_graph);
@@ -822,7 +824,7 @@ struct Engine final : ibpm_handle {
 
     // vort2flux (src/fluid.jl:178-205) over nbatch independent fields.
     // G, psi: level 1 of batch 0, level stride ng, batch stride bs.
-    // qout: level 1 of batch 0 (level stride nq, batch stride qbs).  curl_all=false
+    // qout: level 1 of batch 0 (level stride nq, batch stride qbs; null: psi alone).  curl_all=false
     // computes q only at level 1 (the only level a caller reads) and solves each
     // coarser level (FP64) as far as its finer level's boundary values: of their psi only
     // level 2's four lines are written, where a face of bbox (device; batch b's at
@@ -865,7 +867,7 @@ struct Engine final : ibpm_handle {
         } else if (!levels_dst(psi_, Gm, bs, nbatch, hi1, win, central)) {
             return;
         }
-        curl(psi_, qout, bs, qbs, nbatch, curl_all, win);
+        if (qout) curl(psi_, qout, bs, qbs, nbatch, curl_all, win);
     }
 
     // vort2flux's solves, the y direction direct
@@ -1102,9 +1104,16 @@ struct Engine final : ibpm_handle {
     void step_body();
     // CUDA graphs of step_body (static bodies), one per buffer parity
     bool use_graphs = true;
-    cudaGraph_t graph[2] = {nullptr, nullptr};
-    cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
-    long long graph_launches[2] = {0, 0};
+    // (second index: q_given)
+    cudaGraph_t graph[2][2] = {};
+    cudaGraphExec_t graph_exec[2][2] = {};
+    long long graph_launches[2][2] = {};
+    // The steps read the flux as psi's curl and store none: q holds it only while
+    // q_current (ensure_q).  q_given: a caller set a q that is not psi's curl, which
+    // the next step therefore reads itself.
+    bool q_current = true, q_given = false;
+    void ensure_q();
+    void check_q();
     void materialise_q0();
 };
 
@@ -1905,7 +1914,8 @@ void Engine<T>::step(const ibpm_step_params &sp) {
     // moving bodies it holds the CG loop as a WHILE node.
     if (use_graphs && !prof) {
         const int p = gc;
-        if (!graph_exec[p]) {
+        const int v = q_given ? 1 : 0;
+        if (!graph_exec[p][v]) {
             const int gc0 = gc, nc0 = nc;
             const long long l0 = launches;  // the capture launches nothing
             CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -1921,21 +1931,23 @@ void Engine<T>::step(const ibpm_step_params &sp) {
                 launches = l0;
                 throw;
             }
-            CK(cudaStreamEndCapture(st, &graph[p]));
-            CK(cudaGraphInstantiate(&graph_exec[p], graph[p], 0));
+            CK(cudaStreamEndCapture(st, &graph[p][v]));
+            CK(cudaGraphInstantiate(&graph_exec[p][v], graph[p][v], 0));
             gc = gc0;
             nc = nc0;
             launches = l0;
         }
-        CK(cudaGraphLaunch(graph_exec[p], st));
-        launches += graph_launches[p];
+        CK(cudaGraphLaunch(graph_exec[p][v], st));
+        launches += graph_launches[p][v];
         gc = 1 - gc;
         nc = 1 - nc;
+        q_current = q_given = false;
         if (static_bodies) last_cg_iters = 0;
         cg_pending = !static_bodies;
         return;
     }
     step_body();
+    q_current = q_given = false;
 }
 
 // The device work of one step after the per-step parameters are uploaded.
@@ -1951,10 +1963,13 @@ void Engine<T>::step_body() {
     // get_trial_state (src/fluid.jl:467-506), all levels at once: the levels
     // only read the previous step's Gamma and q.
     {
-        NonlinArgs<T> a{q, Gold, N1, N2, rest, prm, g};
+        NonlinArgs<T> a{psi, q, Gold, N1, N2, rest, prm, g};
         const dim3 blk(kNlTX, kNlBY), grd((nx - 1 + kNlTX - 1) / kNlTX, (ny - 1 + kNlTY - 1) / kNlTY, L);
         const int pe = prof_begin();
-        nonlinear_kernel<<<grd, blk, 0, st>>>(a);
+        if (q_given)
+            nonlinear_kernel<T, T, false, true><<<grd, blk, 0, st>>>(a);
+        else
+            nonlinear_kernel<T><<<grd, blk, 0, st>>>(a);
         check_launch();
         prof_end(pe, IBPM_KCLASS_NONLINEAR, 8.0 * (double)(nq + 4 * ng) * L);
     }
@@ -2069,9 +2084,9 @@ void Engine<T>::step_body() {
     yimp(t1, 1);
     xpass(in_scratch(t1), OutSub<T>{Gnew, ng, nx - 1}, 1);
     // vort2flux!(state.psi, state.q, state.Gamma)
-    vort2flux(psi, q, Gnew, 0, 0, 1, true);
+    vort2flux(psi, nullptr, Gnew, 0, 0, 1, true);  // its q: ensure_q
     gc = 1 - gc;
-    graph_launches[1 - gc] = launches - launches0;
+    graph_launches[1 - gc][q_given ? 1 : 0] = launches - launches0;
 }
 
 // IBPM_MIXED_L1's step: the body's level (level 1) in FP64 -- its Gamma, flux,
@@ -2089,17 +2104,24 @@ void Engine<T>::step_body_l1d() {
     // nonlinear + rhs assembly (src/fluid.jl:467-493): level 1 in FP64, its coarser
     // level's Gamma in FP32; levels 2..L in FP32
     {
-        NonlinArgs<double, T> a{q1, G1o, N11, N12, rest1, prm, g};
+        NonlinArgs<double, T> a{psi1, q1, G1o, N11, N12, rest1, prm, g};
         a.coarse = L > 1 ? Gold + ng : nullptr;
+        a.psi_coarse = L > 1 ? psi + ng : nullptr;
         const dim3 grd((nx - 1 + kNlTX - 1) / kNlTX, (ny - 1 + kNlTY - 1) / kNlTY, 1);
-        nonlinear_kernel<double, T, true><<<grd, blk, 0, st>>>(a);
+        if (q_given)
+            nonlinear_kernel<double, T, true, true><<<grd, blk, 0, st>>>(a);
+        else
+            nonlinear_kernel<double, T, true><<<grd, blk, 0, st>>>(a);
         check_launch();
     }
     if (L > 1) {
-        NonlinArgs<T> a{q + nq, Gold + ng, N1 + ng, N2 + ng, rest + ng, prm, g};
+        NonlinArgs<T> a{psi + ng, q + nq, Gold + ng, N1 + ng, N2 + ng, rest + ng, prm, g};
         a.lev0 = 2;
         const dim3 grd((nx - 1 + kNlTX - 1) / kNlTX, (ny - 1 + kNlTY - 1) / kNlTY, L - 1);
-        nonlinear_kernel<T, T, true><<<grd, blk, 0, st>>>(a);
+        if (q_given)
+            nonlinear_kernel<T, T, true, true><<<grd, blk, 0, st>>>(a);
+        else
+            nonlinear_kernel<T, T, true><<<grd, blk, 0, st>>>(a);
         check_launch();
     }
     trial_dst<double>(G1o, rest1, G1n, 1, coef_lev, t1d, t2d);
@@ -2123,9 +2145,9 @@ void Engine<T>::step_body_l1d() {
     yimp(t1d, 1);
     xpass<double>(InPlain<double>{t1d, nt, ldt}, OutSub<double>{G1n, ng, nx - 1}, 1);
     // vort2flux!(state.psi, state.q, state.Gamma)
-    vort2flux_l1d(G1n, Gnew, q, psi1, q1, true);
+    vort2flux_l1d(G1n, Gnew, nullptr, psi1, nullptr, true);  // its q: ensure_q
     gc = 1 - gc;
-    graph_launches[1 - gc] = launches - launches0;
+    graph_launches[1 - gc][q_given ? 1 : 0] = launches - launches0;
 }
 
 // vort2flux (src/fluid.jl:178-205) with level 1 in FP64 (G1v; psi1_out, q1_out)
@@ -2153,7 +2175,7 @@ void Engine<T>::vort2flux_l1d(const double *G1v, T *Gm, T *qout, double *psi1_ou
         ylap(t1, 1);
         xpass(in_scratch(t1), out_plain(Pl, 0), 1);
     }
-    if (curl_all && L > 1) {
+    if (qout && curl_all && L > 1) {
         curl_kernel<T, T, T><<<dim3(qgrd.x, qgrd.y, L - 1), qblk, 0, st>>>(qout + nq, nq, psi + ng, ng,
                                                                           L > 2 ? psi + 2 * ng : nullptr, ng, g, nullptr,
                                                                           L - 1);
@@ -2166,6 +2188,7 @@ void Engine<T>::vort2flux_l1d(const double *G1v, T *Gm, T *qout, double *psi1_ou
         xpass<double>(InPlain<double>{G1v, 0, nx - 1}, OutPlain<double>{t1d, nt, ldt}, 1);
     ylap(t1d, 1);
     xpass<double>(InPlain<double>{t1d, nt, ldt}, OutPlain<double>{psi1_out, ng, nx - 1}, 1);
+    if (!q1_out) return;
     curl_kernel<double, double, T><<<qgrd, qblk, 0, st>>>(q1_out, 0, psi1_out, 0, coarse, 0, g);
     check_launch();
 }
@@ -2199,6 +2222,41 @@ __global__ void convert_kernel(B *__restrict__ dst, const A *__restrict__ src, l
         dst[k] = (B)src[k];
 }
 }  // namespace
+
+// q from psi, where a reader wants it after steps
+template <class T>
+void Engine<T>::ensure_q() {
+    if (q_current) return;
+    curl(psi, q, 0, 0, 1, true, nullptr);
+    if (l1d) {
+        const dim3 blk(64, 4), grd((nx + 1 + 63) / 64, (ny + 1 + 3) / 4, 1);
+        curl_kernel<double, double, T><<<grd, blk, 0, st>>>(q1, 0, psi1, 0, L > 1 ? psi + ng : nullptr, 0, g);
+        check_launch();
+    }
+    q_current = true;
+}
+
+// whether the q a caller set is psi's curl (waits for the stream)
+template <class T>
+void Engine<T>::check_q() {
+    const dim3 blk(64, 4), grd((nx + 1 + 63) / 64, (ny + 1 + 3) / 4, 1);
+    int *flag = err + 6;
+    CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
+    const int lo = l1d ? 1 : 0;  // the mixed engine's level 1 is the FP64 one
+    if (L > lo) {
+        curl_kernel<T, T, T, true><<<dim3(grd.x, grd.y, L - lo), blk, 0, st>>>(
+            q + lo * nq, nq, psi + lo * ng, ng, L - lo > 1 ? psi + (lo + 1) * ng : nullptr, ng, g, nullptr, L - lo, flag);
+        check_launch();
+    }
+    if (l1d) {
+        curl_kernel<double, double, T, true><<<grd, blk, 0, st>>>(q1, 0, psi1, 0, L > 1 ? psi + ng : nullptr, 0, g, nullptr,
+                                                                  1, flag);
+        check_launch();
+    }
+    CK(cudaMemcpyAsync(err_h + 6, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    q_given = err_h[6] != 0;
+}
 
 template <class T>
 void Engine<T>::upload(T *dst, const double *src, size_t n) {
@@ -2313,7 +2371,10 @@ void Engine<T>::get_field(int field, int level, double *out) {
         throw ApiError{IBPM_ERR_INVALID, "unknown field"};
     if (!out) throw ApiError{IBPM_ERR_INVALID, "null output"};
     if (!field_d) field_d = dalloc<double>((size_t)std::max<long long>(nq, ng));
-    if (field != IBPM_FIELD_VORTICITY) materialise_q0();
+    if (field != IBPM_FIELD_VORTICITY) {
+        ensure_q();
+        materialise_q0();
+    }
     if (l1d && level == 1) {
         // level 1 from its FP64 fields (q0 of the last step's callback values)
         if (field != IBPM_FIELD_VORTICITY) {
@@ -2450,6 +2511,7 @@ void Engine<T>::set_state(const ibpm_state_view *s) {
     const size_t np2 = sizeof(double) * 2 * np;
     index = s->index;
     t0 = s->t0;
+    ensure_q();  // q and psi may be set one without the other
     if (s->q) upload(q, s->q, nqL);
     if (s->q0) {
         if (!q0mat) q0mat = dalloc<T>(nq * L);
@@ -2482,7 +2544,7 @@ void Engine<T>::set_state(const ibpm_state_view *s) {
     // update_vars! (problem.jl:676-685)
     binv_reduce_kernel<<<1, 1024, 0, st>>>(nullptr, 0, 2 * np, Fbt, fb, total, g.h, g.dt, 0);
     check_launch();
-    CK(cudaStreamSynchronize(st));
+    check_q();
 }
 
 template <class T>
@@ -2494,7 +2556,10 @@ void Engine<T>::get_state(ibpm_state_view *s) {
     s->t0 = t0;
     s->freestream[0] = fs_last[0];
     s->freestream[1] = fs_last[1];
-    if (s->q) download(s->q, q, nqL);
+    if (s->q) {
+        ensure_q();
+        download(s->q, q, nqL);
+    }
     if (s->q0) {
         materialise_q0();
         download(s->q0, q0mat, nqL);
@@ -2735,8 +2800,9 @@ struct CaseGroup {
     bool stage_used[kStage] = {};
     int stage_next = 0;
     int gc = 0, nc = 0;
-    cudaGraph_t graph[2] = {nullptr, nullptr};
-    cudaGraphExec_t exec[2] = {nullptr, nullptr};
+    cudaGraph_t graph[2][2] = {};  // second index: q_given
+    cudaGraphExec_t exec[2][2] = {};
+    bool q_given = false;  // a case's q is not its psi's curl: this step reads every case's q
     std::vector<void *> mem;
 
     template <class U>
@@ -2892,8 +2958,10 @@ struct CaseGroup {
         } catch (...) {
         }
         for (int p = 0; p < 2; ++p) {
-            if (exec[p]) cudaGraphExecDestroy(exec[p]);
-            if (graph[p]) cudaGraphDestroy(graph[p]);
+            for (int v = 0; v < 2; ++v) {
+                if (exec[p][v]) cudaGraphExecDestroy(exec[p][v]);
+                if (graph[p][v]) cudaGraphDestroy(graph[p][v]);
+            }
         }
         for (void *p : mem) cudaFree(p);
         for (int k = 0; k < kStage; ++k) {
@@ -2946,9 +3014,12 @@ struct CaseGroup {
         T *N1 = nl[nc], *N2 = nl[1 - nc];
         const long long bsG = ng * L, bsQ = nq * L;
         {
-            NonlinArgs<T> a{q, Gold, N1, N2, rest, prm_tab, e.g, re_tab, 1};
+            NonlinArgs<T> a{psi, q, Gold, N1, N2, rest, prm_tab, e.g, re_tab, 1};
             const dim3 blk(kNlTX, kNlBY), grd((e.nx - 1 + kNlTX - 1) / kNlTX, (e.ny - 1 + kNlTY - 1) / kNlTY, C * L);
-            nonlinear_kernel<T, T, true><<<grd, blk, 0, st>>>(a);
+            if (q_given)
+                nonlinear_kernel<T, T, true, true><<<grd, blk, 0, st>>>(a);
+            else
+                nonlinear_kernel<T, T, true><<<grd, blk, 0, st>>>(a);
             e.check_launch();
         }
         if constexpr (std::is_same<T, double>::value)
@@ -2979,7 +3050,7 @@ struct CaseGroup {
         else
             e.ypass_dst(t1, C, coef_all, L);
         e.xpass(e.in_scratch(t1), OutSub<T>{Gnew, bsG, e.nx - 1}, C);
-        e.vort2flux(psi, q, Gnew, bsG, bsQ, C, true);
+        e.vort2flux(psi, nullptr, Gnew, bsG, bsQ, C, true);  // its q: ensure_q
         gc = 1 - gc;
     }
 
@@ -2998,8 +3069,15 @@ struct CaseGroup {
         }
         CK(cudaMemcpyAsync(prm_tab, stage_h[k], sizeof(StepDev) * C, cudaMemcpyHostToDevice, st));
         CK(cudaEventRecord(stage_ev[k], st));
-        const int p = gc;
-        if (!exec[p]) {
+        q_given = false;
+        for (const Engine<T> *e : cs) q_given = q_given || e->q_given;
+        if (q_given)
+            for (Engine<T> *e : cs) {
+                e->ensure_q();
+                CK(cudaStreamSynchronize(e->st));
+            }
+        const int p = gc, v = q_given ? 1 : 0;
+        if (!exec[p][v]) {
             const int gc0 = gc, nc0 = nc;
             const long long l0 = e0->launches;
             CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -3015,13 +3093,13 @@ struct CaseGroup {
                 e0->launches = l0;
                 throw;
             }
-            CK(cudaStreamEndCapture(st, &graph[p]));
-            CK(cudaGraphInstantiate(&exec[p], graph[p], 0));
+            CK(cudaStreamEndCapture(st, &graph[p][v]));
+            CK(cudaGraphInstantiate(&exec[p][v], graph[p][v], 0));
             gc = gc0;
             nc = nc0;
             e0->launches = l0;
         }
-        CK(cudaGraphLaunch(exec[p], st));
+        CK(cudaGraphLaunch(exec[p][v], st));
         gc = 1 - gc;
         nc = 1 - nc;
         for (int c = 0; c < C; ++c) {
@@ -3029,6 +3107,7 @@ struct CaseGroup {
             ++e.index;
             e.gc = gc;
             e.nc = nc;
+            e.q_current = e.q_given = false;
             e.q0_zero = false;
             e.q0_from_user = false;
             e.last_cg_iters = 0;

@@ -715,7 +715,8 @@ __global__ void __launch_bounds__(D::TPF *NG, trial_occ<D>() / (D::TPF * NG))
 // with Gamma_bc = 0.25 get_bc(Gamma[:, lev+1]) (src/fluid.jl:473-483).  Batch b = level - 1.
 template <class T, class TC = T>
 struct NonlinArgs {
-    const T *q;           // nq x L
+    const T *psi;         // ng x L: the flux q is its curl (with the coarser level's psi around it)
+    const T *q;           // nq x L, read instead of psi by the FROMQ form
     const T *gam;         // ng x L
     T *out;               // ng x L (state.nonlin[1])
     const T *n2;          // ng x L (state.nonlin[2]); with rest != nullptr
@@ -731,6 +732,7 @@ struct NonlinArgs {
     // of another precision); otherwise a field's coarser level is the next batch.
     int lev0 = 1;
     const TC *coarse = nullptr;
+    const TC *psi_coarse = nullptr;  // likewise psi of level lev0 + 1
 };
 
 // Tile of the nonlinear kernel: kNlTX x kNlTY circulation points per block of
@@ -748,7 +750,11 @@ constexpr int kNlTX = 32, kNlTY = 16, kNlBY = 8;
 // EXT: the ensemble / mixed-precision features of NonlinArgs (levels from lev0,
 // per-case tables, a coarse field of another type); without them the kernel
 // keeps the single-case code (fewer live registers, more resident blocks).
-template <class T, class TC = T, bool EXT = false>
+// The flux is formed from psi's tile, each face the difference curl! stores: one
+// tile instead of two (five 1024^2 FP64 levels 75.8 us against 86.6), and the steps
+// keep no flux of their own (its curl: 42 us and 84 MB written and read again).  FROMQ reads q itself, for the
+// first step after a caller set a q that is not psi's curl.
+template <class T, class TC = T, bool EXT = false, bool FROMQ = false>
 __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(NonlinArgs<T, TC> a) {
     const Grid &g = a.g;
     const int nx = g.nx, ny = g.ny;
@@ -765,20 +771,24 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
     const int I0 = blockIdx.x * kNlTX, J0 = blockIdx.y * kNlTY;  // outputs I0+1..I0+TX, J0+1..J0+TY
     const long long nq = (long long)(nx + 1) * ny + (long long)nx * (ny + 1), ng = (long long)(nx - 1) * (ny - 1);
     const long long nu = (long long)(nx + 1) * ny;
-    const T *q = a.q + b * nq;
+    const T *q = FROMQ ? a.q + b * nq : a.psi + b * ng;
     const T *Gt = a.gam + b * ng;
-    const TC *C = nullptr;
+    const TC *C = nullptr, *CP = nullptr;  // the coarser level's Gamma and psi
     if (lev < g.L) {
-        if (EXT && a.coarse != nullptr)
+        if (EXT && a.coarse != nullptr) {
             C = a.coarse + cs * ng;
-        else if constexpr (std::is_same<T, TC>::value)
+            if (!FROMQ) CP = a.psi_coarse + cs * ng;
+        } else if constexpr (std::is_same<T, TC>::value) {
             C = a.gam + (b + 1) * ng;
+            if (!FROMQ) CP = a.psi + (b + 1) * ng;
+        }
     }
     __shared__ double aqy[kNlTY + 2][kNlTX];      // avg_qy(i, j), i = I0+2+x, j = J0+1+y
     __shared__ double aqx[kNlTY][kNlTX + 2];      // avg_qx(i, j), i = I0+1+x, j = J0+2+y
     __shared__ T gm[kNlTY + 2][kNlTX + 2];        // Gamma(i, j),  i = I0+x,   j = J0+y
-    __shared__ T ru[kNlTY + 1][kNlTX + 2];        // q_u(i, j),    i = I0+1+x, j = J0+1+y
-    __shared__ T rv[kNlTY + 2][kNlTX + 1];        // q_v(i, j),    i = I0+1+x, j = J0+1+y
+    __shared__ T ru[FROMQ ? kNlTY + 1 : 1][FROMQ ? kNlTX + 2 : 1];  // q_u(i, j), i = I0+1+x, j = J0+1+y
+    __shared__ T rv[FROMQ ? kNlTY + 2 : 1][FROMQ ? kNlTX + 1 : 1];  // q_v(i, j), i = I0+1+x, j = J0+1+y
+    __shared__ T pm[FROMQ ? 1 : kNlTY + 2][FROMQ ? 1 : kNlTX + 2];  // psi(i, j), i = I0+x, j = J0+y
     __shared__ T rn[kNlTY][kNlTX];                // N2(i, j),     i = I0+1+x, j = J0+1+y
     const int tid = threadIdx.y * kNlTX + threadIdx.x;
     constexpr int NT = kNlTX * kNlBY;
@@ -786,33 +796,44 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
     // base_flux! of a static grid is U hc on every face (fluid.jl:22-32)
     const double sbx = prm_of()->fs[0] * hc, sby = prm_of()->fs[1] * hc;
     const bool moving = g.grid_moving;
+    auto around = [&](int i, int j) -> double {  // psi on the domain's boundary, from the coarser level
+        if (j == 0 || j == ny) return getbc(CP, g, j == 0 ? SIDE_B : SIDE_T, i + 1);
+        return getbc(CP, g, i == 0 ? SIDE_L : SIDE_R, j + 1);
+    };
     // the tile's raw faces, Gamma and N2, all in flight at once (zeros outside the grid)
+    if constexpr (FROMQ) {
 #pragma unroll
-    for (int e = tid; e < (kNlTY + 1) * (kNlTX + 2); e += NT) {
-        const int x = e % (kNlTX + 2), y = e / (kNlTX + 2);
-        const int i = I0 + 1 + x, j = J0 + 1 + y;
-        if (i <= nx + 1 && j <= ny)
-            cp_async_elem(&ru[y][x], q + UI(i, j));
-        else
-            ru[y][x] = T(0);
-    }
+        for (int e = tid; e < (kNlTY + 1) * (kNlTX + 2); e += NT) {
+            const int x = e % (kNlTX + 2), y = e / (kNlTX + 2);
+            const int i = I0 + 1 + x, j = J0 + 1 + y;
+            if (i <= nx + 1 && j <= ny)
+                cp_async_elem(&ru[y][x], q + UI(i, j));
+            else
+                ru[y][x] = T(0);
+        }
 #pragma unroll
-    for (int e = tid; e < (kNlTY + 2) * (kNlTX + 1); e += NT) {
-        const int x = e % (kNlTX + 1), y = e / (kNlTX + 1);
-        const int i = I0 + 1 + x, j = J0 + 1 + y;
-        if (i <= nx && j <= ny + 1)
-            cp_async_elem(&rv[y][x], q + VI(i, j));
-        else
-            rv[y][x] = T(0);
+        for (int e = tid; e < (kNlTY + 2) * (kNlTX + 1); e += NT) {
+            const int x = e % (kNlTX + 1), y = e / (kNlTX + 1);
+            const int i = I0 + 1 + x, j = J0 + 1 + y;
+            if (i <= nx && j <= ny + 1)
+                cp_async_elem(&rv[y][x], q + VI(i, j));
+            else
+                rv[y][x] = T(0);
+        }
     }
 #pragma unroll
     for (int e = tid; e < (kNlTY + 2) * (kNlTX + 2); e += NT) {
         const int x = e % (kNlTX + 2), y = e / (kNlTX + 2);
         const int i = I0 + x, j = J0 + y;
-        if (i >= 1 && i <= nx - 1 && j >= 1 && j <= ny - 1)
+        if (i >= 1 && i <= nx - 1 && j >= 1 && j <= ny - 1) {
             cp_async_elem(&gm[y][x], Gt + GI(i, j));
-        else
+            if constexpr (!FROMQ) cp_async_elem(&pm[y][x], q + GI(i, j));
+        } else {
             gm[y][x] = T(0);
+            // FP64: the coarser level's values around the field go into the tile; they
+            // are not FP32 numbers, so FP32's edge tiles form them where they are used
+            if constexpr (!FROMQ) pm[y][x] = sizeof(T) == 8 && i <= nx && j <= ny ? (T)around(i, j) : T(0);
+        }
     }
     if (a.rest) {
 #pragma unroll
@@ -827,6 +848,23 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
     }
     cp_async_wait_all();
     __syncthreads();
+    // the faces of the tile, i = I0+1+x, j = J0+1+y: read, or psi's differences
+    // (curl!, fluid.jl:230-276; FP32's own subtraction rounds as the FP64 one cast)
+    const bool edge = sizeof(T) == 4 && (I0 == 0 || J0 == 0 || I0 + kNlTX + 1 >= nx || J0 + kNlTY + 1 >= ny);
+    auto vertex = [&](int x, int y) -> double {  // psi(I0 + x, J0 + y)
+        const int i = I0 + x, j = J0 + y;
+        return i >= 1 && i <= nx - 1 && j >= 1 && j <= ny - 1 ? (double)pm[y][x] : around(i, j);
+    };
+    auto face_u = [&](int y, int x) -> double {
+        if constexpr (FROMQ) return (double)ru[y][x];
+        if (edge) return (double)(T)(vertex(x, y + 1) - vertex(x, y));
+        return (double)(pm[y + 1][x] - pm[y][x]);
+    };
+    auto face_v = [&](int y, int x) -> double {
+        if constexpr (FROMQ) return (double)rv[y][x];
+        if (edge) return (double)(T)(vertex(x, y) - vertex(x + 1, y));
+        return (double)(pm[y][x] - pm[y][x + 1]);
+    };
     // face averages Q = (q + q0) pair sums / 2 (avg_flux!), each formed once per tile
 #pragma unroll
     for (int e = tid; e < (kNlTY + 2) * kNlTX; e += NT) {
@@ -834,12 +872,12 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
         const int i = I0 + 2 + x, j = J0 + 1 + y;
         double v = 0.0;
         if (i <= nx && j <= ny + 1) {
-            // q_v(i, j) = rv[y][x + 1], q_v(i - 1, j) = rv[y][x]
+            // q_v(i, j) and q_v(i - 1, j)
             if (moving)
-                v = ((double)rv[y][x + 1] + (double)rv[y][x] + base_flux_y(g, prm_of(), lev, i, j) +
+                v = (face_v(y, x + 1) + face_v(y, x) + base_flux_y(g, prm_of(), lev, i, j) +
                      base_flux_y(g, prm_of(), lev, i - 1, j)) / 2;
             else
-                v = ((double)rv[y][x + 1] + (double)rv[y][x] + sby + sby) / 2;
+                v = (face_v(y, x + 1) + face_v(y, x) + sby + sby) / 2;
         }
         aqy[y][x] = v;
     }
@@ -849,12 +887,12 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
         const int i = I0 + 1 + x, j = J0 + 2 + y;
         double v = 0.0;
         if (i <= nx + 1 && j <= ny) {
-            // q_u(i, j) = ru[y + 1][x], q_u(i, j - 1) = ru[y][x]
+            // q_u(i, j) and q_u(i, j - 1)
             if (moving)
-                v = ((double)ru[y + 1][x] + (double)ru[y][x] + base_flux_x(g, prm_of(), lev, i, j) +
+                v = (face_u(y + 1, x) + face_u(y, x) + base_flux_x(g, prm_of(), lev, i, j) +
                      base_flux_x(g, prm_of(), lev, i, j - 1)) / 2;
             else
-                v = ((double)ru[y + 1][x] + (double)ru[y][x] + sbx + sbx) / 2;
+                v = (face_u(y + 1, x) + face_u(y, x) + sbx + sbx) / 2;
         }
         aqx[y][x] = v;
     }
@@ -912,10 +950,11 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
 // coarser field.
 // win (device, may be null): only the faces in i0..i1 x j0..j1 are written, by a
 // grid of any size sweeping the window.
-template <class T, class TP, class TC>
+// differs (CHECK form): set to 1 if q holds anything else than those faces.
+template <class T, class TP, class TC, bool CHECK = false>
 __global__ void curl_kernel(T *__restrict__ qout, long long qbs, const TP *__restrict__ psi, long long bs,
                             const TC *__restrict__ coarse, long long cbs, Grid g, const int *__restrict__ win = nullptr,
-                            int nl = 1) {
+                            int nl = 1, int *differs = nullptr) {
     const int nx = g.nx, ny = g.ny;
     const long long nu = (long long)(nx + 1) * ny;
     const int b = blockIdx.z;
@@ -923,11 +962,18 @@ __global__ void curl_kernel(T *__restrict__ qout, long long qbs, const TP *__res
     const TC *C = coarse && (nl == 1 || (b + 1) % nl != 0) ? coarse + b * cbs : nullptr;
     T *q = qout + b * qbs;
     auto P = [&](long long k) -> double { return (double)Pt[k]; };
+    auto put = [&](long long k, double v) {
+        if constexpr (CHECK) {
+            if (!(q[k] == (T)v)) *differs = 1;
+        } else {
+            q[k] = (T)v;
+        }
+    };
     auto face = [&](int i, int j) {
         if (i >= 2 && i <= nx - 1 && j >= 2 && j <= ny - 1) {
             const double pc = P(GI(i - 1, j - 1));
-            q[UI(i, j)] = (T)(P(GI(i - 1, j)) - pc);
-            q[VI(i, j)] = (T)(pc - P(GI(i, j - 1)));
+            put(UI(i, j), P(GI(i - 1, j)) - pc);
+            put(VI(i, j), pc - P(GI(i, j - 1)));
             return;
         }
         if (j <= ny) {
@@ -942,7 +988,7 @@ __global__ void curl_kernel(T *__restrict__ qout, long long qbs, const TP *__res
                 v = getbc(C, g, SIDE_T, i) - P(GI(i - 1, ny - 1));
             else
                 v = P(GI(i - 1, j)) - P(GI(i - 1, j - 1));
-            q[UI(i, j)] = (T)v;
+            put(UI(i, j), v);
         }
         if (i <= nx) {
             double v;
@@ -956,7 +1002,7 @@ __global__ void curl_kernel(T *__restrict__ qout, long long qbs, const TP *__res
                 v = P(GI(nx - 1, j - 1)) - getbc(C, g, SIDE_R, j);
             else
                 v = P(GI(i - 1, j - 1)) - P(GI(i, j - 1));
-            q[VI(i, j)] = (T)v;
+            put(VI(i, j), v);
         }
     };
     const int ti = blockIdx.x * blockDim.x + threadIdx.x, tj = blockIdx.y * blockDim.y + threadIdx.y;
