@@ -751,8 +751,11 @@ constexpr int kNlTX = 32, kNlTY = 16, kNlBY = 8;
 // per-case tables, a coarse field of another type); without them the kernel
 // keeps the single-case code (fewer live registers, more resident blocks).
 // The flux is formed from psi's tile, each face the difference curl! stores: one
-// tile instead of two (five 1024^2 FP64 levels 75.8 us against 86.6), and the steps
-// keep no flux of their own (its curl: 42 us and 84 MB written and read again).  FROMQ reads q itself, for the
+// tile instead of two, and the steps keep no flux of their own (its curl, five 1024^2
+// FP64 levels: 42 us and 84 MB written and read again).  The kernel is bound by
+// instructions, 520 an output with an index division and bounds tests for every
+// element of its tiles; inner tiles do without: five 1024^2 levels 86.6 us reading q,
+// 75.8 psi, 53.0 with inner tiles by rows.  FROMQ reads q itself, for the
 // first step after a caller set a q that is not psi's curl.
 template <class T, class TC = T, bool EXT = false, bool FROMQ = false>
 __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(NonlinArgs<T, TC> a) {
@@ -800,6 +803,33 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
         if (j == 0 || j == ny) return getbc(CP, g, j == 0 ? SIDE_B : SIDE_T, i + 1);
         return getbc(CP, g, i == 0 ? SIDE_L : SIDE_R, j + 1);
     };
+    // A tile whose vertices all lie inside the grid (most of a large one) takes its
+    // rows by warps, without an index division or a bounds test per element, and
+    // two neighbouring output rows per thread, which share a flux product
+    const bool inner = !FROMQ && I0 > 0 && J0 > 0 && I0 + kNlTX + 1 < nx && J0 + kNlTY + 1 < ny;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    if (inner) {
+        const int at = (nx - 1) * (J0 - 1 + ty) + I0 - 1 + tx;  // Gamma(I0 + tx, J0 + ty)
+#pragma unroll
+        for (int k = 0; k < (kNlTY + 2 + kNlBY - 1) / kNlBY; ++k) {
+            const int y = ty + k * kNlBY;
+            if (y < kNlTY + 2) {
+                cp_async_elem(&gm[y][tx], Gt + at + (nx - 1) * (k * kNlBY));
+                cp_async_elem(&pm[FROMQ ? 0 : y][FROMQ ? 0 : tx], q + at + (nx - 1) * (k * kNlBY));
+            }
+        }
+        if (tid < 2 * (kNlTY + 2)) {  // the two columns beyond the warp's width
+            const int y = tid >> 1, x = kNlTX + (tid & 1), o = (nx - 1) * (J0 - 1 + y) + I0 - 1 + x;
+            cp_async_elem(&gm[y][x], Gt + o);
+            cp_async_elem(&pm[FROMQ ? 0 : y][FROMQ ? 0 : x], q + o);
+        }
+        if (a.rest) {
+            const T *n2 = a.n2 + b * ng + at + nx;  // one row and one column on
+#pragma unroll
+            for (int k = 0; k < kNlTY / kNlBY; ++k)
+                cp_async_elem(&rn[ty + k * kNlBY][tx], n2 + (nx - 1) * (k * kNlBY));
+        }
+    } else {
     // the tile's raw faces, Gamma and N2, all in flight at once (zeros outside the grid)
     if constexpr (FROMQ) {
 #pragma unroll
@@ -846,11 +876,12 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
                 rn[y][x] = T(0);
         }
     }
+    }
     cp_async_wait_all();
     __syncthreads();
     // the faces of the tile, i = I0+1+x, j = J0+1+y: read, or psi's differences
     // (curl!, fluid.jl:230-276; FP32's own subtraction rounds as the FP64 one cast)
-    const bool edge = sizeof(T) == 4 && (I0 == 0 || J0 == 0 || I0 + kNlTX + 1 >= nx || J0 + kNlTY + 1 >= ny);
+    const bool edge = sizeof(T) == 4 && !inner;
     auto vertex = [&](int x, int y) -> double {  // psi(I0 + x, J0 + y)
         const int i = I0 + x, j = J0 + y;
         return i >= 1 && i <= nx - 1 && j >= 1 && j <= ny - 1 ? (double)pm[y][x] : around(i, j);
@@ -866,6 +897,22 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
         return (double)(pm[y][x] - pm[y][x + 1]);
     };
     // face averages Q = (q + q0) pair sums / 2 (avg_flux!), each formed once per tile
+    if (inner && !moving) {
+        auto ay = [&](int y, int x) {
+            aqy[y][x] = ((double)(pm[y][x + 1] - pm[y][x + 2]) + (double)(pm[y][x] - pm[y][x + 1]) + sby + sby) / 2;
+        };
+        auto ax = [&](int y, int x) {
+            aqx[y][x] = ((double)(pm[y + 2][x] - pm[y + 1][x]) + (double)(pm[y + 1][x] - pm[y][x]) + sbx + sbx) / 2;
+        };
+        if constexpr (!FROMQ) {
+#pragma unroll
+            for (int k = 0; k < (kNlTY + 2 + kNlBY - 1) / kNlBY; ++k)
+                if (ty + k * kNlBY < kNlTY + 2) ay(ty + k * kNlBY, tx);
+#pragma unroll
+            for (int k = 0; k < kNlTY / kNlBY; ++k) ax(ty + k * kNlBY, tx);
+            if (tid < 2 * kNlTY) ax(tid >> 1, kNlTX + (tid & 1));
+        }
+    } else {
 #pragma unroll
     for (int e = tid; e < (kNlTY + 2) * kNlTX; e += NT) {
         const int x = e % kNlTX, y = e / kNlTX;
@@ -896,7 +943,40 @@ __global__ void __launch_bounds__(kNlTX *kNlBY, EXT ? 4 : 5) nonlinear_kernel(No
         }
         aqx[y][x] = v;
     }
+    }
     __syncthreads();
+    // the FP64 engine's results of an inner tile; the FP32 one keeps the general form
+    // below, whose multiply-adds are contracted in one fixed way (its results are
+    // reproducible bit for bit)
+    if constexpr (sizeof(T) == 8 && std::is_same<T, TC>::value && !FROMQ) {
+        if (inner) {
+            auto fx = [&](int yj) { return (aqy[yj][tx] * gm[yj][tx + 1] + aqy[yj - 1][tx] * gm[yj - 1][tx + 1]) / 2; };
+            auto fy = [&](int xi, int y) { return -(aqx[y][xi] * gm[y + 1][xi] + aqx[y][xi - 1] * gm[y + 1][xi - 1]) / 2; };
+            const double ih2 = 1 / (hc * hc);
+            const double cg = a.rest ? 0.5 * (g.dt / (re_of() * (hc * hc))) : 0.0;
+            static_assert(kNlTY == 2 * kNlBY, "two output rows a thread");
+            const int y0 = 2 * ty;
+            const long long o = b * ng + GI(I0 + 1 + tx, J0 + 1 + y0);
+            double f0 = fx(y0 + 1);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int y = y0 + k;
+                const double f1 = fx(y + 2);
+                const double r = (f0 - f1) + (fy(tx + 2, y) - fy(tx + 1, y));
+                f0 = f1;
+                const double n1 = r * ih2;
+                a.out[o + k * (nx - 1)] = (T)n1;
+                if (a.rest) {
+                    double v = (g.dt * 1.5) * n1 + (g.dt * -0.5) * (double)rn[y][tx];
+                    const double gc = gm[y + 1][tx + 1];  // + A Gamma, see below
+                    const double lap = (gm[y + 1][tx] + gm[y + 1][tx + 2] - 2 * gc) + (gm[y][tx + 1] + gm[y + 2][tx + 1] - 2 * gc);
+                    v += gc + cg * lap;
+                    a.rest[o + k * (nx - 1)] = (T)v;
+                }
+            }
+            return;
+        }
+    }
     const int x = threadIdx.x, I = I0 + 1 + x;
     if (I > nx - 1) return;
     // x-flux product at (I+1, j) (direct_product_loops!, fluid.jl:396-415)
