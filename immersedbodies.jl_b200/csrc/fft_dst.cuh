@@ -29,6 +29,10 @@ namespace ibpm {
 constexpr int kTPF = 64;        // threads per FFT group (two warps)
 constexpr int kMaxV = 20;       // complex values a thread holds in one stage
 constexpr int kMaxE = 8;        // scan values per thread (M/2/kTPF, M <= 1024)
+// the same for lengths up to MX (radices 2 to 5): sized for 1024 points, the short
+// transforms' register arrays spilled (880 bytes a thread)
+__host__ __device__ constexpr int max_values(int MX) { return MX <= 256 ? 6 : MX <= 512 ? 10 : kMaxV; }
+__host__ __device__ constexpr int max_scan(int MX) { return (MX / 2 + kTPF - 1) / kTPF; }
 constexpr int kMaxStages = 12;
 constexpr int kMaxM = 1024;     // largest transform length (nx or ny)
 
@@ -128,29 +132,33 @@ struct Dft<5, C> {
 
 // One Stockham stage of radix R over buf[0..M).  Every thread of the block
 // must call it (it contains block barriers).
-template <int R, class C>
+template <int R, int V, class C>
 __device__ __forceinline__ void fft_stage(C *buf, int M, int Ns, const C *__restrict__ tw, int t) {
-    constexpr int KMAX = kMaxV / R;
+    constexpr int KMAX = V / R;
     const int nb = M / R;
     const int twstep = M / (Ns * R);
+    // j / Ns for j < 1024: exact, since j (inv Ns - 2^20) < 2^20
+    const unsigned inv = ((1u << 20) + Ns - 1) / Ns;
     C v[KMAX][R];
     int dst[KMAX];
 #pragma unroll
     for (int kb = 0; kb < KMAX; ++kb) {
+        if (kb * kTPF >= nb) break;  // uniform: the unrolled rest is jumped over
         const int j = t + kb * kTPF;
         dst[kb] = -1;
         if (j < nb) {
-            const int k = j % Ns;
+            const int d = (int)(((unsigned)j * inv) >> 20) * Ns, k = j - d;
             v[kb][0] = buf[j];
 #pragma unroll
             for (int r = 1; r < R; ++r) v[kb][r] = cmul(buf[j + r * nb], __ldg(&tw[r * k * twstep]));
             Dft<R, C>::run(v[kb]);
-            dst[kb] = (j / Ns) * Ns * R + k;
+            dst[kb] = d * R + k;
         }
     }
     __syncthreads();
 #pragma unroll
     for (int kb = 0; kb < KMAX; ++kb) {
+        if (kb * kTPF >= nb) break;
         if (dst[kb] >= 0) {
 #pragma unroll
             for (int r = 0; r < R; ++r) buf[dst[kb] + r * Ns] = v[kb][r];
@@ -160,20 +168,20 @@ __device__ __forceinline__ void fft_stage(C *buf, int M, int Ns, const C *__rest
 }
 
 // Forward complex FFT of buf[0..M) in place (natural order in and out).
-template <class T>
+template <class T, int MX>
 __device__ __forceinline__ void fft(typename Cx<T>::type *buf, const PlanT<T> &pl, int t) {
     using C = typename Cx<T>::type;
     int Ns = 1;
     for (int s = 0; s < pl.nst; ++s) {
         const int R = pl.radix[s];
         if (R == 4)
-            fft_stage<4, C>(buf, pl.M, Ns, pl.tw, t);
+            fft_stage<4, max_values(MX), C>(buf, pl.M, Ns, pl.tw, t);
         else if (R == 2)
-            fft_stage<2, C>(buf, pl.M, Ns, pl.tw, t);
+            fft_stage<2, max_values(MX), C>(buf, pl.M, Ns, pl.tw, t);
         else if (R == 3)
-            fft_stage<3, C>(buf, pl.M, Ns, pl.tw, t);
+            fft_stage<3, max_values(MX), C>(buf, pl.M, Ns, pl.tw, t);
         else
-            fft_stage<5, C>(buf, pl.M, Ns, pl.tw, t);
+            fft_stage<5, max_values(MX), C>(buf, pl.M, Ns, pl.tw, t);
         Ns *= R;
     }
 }
@@ -202,17 +210,18 @@ __device__ __forceinline__ void dst_pre(typename Cx<T>::type *buf, const PlanT<T
 
 // DST post-processing: buf[0..M) holds V; on return buf[1..M-1] holds y and
 // buf[0] = buf[M] = 0.  wt: two double2 scratch slots for this group.
-template <class T>
+template <class T, int MX>
 __device__ __forceinline__ void dst_post(typename Cx<T>::type *buf, const PlanT<T> &pl, int t, double2 *wt) {
     using C = typename Cx<T>::type;
+    constexpr int KE = max_scan(MX);
     const int M = pl.M, H = M >> 1;
     const int E = (H + kTPF - 1) / kTPF;
     const int k0 = t * E;
-    double2 c[kMaxE];
-    C ev[kMaxE];
+    double2 c[KE];
+    C ev[KE];
     double2 run = make_double2(0.0, 0.0);
 #pragma unroll
-    for (int e = 0; e < kMaxE; ++e) {
+    for (int e = 0; e < KE; ++e) {
         const int k = k0 + e;
         c[e] = make_double2(0.0, 0.0);
         ev[e] = Cx<T>::make(0, 0);
@@ -246,7 +255,7 @@ __device__ __forceinline__ void dst_post(typename Cx<T>::type *buf, const PlanT<
     __syncthreads();  // all reads of buf done, warp totals visible
     if (w == 1) excl = excl + wt[0];
 #pragma unroll
-    for (int e = 0; e < kMaxE; ++e) {
+    for (int e = 0; e < KE; ++e) {
         const int k = k0 + e;
         if (e < E && k < H) {
             buf[2 * k + 1] = from_d2<C>(c[e] + excl);
@@ -261,11 +270,11 @@ __device__ __forceinline__ void dst_post(typename Cx<T>::type *buf, const PlanT<
 }
 
 // Full DST-I of the packed lines in buf[1..M-1] (in place).
-template <class T>
+template <class T, int MX>
 __device__ __forceinline__ void dst_inplace(typename Cx<T>::type *buf, const PlanT<T> &pl, int t, double2 *wt) {
     dst_pre<T>(buf, pl, t);
-    fft<T>(buf, pl, t);
-    dst_post<T>(buf, pl, t, wt);
+    fft<T, MX>(buf, pl, t);
+    dst_post<T, MX>(buf, pl, t, wt);
 }
 
 }  // namespace ibpm

@@ -512,8 +512,8 @@ struct MixDst : Pow2Dst<M, T, PL> {
 };
 
 // The runtime mixed-radix transform behind the same interface (any even M <= 1024
-// of the form 2^a 3^b 5^c), unpadded.
-template <class T>
+// of the form 2^a 3^b 5^c), unpadded, for lengths up to MX.
+template <class T, int MX = kMaxM>
 struct GenericDst {
     static constexpr int OCC = 512;
     static constexpr int MC = 0;  // transform length known only at run time
@@ -524,8 +524,21 @@ struct GenericDst {
     static __host__ __device__ constexpr int smem_len(int m) { return m + 1; }
     static __device__ __forceinline__ int idx(int i) { return i; }
     static __device__ __forceinline__ void dst(C *buf, const PlanT<T> &pl, int t, double2 *wt) {
-        dst_inplace<T>(buf, pl, t, wt);
+        dst_inplace<T, MX>(buf, pl, t, wt);
     }
 };
+
+// calls f with the line transform (of element type R) of length M
+template <class R, class F>
+auto with_dst(int M, F &&f) {
+    switch (M) {
+        case 1024: return f(Pow2Dst<1024, R>{});
+        case 512: return f(Pow2Dst<512, R>{});
+        case 256: return f(Pow2Dst<256, R>{});
+        case 384: return f(MixDst<384, R>{});
+        default: break;
+    }
+    return M <= 256 ? f(GenericDst<R, 256>{}) : M <= 512 ? f(GenericDst<R, 512>{}) : f(GenericDst<R, kMaxM>{});
+}
 
 }  // namespace ibpm

@@ -395,13 +395,20 @@ __global__ void __launch_bounds__(D::TPF *NG, D::OCC / (D::TPF * NG))
             if (i <= D::MC) buf[D::idx(i)] = Cx<T>::make(za[k], zb[k]);
         }
     } else {
-        for (int i = t; i <= M; i += TPF) {
-            C z = Cx<T>::make(0, 0);
-            if (i >= 1 && i < M) {
-                if (va) z.x = (T)in(b, i, ja);
-                if (vb) z.y = (T)in(b, i, jb);
+        // loads of eight elements of both rows in flight before their stores
+        constexpr int CH = 8;
+        for (int i0 = t; i0 <= M; i0 += CH * TPF) {
+            T za[CH], zb[CH];
+#pragma unroll
+            for (int k = 0; k < CH; ++k) {
+                const int i = i0 + k * TPF;
+                const bool in_line = i >= 1 && i < M;
+                za[k] = (in_line && va) ? (T)in(b, i, ja) : (T)0;
+                zb[k] = (in_line && vb) ? (T)in(b, i, jb) : (T)0;
             }
-            buf[D::idx(i)] = z;
+#pragma unroll
+            for (int k = 0; k < CH; ++k)
+                if (i0 + k * TPF <= M) buf[D::idx(i0 + k * TPF)] = Cx<T>::make(za[k], zb[k]);
         }
     }
     __syncthreads();

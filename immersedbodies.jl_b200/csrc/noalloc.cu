@@ -111,12 +111,15 @@ inline cudaLaunchConfig_t launch_cfg(dim3 grid, dim3 block, size_t smem, cudaStr
     return c;
 }
 
-template <class D, class In, class Out>
+template <class In, class Out>
 cudaError_t xpass_na(const PlanT<double> &pl, In in, Out out, int nrows, cudaStream_t st) {
-    constexpr int NG = 2;
-    const cudaLaunchConfig_t c =
-        launch_cfg(dim3(((nrows + 1) / 2 + NG - 1) / NG, 1), dim3(NG * D::TPF), pass_smem<D>(pl.M, NG, NG), st);
-    return cudaLaunchKernelEx(&c, xpass_kernel<D, NG, In, Out>, in, out, pl, nrows, (const int *)nullptr, 0, 0, 1);
+    return with_dst<double>(pl.M, [&](auto d) {
+        using D = decltype(d);
+        constexpr int NG = D::MC > 0 ? 2 : 1;
+        const cudaLaunchConfig_t c =
+            launch_cfg(dim3(((nrows + 1) / 2 + NG - 1) / NG, 1), dim3(NG * D::TPF), pass_smem<D>(pl.M, NG, NG), st);
+        return cudaLaunchKernelEx(&c, xpass_kernel<D, NG, In, Out>, in, out, pl, nrows, (const int *)nullptr, 0, 0, 1);
+    });
 }
 
 cudaError_t tables_na(double2 *tw, double *sn, double *cs, int M, cudaStream_t st) {
@@ -182,12 +185,11 @@ int ibpm_lap_inv_noalloc(int nx, int ny, const double *b, double *x, void *strea
     const YSolve m{reinterpret_cast<const YCol *>(tab + kYTables),
                    tab + kYTables + kYColD * kNoAllocMaxM,
                    reinterpret_cast<const double2 *>(tab + kYTables + kYColD * kNoAllocMaxM + kYDiff), 0, 0};
-    using D = GenericDst<double>;
     const int ld = (nx + 3) / 4 * 4;
-    cudaError_t e = xpass_na<D>(plx, InPlain<double>{b, 0, nx - 1}, OutPlain<double>{t1, 0, ld}, ny - 1, st);
+    cudaError_t e = xpass_na(plx, InPlain<double>{b, 0, nx - 1}, OutPlain<double>{t1, 0, ld}, ny - 1, st);
     if (e == cudaSuccess) e = launch_ytri(t1, 0, ld, nx - 1, ny, 1, ytri_wshift(nx - 1, 1), m, st);
     if (e == cudaSuccess)
-        e = xpass_na<D>(plx, InPlain<double>{t1, 0, ld}, OutPlain<double>{x, 0, nx - 1}, ny - 1, st);
+        e = xpass_na(plx, InPlain<double>{t1, 0, ld}, OutPlain<double>{x, 0, nx - 1}, ny - 1, st);
     if (e != cudaSuccess) return fail(IBPM_ERR_CUDA, cudaGetErrorString(e));
     return IBPM_OK;
 }
