@@ -118,12 +118,16 @@ __global__ void bbox_kernel(Panels P, Grid g) {
 // faces: the block lists, in panel order, the panels whose support meets the
 // tile, then every face sums w * f over that list in panel order -- the same
 // accumulation order as the reference's sequential loop over panels.
+// The listed panels' places and forces sit in shared memory and eight panels'
+// weights are fetched before they are added: one at a time, each waiting for its
+// own, they were the kernel's length (a tile near the body lists some thirty).
 // f: 2np per batch (x block then y block); patch output per batch; (bx, by): the
 // tile's place in the bounding box.
 template <class T>
 __device__ __forceinline__ void reg_patch_tile(const Panels &P, const double *__restrict__ fb, T *__restrict__ out,
                                                int bx, int by) {
-    __shared__ int list[1024];
+    __shared__ int list[256], lix[256], liy[256];
+    __shared__ double lfx[256], lfy[256];
     __shared__ int warp_cnt[8];
     __shared__ int total;
     const int i0 = P.bbox[0], i1 = P.bbox[1], j0 = P.bbox[2], j1 = P.bbox[3];
@@ -135,13 +139,14 @@ __device__ __forceinline__ void reg_patch_tile(const Panels &P, const double *__
     const int li = tid % kTile, lj = tid / kTile;
     const int i = ti0 + li, j = tj0 + lj;
     double accx = 0.0, accy = 0.0;
-    int base = 0;
     for (int c0 = 0; c0 < P.np; c0 += 256) {
         if (tid == 0) total = 0;
         const int p = c0 + tid;
         bool hit = false;
+        int ix = 0, iy = 0;
         if (p < P.np) {
-            const int ix = P.pc[2 * p], iy = P.pc[2 * p + 1];
+            ix = P.pc[2 * p];
+            iy = P.pc[2 * p + 1];
             hit = ix + 3 >= ti0 && ix - 3 <= ti1 && iy + 3 >= tj0 && iy - 3 <= tj1;
         }
         const unsigned m = __ballot_sync(0xffffffffu, hit);
@@ -149,24 +154,46 @@ __device__ __forceinline__ void reg_patch_tile(const Panels &P, const double *__
         __syncthreads();
         int off = 0;
         for (int k = 0; k < w; ++k) off += warp_cnt[k];
-        if (hit) list[off + __popc(m & ((1u << lane) - 1))] = p;
+        if (hit) {
+            const int at = off + __popc(m & ((1u << lane) - 1));
+            list[at] = p;
+            lix[at] = ix;
+            liy[at] = iy;
+            lfx[at] = fb[p];
+            lfy[at] = fb[P.np + p];
+        }
         if (tid == 255) {
             int s = 0;
             for (int k = 0; k < 8; ++k) s += warp_cnt[k];
             total = s;
         }
         __syncthreads();
-        (void)base;
         const int n = total;
         if (i <= ti1 && j <= tj1) {
-            for (int k = 0; k < n; ++k) {
-                const int q = list[k];
-                const int ix = P.pc[2 * q], iy = P.pc[2 * q + 1];
-                const int da = i - ix + 3, db = j - iy + 3;
-                if (da >= 0 && da < 7 && db >= 0 && db < 7) {
-                    accx = accx + P.w[(long long)(q * 2) * 49 + db * 7 + da] * fb[q];
-                    accy = accy + P.w[(long long)(q * 2 + 1) * 49 + db * 7 + da] * fb[P.np + q];
+            constexpr int U = 8;
+            for (int k0 = 0; k0 < n; k0 += U) {
+                double wx[U], wy[U];
+                bool in[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int k = k0 + u;
+                    in[u] = false;
+                    if (k < n) {
+                        const int da = i - lix[k] + 3, db = j - liy[k] + 3;
+                        in[u] = da >= 0 && da < 7 && db >= 0 && db < 7;
+                        if (in[u]) {
+                            const double *w0 = P.w + (long long)(list[k] * 2) * 49 + db * 7 + da;
+                            wx[u] = __ldg(w0);
+                            wy[u] = __ldg(w0 + 49);
+                        }
+                    }
                 }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (in[u]) {
+                        accx = accx + wx[u] * lfx[k0 + u];
+                        accy = accy + wy[u] * lfy[k0 + u];
+                    }
             }
         }
         __syncthreads();
