@@ -31,6 +31,31 @@ struct Cx<float> {
     static __host__ __device__ __forceinline__ float2 make(float a, float b) { return make_float2(a, b); }
 };
 
+// Programmatic dependent launch: a kernel that begins with overlap_begin() may be
+// launched (launch_overlapped) while the kernel before it in the stream still
+// runs; it lets its own successor in and then waits for its predecessor's end and
+// writes.  Launched without the attribute both are no-ops.
+__device__ __forceinline__ void overlap_begin() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// Launches k on st, overlapped with its predecessor if wanted; the return code is
+// the launch's own.
+template <class... P, class... A>
+cudaError_t launch_overlapped(bool overlap, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
+
 struct Grid {
     int nx, ny, L;
     double h, x0, y0, Re, dt;

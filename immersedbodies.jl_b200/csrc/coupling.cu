@@ -207,6 +207,7 @@ __device__ __forceinline__ void reg_patch_tile(const Panels &P, const double *__
 template <class T>
 __global__ void __launch_bounds__(256) reg_patch_kernel(Panels P, const double *__restrict__ f, long long fbs,
                                                         T *__restrict__ patch, long long pbs) {
+    overlap_begin();
     const int b = blockIdx.z;
     // the blocks walk the tiles of the bounding box (its size is known on the device only)
     const int pw = P.bbox[1] - P.bbox[0] + 1, ph = P.bbox[3] - P.bbox[2] + 1;
@@ -262,6 +263,7 @@ template <class T>
 __global__ void __launch_bounds__(32 * kRegTWarps) regT_kernel(Panels P, const T *__restrict__ q, long long qbs,
                                                                 double *__restrict__ out, long long obs, int nbatch,
                                                                 int add_q0, const StepDev *__restrict__ prm, Grid g) {
+    overlap_begin();
     __shared__ double prod[kRegTWarps][49];
     const int t = blockIdx.x * kRegTWarps + (threadIdx.x >> 5);
     const int np = P.np;
@@ -316,15 +318,16 @@ static int patch_grid(int n, int nbatch) {
 
 template <class T>
 void launch_reg_patch(const Panels &P, const double *f, long long fbs, T *patch, long long pbs, int nbatch,
-                      const Grid &g, cudaStream_t st) {
-    reg_patch_kernel<T><<<dim3(patch_grid(g.nx, nbatch), patch_grid(g.ny, nbatch), nbatch), 256, 0, st>>>(P, f, fbs, patch, pbs);
+                      const Grid &g, cudaStream_t st, bool overlap) {
+    launch_overlapped(overlap, reg_patch_kernel<T>, dim3(patch_grid(g.nx, nbatch), patch_grid(g.ny, nbatch), nbatch), dim3(256), 0,
+                      st, P, f, fbs, patch, pbs);
 }
 template <class T>
 void launch_regT(const Panels &P, const T *q, long long qbs, double *out, long long obs, int nbatch, int add_q0,
-                 const StepDev *prm, const Grid &g, cudaStream_t st) {
+                 const StepDev *prm, const Grid &g, cudaStream_t st, bool overlap) {
     const int nt = 2 * P.np * nbatch;
-    regT_kernel<T><<<(nt + kRegTWarps - 1) / kRegTWarps, 32 * kRegTWarps, 0, st>>>(P, q, qbs, out, obs, nbatch,
-                                                                                  add_q0, prm, g);
+    launch_overlapped(overlap, regT_kernel<T>, dim3((nt + kRegTWarps - 1) / kRegTWarps), dim3(32 * kRegTWarps), 0, st, P, q, qbs,
+                      out, obs, nbatch, add_q0, prm, g);
 }
 template <class T>
 void launch_reg_patch_multi(const CaseView *tab, int ncase, const Grid &g, cudaStream_t st) {
@@ -343,13 +346,13 @@ template void launch_regT_multi<double>(const CaseView *, int, int, const double
 template void launch_regT_multi<float>(const CaseView *, int, int, const float *, long long, const StepDev *,
                                        const Grid &, cudaStream_t);
 template void launch_reg_patch<double>(const Panels &, const double *, long long, double *, long long, int,
-                                       const Grid &, cudaStream_t);
+                                       const Grid &, cudaStream_t, bool);
 template void launch_reg_patch<float>(const Panels &, const double *, long long, float *, long long, int,
-                                      const Grid &, cudaStream_t);
+                                      const Grid &, cudaStream_t, bool);
 template void launch_regT<double>(const Panels &, const double *, long long, double *, long long, int, int,
-                                  const StepDev *, const Grid &, cudaStream_t);
+                                  const StepDev *, const Grid &, cudaStream_t, bool);
 template void launch_regT<float>(const Panels &, const float *, long long, double *, long long, int, int,
-                                 const StepDev *, const Grid &, cudaStream_t);
+                                 const StepDev *, const Grid &, cudaStream_t, bool);
 void launch_rigid_motion(const Panels &P, const double *ref_xb, const double *motion, int p0, int p1,
                          cudaStream_t st) {
     if (p1 > p0) rigid_motion_kernel<<<(p1 - p0 + 127) / 128, 128, 0, st>>>(P, ref_xb, motion, p0, p1);

@@ -505,6 +505,11 @@ struct Engine final : ibpm_handle {
     // ---- line passes ----
     // Dispatch on the transform length: compile-time transforms for
     // M in {256, 384, 512, 1024}, the runtime mixed-radix one otherwise.
+    // Whether a launch over nb fields overlaps its predecessor's end
+    // (launch_overlapped): groups and batches, whose last waves leave room (a step of
+    // 16 FP64 cases 546 -> 497 us); one field's chain of small kernels gains nothing
+    // (200^2 x 3 132 -> 139 us).  Not in conditional graph bodies.
+    bool overlap(int nb) const { return nb >= 4 && st != st_side; }
     // The rows an X pass covers: see xpass_kernel (rows null: every row)
     struct XOpt {
         const int *rows = nullptr;
@@ -524,8 +529,8 @@ struct Engine final : ibpm_handle {
             constexpr int NG = D::MC > 0 ? kNG : 1;
             const int pairs = (nrows + 1) / 2;
             const dim3 grid((pairs + NG - 1) / NG, nbatch);
-            xpass_kernel<D, NG, In, Out><<<grid, NG * D::TPF, pass_smem<D>(pl.M, NG, NG), st>>>(
-                in, out, pl, nrows, o.rows, o.zero_outside, o.rows_stride, o.rows_mod);
+            CK(launch_overlapped(overlap(nbatch), xpass_kernel<D, NG, In, Out>, grid, dim3(NG * D::TPF), pass_smem<D>(pl.M, NG, NG),
+                                 st, in, out, pl, nrows, o.rows, o.zero_outside, o.rows_stride, o.rows_mod));
         });
         check_launch();
         prof_end(pe, IBPM_KCLASS_XPASS, 2.0 * sizeof(R) * (double)ng * nbatch);
@@ -537,8 +542,9 @@ struct Engine final : ibpm_handle {
         with_dst<T>(plx.M, [&](auto d) {
             using D = decltype(d);
             constexpr int NB = 64 / D::TPF;
-            xlines_kernel<D><<<dim3(1 + (ny / 2 + nx + 1) / 2, nbatch), 64, pass_smem<D>(plx.M, NB, NB), st>>>(
-                in, ring_out(), plx, line_w, line_w + nx, psi_, pbs, win, win_stride);
+            CK(launch_overlapped(overlap(nbatch), xlines_kernel<D>, dim3(1 + (ny / 2 + nx + 1) / 2, nbatch), dim3(64),
+                                 pass_smem<D>(plx.M, NB, NB), st, in, ring_out(), plx, line_w, line_w + nx, psi_, pbs, win,
+                                 win_stride));
         });
         check_launch();
         prof_end(pe, IBPM_KCLASS_XPASS, 0.5 * sizeof(T) * (double)ng * nbatch);
@@ -567,7 +573,7 @@ struct Engine final : ibpm_handle {
     }
     void ypass_launch(int ngy, double *f, int nbatch, const YSolve &m, long long bs, const YRing &ring = {}) {
         const int wshift = ngy <= 1 ? 1 : ngy == 2 ? 2 : 3;  // at most kYMaxW columns a block
-        CK(launch_ytri(f, bs, ldt, nx - 1, ny, nbatch, wshift, m, st, ring));
+        CK(launch_ytri(f, bs, ldt, nx - 1, ny, nbatch, wshift, m, st, ring, overlap(nbatch)));
     }
     // by transforms; c null: the Laplacian inverse
     template <class R>
@@ -840,8 +846,8 @@ struct Engine final : ibpm_handle {
         for (int lev = 2; lev <= L; ++lev) {
             const int nx2 = nx / 2, ny2 = ny / 2;
             const dim3 blk(16, 16), grd((nx2 + 15) / 16, (ny2 + 15) / 16, nbatch);
-            coarsify_kernel<<<grd, blk, 0, st>>>(Gm + (lev - 1) * ng, Gm + (lev - 2) * ng, bs, g,
-                                                 central && lev - 1 >= 2 ? 1 : 0);
+            CK(launch_overlapped(overlap(nbatch), coarsify_kernel<T, T>, grd, blk, 0, st, Gm + (lev - 1) * ng, Gm + (lev - 2) * ng, bs, g,
+                                 central && lev - 1 >= 2 ? 1 : 0));
             check_launch();
         }
         if constexpr (std::is_same<T, double>::value) {
@@ -931,7 +937,8 @@ struct Engine final : ibpm_handle {
         if (curl_all)  // batch and level strides agree: fields are case-major
             curl_kernel<T, T, T><<<grd, blk, 0, st>>>(qout, nq, psi_, ng, L > 1 ? psi_ + ng : nullptr, ng, g, nullptr, L);
         else
-            curl_kernel<T, T, T><<<grd, blk, 0, st>>>(qout, qbs, psi_, bs, L > 1 ? psi_ + ng : nullptr, bs, g, win);
+            CK(launch_overlapped(overlap(nbatch), curl_kernel<T, T, T>, grd, blk, 0, st, qout, qbs, psi_, bs,
+                                 L > 1 ? psi_ + ng : nullptr, bs, g, win, 1, nullptr));
         check_launch();
         prof_end(pe, IBPM_KCLASS_CURL, 8.0 * (double)(ng + nq) * grd.z);
     }
@@ -967,7 +974,7 @@ struct Engine final : ibpm_handle {
 
     // Regularisation patch of nbatch force vectors f (stride 2np).
     void reg_patch(const double *f, int nbatch) {
-        launch_reg_patch(P, f, 2 * np, patch, patch_stride, nbatch, g, st);
+        launch_reg_patch(P, f, 2 * np, patch, patch_stride, nbatch, g, st, overlap(nbatch));
         check_launch();
     }
 
@@ -992,7 +999,7 @@ struct Engine final : ibpm_handle {
         }
         // E reads the bbox only; Gw's coarse levels are zero outside coarsify!'s block
         vort2flux(psiw, qw, Gw, ng * L, nq, nbatch, false, false, P.bbox, true);
-        launch_regT(P, qw, nq, x, xs, nbatch, 0, prm, g, st);
+        launch_regT(P, qw, nq, x, xs, nbatch, 0, prm, g, st, overlap(nbatch));
         check_launch();
     }
 

@@ -267,6 +267,7 @@ __global__ void __launch_bounds__(64)
     xlines_kernel(InPlain<typename D::Real> in, RingOut ro, PlanT<typename D::Real> pl, const double *__restrict__ wl,
                   const double *__restrict__ wr, typename D::Real *psi, long long pbs, const int *__restrict__ win,
                   int win_stride) {
+    overlap_begin();
     using T = typename D::Real;
     using C = typename D::C;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -345,6 +346,7 @@ template <class D, int NG, class In, class Out>
 __global__ void __launch_bounds__(D::TPF *NG, D::OCC / (D::TPF * NG))
     xpass_kernel(In inp, Out out, PlanT<typename D::Real> pl, int nrows, const int *__restrict__ rows = nullptr,
                  int zero_outside = 0, int rows_stride = 0, int rows_mod = 1) {
+    overlap_begin();
     const int bx = blockIdx.x;
     if (rows != nullptr) {  // uniform over the block: before any barrier
         rows += (long long)rows_stride * (blockIdx.y % rows_mod);
@@ -1080,6 +1082,7 @@ template <class T, class TP, class TC, bool CHECK = false>
 __global__ void curl_kernel(T *__restrict__ qout, long long qbs, const TP *__restrict__ psi, long long bs,
                             const TC *__restrict__ coarse, long long cbs, Grid g, const int *__restrict__ win = nullptr,
                             int nl = 1, int *differs = nullptr) {
+    overlap_begin();
     const int nx = g.nx, ny = g.ny;
     const long long nu = (long long)(nx + 1) * ny;
     const int b = blockIdx.z;
@@ -1149,6 +1152,7 @@ __global__ void curl_kernel(T *__restrict__ qout, long long qbs, const TP *__res
 template <class T, class TF = T>
 __global__ void coarsify_kernel(T *__restrict__ coarse, const TF *__restrict__ fine, long long bs, Grid g,
                                 int fine_central = 0) {
+    overlap_begin();
     const int nx = g.nx, ny = g.ny;
     const int ni = (nx / 2 - 2 - (-nx / 2 + 2)) / 2 + 1, nic = (nx / 4 - 1) - (-nx / 4 + 1) + 1;
     const int nj = (ny / 2 - 2 - (-ny / 2 + 2)) / 2 + 1, njc = (ny / 4 - 1) - (-ny / 4 + 1) + 1;

@@ -109,6 +109,7 @@ struct YSolve {
 template <int MR, bool RING>
 __global__ void __launch_bounds__(kYChunks *kYMaxW)
     ytri_kernel(double *f, long long bs, int ld, int ncols, int M, int wshift, YSolve ys, YRing yr) {
+    overlap_begin();
     constexpr int kPad = kYMaxW * (kYChunks + 2);
     // chunk totals, then starts of P and Q; r^(row) of the homogeneous terms.  Row
     // stride 64 + 16 / W: the threads' stores and the scan's 16-byte loads are free
@@ -411,12 +412,11 @@ inline cudaError_t launch_ycols(YCol *cols, double *diff, double2 *phase, const 
 // Enqueues the Y solve, in place, of nbatch fields with 1 << wshift columns a block; the
 // return code is the launch's own.
 inline cudaError_t launch_ytri(double *f, long long bs, int ld, int ncols, int M, int nbatch, int wshift,
-                               const YSolve &ys, cudaStream_t st, const YRing &yr = {}) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((ncols + (1 << wshift) - 1) >> wshift, nbatch);
-    cfg.blockDim = dim3(kYChunks << wshift);
-    cfg.stream = st;
-    auto go = [&](auto *k) { return cudaLaunchKernelEx(&cfg, k, f, bs, ld, ncols, M, wshift, ys, yr); };
+                               const YSolve &ys, cudaStream_t st, const YRing &yr = {}, bool overlap = false) {
+    auto go = [&](auto *k) {
+        return launch_overlapped(overlap, k, dim3((ncols + (1 << wshift) - 1) >> wshift, nbatch), dim3(kYChunks << wshift), 0,
+                                 st, f, bs, ld, ncols, M, wshift, ys, yr);
+    };
     switch (ytri_rows(M)) {
         case 1: return yr.lines ? go(ytri_kernel<1, true>) : go(ytri_kernel<1, false>);
         case 2: return yr.lines ? go(ytri_kernel<2, true>) : go(ytri_kernel<2, false>);
