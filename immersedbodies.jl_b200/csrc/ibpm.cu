@@ -9,8 +9,10 @@
 //   _cycle!), panels, F~b, fb.  q0 is never stored on the hot path: every
 //   consumer evaluates base_flux! per face; it is materialised only for
 //   ibpm_get_state.
-// One step (advance!, src/solver.jl:155-190) is ~60 kernels on one stream;
-// each 2D DST solve is three line passes (see fft_dst.cuh).
+// The step stores no q: the nonlinear term forms its faces from psi, and q is
+// materialised when it is asked for.  One step (advance!, src/solver.jl:155-190)
+// is 30 to 40 kernels on one stream; each 2D DST solve is three line passes (see
+// fft_dst.cuh).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -290,6 +292,7 @@ struct Engine final : ibpm_handle {
     // after the copies that read it have run (asynchronous copies read pinned
     // host memory when they execute, not when they are enqueued).
     static constexpr int kStage = 8;
+    char *pinned = nullptr;  // the handle's pinned host memory: what these, cg_s_h and err_h point into
     StepDev *stage_prm[kStage] = {};
     double *stage_motion[kStage] = {};
     cudaEvent_t stage_ev[kStage] = {};
@@ -390,6 +393,44 @@ struct Engine final : ibpm_handle {
     }
     std::vector<void *> allocs;
     std::vector<long long> alloc_bytes;  // size of each entry of allocs
+    // Device memory that several of the handle's allocations share: a block goes
+    // back when its last one is freed.  An allocation or a release costs the host
+    // 0.05-0.4 ms whatever its size, and a handle makes some sixty: creating and
+    // closing a 256^2 x 3 handle took 22.3 ms, 14.3 with blocks for the fields, the
+    // column work (each freed together) and the rest.  Nothing is carved twice, so
+    // freed ranges are never handed out again while their block lives.
+    struct Block {
+        char *base = nullptr;
+        size_t size = 0, used = 0;
+        int live = 0;
+    };
+    std::vector<Block> blocks;
+    int open_block = -1;  // the block dalloc carves from (none: allocations of their own)
+    static size_t carved(size_t bytes) { return (std::max<size_t>(bytes, 1) + 511) & ~(size_t)511; }
+    // opens a block of the given bytes (sizes rounded by carved()); returns the one
+    // open before, for open_block to be set back to
+    int reserve(size_t bytes) {
+        void *p = nullptr;
+        if (cudaMalloc(&p, bytes) != cudaSuccess) {
+            (void)cudaGetLastError();  // not sticky: clear it so later launch checks do not report it
+            throw ApiError{IBPM_ERR_NOMEM, "cudaMalloc of " + std::to_string(bytes) + " bytes failed"};
+        }
+        size_t i = 0;
+        while (i < blocks.size() && blocks[i].base) ++i;
+        if (i == blocks.size()) blocks.emplace_back();
+        blocks[i].base = static_cast<char *>(p);
+        blocks[i].size = bytes;
+        blocks[i].used = 0;
+        blocks[i].live = 0;
+        const int before = open_block;
+        open_block = (int)i;
+        return before;
+    }
+    Block *block_of(void *p) {
+        for (Block &b : blocks)
+            if (b.base && p >= b.base && p < b.base + b.size) return &b;
+        return nullptr;
+    }
     // frees one allocation of this handle
     void dfree(void *p) {
         if (!p) return;
@@ -399,6 +440,12 @@ struct Engine final : ibpm_handle {
             dev_bytes -= alloc_bytes[i];
             alloc_bytes.erase(alloc_bytes.begin() + (long)i);
             allocs.erase(it);
+        }
+        if (Block *b = block_of(p)) {
+            if (--b->live > 0) return;
+            if (open_block == (int)(b - blocks.data())) open_block = -1;
+            p = b->base;
+            b->base = nullptr;
         }
         cudaFree(p);
     }
@@ -422,13 +469,18 @@ struct Engine final : ibpm_handle {
                                  sizeof(T) * (size_t)(ng * L * kb), sizeof(T) * (size_t)(ng * L * kb),
                                  sizeof(T) * (size_t)(nq * kb),     sizeof(double) * 2 * (size_t)np * kb,
                                  sizeof(double) * (size_t)(line_len() * kb)};
+        size_t total_bytes = 0;
+        for (size_t s : sizes) total_bytes += carved(s);
         void *fresh[7] = {};
+        const int before = reserve(total_bytes);
         try {
             for (int k = 0; k < 7; ++k) fresh[k] = dalloc<unsigned char>(sizes[k]);
         } catch (...) {
+            open_block = before;
             for (void *p : fresh) dfree(p);
             throw;
         }
+        open_block = before;
         drop_graphs();
         for (void *p : {(void *)t1, (void *)patch, (void *)Gw, (void *)psiw, (void *)qw, (void *)fcol, (void *)lines})
             dfree(p);
@@ -447,8 +499,12 @@ struct Engine final : ibpm_handle {
     U *dalloc(size_t n) {
         void *p = nullptr;
         if (n == 0) n = 1;
-        cudaError_t e = cudaMalloc(&p, n * sizeof(U));
-        if (e != cudaSuccess) {
+        Block *b = open_block < 0 ? nullptr : &blocks[(size_t)open_block];
+        if (b && b->used + carved(n * sizeof(U)) <= b->size) {
+            p = b->base + b->used;
+            b->used += carved(n * sizeof(U));
+            ++b->live;
+        } else if (cudaMalloc(&p, n * sizeof(U)) != cudaSuccess) {
             (void)cudaGetLastError();  // not sticky: clear it so later launch checks do not report it
             throw ApiError{IBPM_ERR_NOMEM, "cudaMalloc of " + std::to_string(n * sizeof(U)) + " bytes failed"};
         }
@@ -478,14 +534,13 @@ struct Engine final : ibpm_handle {
         drop_graphs();
         if (tc) tc_destroy(tc);
         for (cudaEvent_t e : ev_pool) cudaEventDestroy(e);
-        for (void *p : allocs) cudaFree(p);
-        for (int k = 0; k < kStage; ++k) {
-            if (stage_prm[k]) cudaFreeHost(stage_prm[k]);
-            if (stage_motion[k]) cudaFreeHost(stage_motion[k]);
+        for (void *p : allocs)
+            if (!block_of(p)) cudaFree(p);
+        for (Block &b : blocks)
+            if (b.base) cudaFree(b.base);
+        for (int k = 0; k < kStage; ++k)
             if (stage_ev[k]) cudaEventDestroy(stage_ev[k]);
-        }
-        if (cg_s_h) cudaFreeHost(cg_s_h);
-        if (err_h) cudaFreeHost(err_h);
+        if (pinned) cudaFreeHost(pinned);
         if (st_side) cudaStreamDestroy(st_side);
         if (st) cudaStreamDestroy(st);
     }
@@ -1128,6 +1183,17 @@ void Engine<T>::setup() {
     CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     if (!make_plan(nx, plx) || !make_plan(ny, ply))
         throw ApiError{IBPM_ERR_INVALID, "nx and ny must be even, <= 1024 and of the form 2^a 3^b 5^c"};
+    // What the setup allocates besides the fields and the column work: the larger
+    // ones by size, half a megabyte for the tables and the panels' small arrays (what
+    // does not fit gets memory of its own)
+    {
+        const bool f32 = !std::is_same<T, double>::value;
+        const size_t n = 2 * (size_t)np, g = (size_t)ng, f = (size_t)nq;
+        const bool dense = static_bodies || (!f32 && n <= (size_t)kDenseN);
+        reserve(sizeof(T) * ((size_t)nt + (f32 ? 2 : 1) * g * L + f) + (f32 ? sizeof(double) * (g + f + (size_t)nt) : 0) +
+                sizeof(double) * ((size_t)ring_ld() * (nx - 1) + (n + 63) / 64 * n + 2 * 49 * n + (dense ? n * n : 0)) +
+                sizeof(YCol) * (size_t)(nx - 1) * (L + 1) + ((size_t)1 << 19));
+    }
     // transform tables
     auto tables = [&](int M, C *&tw, T *&sn, double *&cs, PlanT<T> &pl) {
         std::vector<C> htw(M);
@@ -1209,12 +1275,15 @@ void Engine<T>::setup() {
         }
     }
 
+    // the fields, which go back together when an ensemble takes them over
+    const int rest_block = reserve(carved(sizeof(T) * nq * L) + 5 * carved(sizeof(T) * ng * L));
     q = dalloc<T>(nq * L);
     psi = dalloc<T>(ng * L);
     G[0] = dalloc<T>(ng * L);
     G[1] = dalloc<T>(ng * L);
     nl[0] = dalloc<T>(ng * L);
     nl[1] = dalloc<T>(ng * L);
+    open_block = rest_block;
     P.np = np;
     P.xb = dalloc<double>(2 * np);
     P.ub = dalloc<double>(2 * np);
@@ -1230,16 +1299,21 @@ void Engine<T>::setup() {
     total = dalloc<double>(2);
     prm = dalloc<StepDev>(1);
     motion = dalloc<double>(6 * (size_t)std::max(nbody, 1));
+    const size_t prm_room = carved(sizeof(StepDev)), motion_room = carved(sizeof(double) * 6 * std::max(nbody, 1));
+    CK(cudaMallocHost(&pinned, kStage * (prm_room + motion_room) + 2 * carved(sizeof(double) * 8)));
+    char *pin = pinned;
     for (int k = 0; k < kStage; ++k) {
-        CK(cudaMallocHost(&stage_prm[k], sizeof(StepDev)));
-        CK(cudaMallocHost(&stage_motion[k], sizeof(double) * 6 * std::max(nbody, 1)));
+        stage_prm[k] = reinterpret_cast<StepDev *>(pin);
+        pin += prm_room;
+        stage_motion[k] = reinterpret_cast<double *>(pin);
+        pin += motion_room;
         CK(cudaEventCreateWithFlags(&stage_ev[k], cudaEventDisableTiming));
         memset(stage_prm[k], 0, sizeof(StepDev));
     }
     prm_h = stage_prm[0];
     motion_h = stage_motion[0];
-    CK(cudaMallocHost(&cg_s_h, sizeof(double) * 8));
-    CK(cudaMallocHost(&err_h, sizeof(int) * 8));
+    cg_s_h = reinterpret_cast<double *>(pin);
+    err_h = reinterpret_cast<int *>(pin + carved(sizeof(double) * 8));
     memset(prm_h, 0, sizeof(StepDev));
     CK(cudaMemcpyAsync(ref_xb_d, ref_xb.data(), sizeof(double) * 2 * np, cudaMemcpyHostToDevice, st));
 
@@ -1248,10 +1322,21 @@ void Engine<T>::setup() {
     if (!static_bodies) kbatch = moving_batch();
     kbatch = std::min(kbatch, 2 * np);
     const int kb = std::max(kbatch, L);
+    patch_stride = 2LL * (nx + 1) * (ny + 1);
+    // the column work, which goes back together (resize_batch_buffers)
+    reserve(carved(sizeof(T) * nt * kb) + carved(sizeof(double) * line_len() * kbatch) +
+            carved(sizeof(T) * patch_stride * kbatch) + 2 * carved(sizeof(T) * ng * L * kbatch) +
+            carved(sizeof(T) * nq * kbatch) + carved(sizeof(double) * 2 * (size_t)np * kbatch));
     t1 = dalloc<T>(nt * kb);
     t1_fields = kb;
-    if (!std::is_same<T, double>::value) t2 = dalloc<T>(ng * L);
     lines = dalloc<double>(line_len() * kbatch);
+    patch = dalloc<T>(patch_stride * kbatch);
+    Gw = dalloc<T>(ng * L * kbatch);
+    psiw = dalloc<T>(ng * L * kbatch);
+    qw = dalloc<T>(nq * kbatch);
+    fcol = dalloc<double>(2 * (size_t)np * kbatch);
+    open_block = rest_block;
+    if (!std::is_same<T, double>::value) t2 = dalloc<T>(ng * L);
     rhs = dalloc<T>(nt);
     rest = dalloc<T>(ng * L);
     qs1 = dalloc<T>(nq);
@@ -1273,12 +1358,6 @@ void Engine<T>::setup() {
     }
     const int nchunk = (2 * np + 63) / 64;
     part = dalloc<double>((size_t)nchunk * 2 * np);
-    patch_stride = 2LL * (nx + 1) * (ny + 1);
-    patch = dalloc<T>(patch_stride * kbatch);
-    Gw = dalloc<T>(ng * L * kbatch);
-    psiw = dalloc<T>(ng * L * kbatch);
-    qw = dalloc<T>(nq * kbatch);
-    fcol = dalloc<double>(2 * (size_t)np * kbatch);
     if (!static_bodies && std::is_same<T, double>::value && 2 * np <= kDenseN) Bd = dalloc<double>(4 * (size_t)np * np);
     cg_u = dalloc<double>(2 * np);
     cg_z = dalloc<double>(2 * np);
@@ -1347,6 +1426,7 @@ void Engine<T>::setup() {
             CK(cudaMemcpy(Binv, e64.Binv, sizeof(double) * n * n, cudaMemcpyDeviceToDevice));
         }
     }
+    open_block = -1;
     CK(cudaStreamSynchronize(st));
 }
 
@@ -1370,8 +1450,11 @@ int Engine<T>::moving_batch() const {
 template <class T>
 void Engine<T>::build_Binv() {
     const int n = 2 * np;
+    int closed = -1;
     Binv = dalloc<double>((size_t)n * n);
+    std::swap(open_block, closed);  // freed below: memory of its own
     Bwork = dalloc<double>((size_t)n * n);
+    std::swap(open_block, closed);
     assemble_invert_B();
     CK(cudaMemcpyAsync(err_h, err, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
