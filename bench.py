@@ -56,16 +56,13 @@ def step_bytes_model(nx: int, ny: int, L: int, npanel: int, s: float = 1.0) -> f
             + 8.0 * (2 * npanel) ** 2)
 
 
-# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the
-# dominant kernel classes, each from one ncu capture (constants, not measured by
-# this run); the command of each capture is in NCU_TRAFFIC_RUN.
-NCU_TRAFFIC = {"ypass": 8454912.0, "xpass": 8417792.0}
-NCU_TRAFFIC_RUN = {"ypass": "ncu --set full --clock-control none -k regex:ypass_kernel -s 210 -c 1 python bench.py "
-                            "--steps 1 --warmup 3 --no-cpu-baseline --no-chosen --no-learned --no-ensemble: one "
-                            "single-level launch (1023^2 FP64), cold-cache replay",
-                   "xpass": "ncu --set full --clock-control none --nvtx --nvtx-include timed/ -k regex:xpass_kernel "
-                            "-s 1 -c 1 python bench.py --steps 2 --warmup 3 --no-cpu-baseline --no-chosen --no-learned "
-                            "--no-ensemble: one single-level launch (1023^2 FP64, vort2flux level 5), cold-cache replay"}
+# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum), the mean
+# over a class's launches in two steps, from one ncu capture (constants, not
+# measured by this run); the capture's command is NCU_TRAFFIC_RUN.
+NCU_TRAFFIC = {"ypass": 11.35e6, "xpass": 18.6e6}
+NCU_TRAFFIC_RUN = ("ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum --clock-control none "
+                   "--nvtx --nvtx-include timed/ -c 120 python bench.py --steps 2 --warmup 3 --no-cpu-baseline "
+                   "--no-chosen --no-learned --no-ensemble: every launch of two steps, cold-cache replay")
 
 
 def read_peaks():
@@ -607,8 +604,9 @@ def main():
     peak, peak_kind = read_peaks()
     # the dominant kernel: the class with the largest device time per step; its
     # achieved bandwidth is the algorithmic bytes of all its launches over their time
-    names = {"ypass": "ypass_kernel (DST along y, multiply by scale/Λ, DST along y)",
-             "xpass": "xpass_kernel (DST along x of row pairs, with the solves' prologues and epilogues)",
+    names = {"ypass": "ytri_kernel (the multiplier scale/Λ along y as a direct solve per column)",
+             "xpass": "xpass_kernel (DST along x of row pairs, with the solves' prologues and epilogues) and xlines_kernel "
+                      "(the next finer level's boundary values)",
              "nonlinear": "nonlinear_kernel", "curl": "curl_kernel", "xtrial": "xpass_trial_kernel",
              "ytrial": "ypass_trial_kernel"}
     dom_key = max(kern, key=lambda k: kern[k][1])
@@ -619,7 +617,7 @@ def main():
     n_y, ms_y, b_y = kern["ypass"]
     roofline = {"kernel": names[dom_key], "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak if achieved else None, "traffic": traffic,
-                "traffic_source": traffic and NCU_TRAFFIC_RUN.get(dom_key),
+                "traffic_source": traffic and NCU_TRAFFIC_RUN,
                 "peak_source": peak_kind,
                 "launches_per_step": n_d / prof_steps if n_d else None,
                 "algorithmic_bytes_per_launch": b_d / n_d if n_d else None,
@@ -693,7 +691,7 @@ def main():
                 "chosen_form": chosen, "chosen_form_plate_aoa30": plate32, "learned_warm_start": learned,
                 "tensor_core_rebuild": tcore, "ensemble": ensemble,
                 "autotune": {"table": ib._abi.tune_table(),
-                             "what": "Y-pass line pairs per block chosen by timing per (GPU, transform length, "
+                             "what": "Y-pass column pairs per block chosen by timing per (GPU, transform length, "
                                      "precision, batch bucket); every choice gives the same bits"}}
         print(json.dumps(line), flush=True)
     if pg:

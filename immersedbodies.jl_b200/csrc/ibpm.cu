@@ -11,7 +11,7 @@
 //   ibpm_get_state.
 // The step stores no q: the nonlinear term forms its faces from psi, and q is
 // materialised when it is asked for.  One step (advance!, src/solver.jl:155-190)
-// is 30 to 40 kernels on one stream; each 2D DST solve is three line passes (see
+// is 30 to 45 kernels on one stream; each 2D DST solve is three line passes (see
 // fft_dst.cuh).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>

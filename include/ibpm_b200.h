@@ -178,13 +178,14 @@ const char *ibpm_ensemble_last_error(const ibpm_ensemble *e);
 int ibpm_ensemble_groups(const ibpm_ensemble *e, int32_t *ngroups, int32_t *nbatched);
 
 /* Pass-shape autotuner (no counterpart in the reference).  The Y pass of the
- * DST-diagonalised solves runs with NG line pairs (2 NG columns) per block, NG
- * in {1, 2, 4, 8}; every NG gives the same bits.  With the environment variable
+ * DST-diagonalised solves runs with NG column pairs per block, NG in {1, 2, 4, 8}
+ * (the FP64 engine's direct y solve runs 8 as 4); every NG gives the same bits.  With the environment variable
  * IBPM_TUNE=1, engines (and ensemble groups) time every NG on the device for
  * each (GPU, transform length, precision, batch bucket) they launch, before
  * their first step, and keep the fastest; IBPM_TUNE_CACHE=<file> reads the table
  * from that file at first use and appends new choices to it.  Untuned keys use
- * NG = 2 (4 from 16 fields per launch).  IBPM_TUNE_FORCE_NG=<n> forces one NG.
+ * a fixed rule on the columns per launch (FP32 and mixed: NG = 2, or 4 from 16
+ * fields per launch).  IBPM_TUNE_FORCE_NG=<n> forces one NG.
  * ibpm_tune_table writes the table as text lines "key NG" into out (len bytes,
  * NUL-terminated) and returns the length it needs. */
 int ibpm_tune_table(char *out, int32_t len);
@@ -204,11 +205,12 @@ int64_t ibpm_kernel_launches(const ibpm_handle *h);
  * launches, summed device time (ms) and algorithmic bytes (one read of each
  * input field and one write of each output field) of a class. */
 #define IBPM_KCLASS_XPASS 0         /* DST along x (row pass) */
-#define IBPM_KCLASS_YPASS 1         /* DST along y, spectral multiply, DST along y */
+#define IBPM_KCLASS_YPASS 1         /* the multiplier along y: FP64 a direct solve per column, else DST,
+                                       multiply, DST */
 #define IBPM_KCLASS_NONLINEAR 2     /* nonlinear advection term */
-#define IBPM_KCLASS_CURL 3          /* curl of the streamfunction */
-#define IBPM_KCLASS_XTRIAL 4        /* trial solve, first X pass (all levels) */
-#define IBPM_KCLASS_YTRIAL 5        /* trial solve, Y pass with the A/Ainv multiplies (all levels) */
+#define IBPM_KCLASS_CURL 3          /* curl of the streamfunction (the step's: level 1, inside the body's box) */
+#define IBPM_KCLASS_XTRIAL 4        /* FP32 and mixed: trial solve, first X pass (all levels); FP64: none */
+#define IBPM_KCLASS_YTRIAL 5        /* FP32 and mixed: trial solve, Y pass with the A/Ainv multiplies; FP64: none */
 #define IBPM_KCLASS_TCDST 6         /* the four tensor-core passes of a batched 2D solve; its third value
                                        counts algorithmic flops (4 nprod P^3 per field), not bytes */
 #define IBPM_KCLASS_TCLINES 7       /* the FP64 prologue of a tensor-core solve into BF16 lines */
@@ -346,7 +348,7 @@ int ibpm_warm_start_sample(ibpm_handle *h, float *features, float *target, float
  * device buffers of (nx-1) x (ny-1) doubles, column-major; x may be b (the
  * first pass reads b into scratch, the last writes x, in stream order).
  * The scratch fields and transform tables live in one static device array of
- * about 4.3 MB that each GPU loading the library keeps until exit; it limits
+ * about 2.3 MB that each GPU loading the library keeps until exit; it limits
  * (nx-1)(ny-1) to 262144 cells (nx, ny even, <= 1024, of the form 2^a 3^b 5^c).
  * Larger sizes return IBPM_ERR_INVALID.  The first call on a device (and the
  * first after a change of nx, ny) writes the tables: make it outside stream
