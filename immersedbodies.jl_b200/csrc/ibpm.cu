@@ -1152,6 +1152,10 @@ struct Engine final : ibpm_handle {
     void cg(double *x, const double *b, bool have_bx = false, bool precond = false, const double *rref = nullptr);
     void cg_collect();
     int *cg_it = nullptr;
+    // kernels of the step graphs' conditional bodies (a CG iteration, the assembled
+    // solve) and the device's counts of both at the last cg_collect
+    long long cg_loop_launches = 0, cg_dense_launches = 0;
+    unsigned cg_loops_seen = 0, cg_solves_seen = 0;
     bool cg_pending = false, cg_hit_maxiter = false;
     cudaStream_t st_side = nullptr;
     void step(const ibpm_step_params &prm_in);
@@ -1300,7 +1304,7 @@ void Engine<T>::setup() {
     prm = dalloc<StepDev>(1);
     motion = dalloc<double>(6 * (size_t)std::max(nbody, 1));
     const size_t prm_room = carved(sizeof(StepDev)), motion_room = carved(sizeof(double) * 6 * std::max(nbody, 1));
-    CK(cudaMallocHost(&pinned, kStage * (prm_room + motion_room) + 2 * carved(sizeof(double) * 8)));
+    CK(cudaMallocHost(&pinned, kStage * (prm_room + motion_room) + carved(sizeof(double) * 8) + carved(sizeof(int) * 16)));
     char *pin = pinned;
     for (int k = 0; k < kStage; ++k) {
         stage_prm[k] = reinterpret_cast<StepDev *>(pin);
@@ -1549,7 +1553,8 @@ void Engine<T>::direct_rebuild() {
 
 namespace {
 // Device-resident CG state: s[0] = ||r||, s[1] = previous ||r||, s[2] = tol,
-// s[3] = 1 while iterating; it[0] = iterations; err[2] = 1 on a non-finite residual.
+// s[3] = 1 while iterating; it[0] = iterations (it[1], it[2]: see captured); err[2] = 1
+// on a non-finite residual.
 // Preconditioned (pre = 1): s[8] = rho = r . z of the last direction, z = M r in z.
 // rref (device, may be null): the residual norm the relative tolerance scales
 // instead of ||r0|| (the reference start's, when CG starts elsewhere).
@@ -1564,7 +1569,8 @@ struct CgArgs {
     int pre;
     double *z;
     const double *rref;
-    int dense;  // the assembled form may take over (kDenseGain)
+    int dense;     // the assembled form may take over (kDenseGain)
+    int captured;  // inside a graph: it[1] counts the loop's iterations and it[2] the assembled solves
 };
 
 __device__ __forceinline__ double cg_block_sum(double v, double *red) {
@@ -1694,6 +1700,7 @@ __global__ void __cluster_dims__(kDenseCtas, 1, 1) __launch_bounds__(kDenseThrea
         a.s[1] = prev;
         a.s[3] = 0.0;
         a.it[0] = it;
+        if (a.captured) ++a.it[2];
         if (bad) a.err[2] = 1;
     }
     cl.sync();  // no block leaves while another may still write to its shared memory
@@ -1807,6 +1814,7 @@ __global__ void cg_update_kernel(CgArgs a, cudaGraphConditionalHandle h, int use
         a.s[0] = res;
         a.s[3] = cont;
         a.it[0] = it;
+        if (a.captured) ++a.it[1];
         if (use_h) cudaGraphSetConditional(h, cont ? 1u : 0u);
     }
 }
@@ -1825,8 +1833,11 @@ void Engine<T>::cg(double *x, const double *b, bool have_bx, bool precond, const
     const int n = 2 * np;
     const int nchunk = (n + 63) / 64;
     const bool dense = !precond && Bd != nullptr;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cs));
+    const bool captured = cs == cudaStreamCaptureStatusActive;
     CgArgs a{n, x, cg_r, cg_u, cg_c, b, cg_s, cg_it, err, opt.cg_maxiter, opt.cg_reltol, opt.cg_abstol, precond ? 1 : 0,
-             cg_z, rref, dense ? 1 : 0};
+             cg_z, rref, dense ? 1 : 0, captured ? 1 : 0};
     // the direction: plain, or preconditioned by Binv (z = Binv r)
     auto direction = [&]() {
         if (precond) {
@@ -1851,9 +1862,7 @@ void Engine<T>::cg(double *x, const double *b, bool have_bx, bool precond, const
         }
     }
     if (!have_bx) apply_B(x, cg_c, n, 1);  // else cg_c already holds B x
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    CK(cudaStreamIsCapturing(st, &cs));
-    if (cs == cudaStreamCaptureStatusActive) {
+    if (captured) {
         cudaGraph_t gr = nullptr;
         const cudaGraphNode_t *deps = nullptr;
         size_t ndeps = 0;
@@ -1864,7 +1873,8 @@ void Engine<T>::cg(double *x, const double *b, bool have_bx, bool precond, const
         cg_init_kernel<<<1, 256, 0, st>>>(a, hnd, hnd_dense, 1);
         check_launch();
         // a conditional node after the stream's last one; its body is captured on
-        // the side stream
+        // the side stream.  Returns the body's kernels, which count when it has run
+        // (cg_collect) and not among the graph's own.
         auto conditional = [&](cudaGraphConditionalNodeType type, cudaGraphConditionalHandle h, auto &&body_fn) {
             CK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &gr, &deps, &ndeps));
             cudaGraphNodeParams cp = {};
@@ -1876,6 +1886,7 @@ void Engine<T>::cg(double *x, const double *b, bool have_bx, bool precond, const
             CK(cudaGraphAddNode(&node, gr, deps, ndeps, &cp));
             CK(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
             cudaGraph_t body = cp.conditional.phGraph_out[0];
+            const long long before = launches;
             cudaStream_t main = st;
             st = st_side;
             try {
@@ -1890,9 +1901,12 @@ void Engine<T>::cg(double *x, const double *b, bool have_bx, bool precond, const
                 throw;
             }
             st = main;
+            const long long n_body = launches - before;
+            launches = before;
+            return n_body;
         };
-        if (dense) conditional(cudaGraphCondTypeIf, hnd_dense, assembled);
-        conditional(cudaGraphCondTypeWhile, hnd, [&] {
+        if (dense) cg_dense_launches = conditional(cudaGraphCondTypeIf, hnd_dense, assembled);
+        cg_loop_launches = conditional(cudaGraphCondTypeWhile, hnd, [&] {
             direction();
             apply_B(cg_u, cg_c, n, 1);
             cg_update_kernel<<<1, 256, 0, st>>>(a, hnd, 1);
@@ -1923,11 +1937,17 @@ void Engine<T>::cg_collect() {
     if (!cg_pending) return;
     CK(cudaMemcpyAsync(cg_s_h, cg_s, sizeof(double) * 8, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(err_h + 2, cg_it, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(err_h + 8, cg_it + 1, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(err_h + 3, err + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
     if (uses_binv_start()) CK(cudaMemcpyAsync(err_h + 1, err + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     if (tc) CK(cudaMemcpyAsync(err_h + 4, err + 4, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     cg_pending = false;
+    // running counts, taken as differences: they may wrap
+    const unsigned loops = (unsigned)err_h[8], solves = (unsigned)err_h[9];
+    launches += (long long)(loops - cg_loops_seen) * cg_loop_launches + (long long)(solves - cg_solves_seen) * cg_dense_launches;
+    cg_loops_seen = loops;
+    cg_solves_seen = solves;
     last_cg_iters = err_h[2];
     last_cg_res = cg_s_h[0];
     first_cg_res = cg_s_h[4];
