@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -462,19 +463,26 @@ struct Engine final : ibpm_handle {
     // Column-batch work buffers for kb columns.  The new buffers are allocated
     // before the old ones are freed, so a failed allocation leaves the handle as
     // it was; the captured graphs, which hold the old addresses, are dropped.
+    // bytes of t1, patch, Gw, psiw, qw, fcol and lines for kb columns
+    std::array<size_t, 7> batch_sizes(int kb) const {
+        const size_t k = (size_t)kb, g = (size_t)ng * L;
+        return {sizeof(T) * (size_t)nt * (size_t)std::max(kb, L), sizeof(T) * (size_t)patch_stride * k, sizeof(T) * g * k,
+                sizeof(T) * g * k, sizeof(T) * (size_t)nq * k, sizeof(double) * 2 * (size_t)np * k,
+                sizeof(double) * (size_t)line_len() * k};
+    }
+    long long batch_bytes(int kb) const {
+        size_t total = 0;
+        for (size_t s : batch_sizes(kb)) total += carved(s);
+        return (long long)total;
+    }
     void resize_batch_buffers(int kb) {
         CK(cudaStreamSynchronize(st));
         const int k2 = std::max(kb, L);
-        const size_t sizes[7] = {sizeof(T) * (size_t)(nt * k2),     sizeof(T) * (size_t)(patch_stride * kb),
-                                 sizeof(T) * (size_t)(ng * L * kb), sizeof(T) * (size_t)(ng * L * kb),
-                                 sizeof(T) * (size_t)(nq * kb),     sizeof(double) * 2 * (size_t)np * kb,
-                                 sizeof(double) * (size_t)(line_len() * kb)};
-        size_t total_bytes = 0;
-        for (size_t s : sizes) total_bytes += carved(s);
+        const auto sizes = batch_sizes(kb);
         void *fresh[7] = {};
-        const int before = reserve(total_bytes);
+        const int before = reserve((size_t)batch_bytes(kb));
         try {
-            for (int k = 0; k < 7; ++k) fresh[k] = dalloc<unsigned char>(sizes[k]);
+            for (size_t k = 0; k < 7; ++k) fresh[k] = dalloc<unsigned char>(sizes[k]);
         } catch (...) {
             open_block = before;
             for (void *p : fresh) dfree(p);
@@ -1148,7 +1156,8 @@ struct Engine final : ibpm_handle {
     void assemble_invert_B();
     void direct_rebuild();
     int batch_width() const;
-    int moving_batch() const;
+    void widen_for_cg();
+    bool cg_widened = false;  // the column work has been sized for the assembled CG
     void cg(double *x, const double *b, bool have_bx = false, bool precond = false, const double *rref = nullptr);
     void cg_collect();
     int *cg_it = nullptr;
@@ -1323,14 +1332,12 @@ void Engine<T>::setup() {
 
     kbatch = batch_width();
     if (!std::is_same<T, double>::value) kbatch = 1;  // FP32 builds B^-1 with an FP64 engine
-    if (!static_bodies) kbatch = moving_batch();
+    if (!static_bodies) kbatch = 2;  // the warm start applies B to two vectors at once; more: widen_for_cg
     kbatch = std::min(kbatch, 2 * np);
     const int kb = std::max(kbatch, L);
     patch_stride = 2LL * (nx + 1) * (ny + 1);
     // the column work, which goes back together (resize_batch_buffers)
-    reserve(carved(sizeof(T) * nt * kb) + carved(sizeof(double) * line_len() * kbatch) +
-            carved(sizeof(T) * patch_stride * kbatch) + 2 * carved(sizeof(T) * ng * L * kbatch) +
-            carved(sizeof(T) * nq * kbatch) + carved(sizeof(double) * 2 * (size_t)np * kbatch));
+    reserve((size_t)batch_bytes(kbatch));
     t1 = dalloc<T>(nt * kb);
     t1_fields = kb;
     lines = dalloc<double>(line_len() * kbatch);
@@ -1441,13 +1448,26 @@ int Engine<T>::batch_width() const {
     return (int)std::min<long long>(2 * np, std::max(1LL, std::min<long long>(64, (4LL << 30) / per_col)));
 }
 
-// Columns of B a moving-body handle applies at once: the warm start two vectors,
-// the assembled CG up to sixteen within about 1 GB of column work.
+// Before the first step whose CG may assemble B (kDenseGain): column work for up
+// to sixteen columns, within 1 GB and a 64th of the free memory, so that handles
+// that share a GPU leave each other room.  Fewer columns mean more batches an
+// assembly (512^2 x 4, 101 points: 16, 8, 4, 2 columns 6.4, 7.3, 9.4, 12.2 ms a
+// step, 45.8 with B applied each iteration), so a handle that gets none goes on
+// with the two it has.
 template <class T>
-int Engine<T>::moving_batch() const {
-    if (!std::is_same<T, double>::value || 2 * np > kDenseN) return 2;
-    const long long per_col = (2 * ng * L + nq + 2 * ng) * (long long)sizeof(T);
-    return (int)std::max(2LL, std::min<long long>(16, (1LL << 30) / per_col));
+void Engine<T>::widen_for_cg() {
+    if (cg_widened || Bd == nullptr || preconditioned()) return;
+    cg_widened = true;
+    size_t free_b = 0, total_b = 0;
+    CK(cudaMemGetInfo(&free_b, &total_b));
+    const long long room = std::min<long long>(1LL << 30, (long long)(free_b / 64));
+    int kb = std::min(16, 2 * np);
+    while (kb > kbatch && batch_bytes(kb) > room) --kb;
+    try {
+        grow_batch_buffers(kb);
+    } catch (const ApiError &e) {
+        if (e.code != IBPM_ERR_NOMEM) throw;
+    }
 }
 
 // _Binv_precomputed (src/coupling.jl:187-192): B column by column, then its inverse.
@@ -1975,6 +1995,7 @@ void Engine<T>::cg_collect() {
 // advance!(::CnabSolver) (src/solver.jl:155-190)
 template <class T>
 void Engine<T>::step(const ibpm_step_params &sp) {
+    widen_for_cg();
     // inc_time_index! and the host callbacks' values
     ++index;
     stage_acquire();
@@ -2576,6 +2597,7 @@ void Engine<T>::set_warm_start(ibpm_net *net, int mode, int depth) {
     CK(cudaStreamSynchronize(st));
     ws = net;
     ws_mode = mode;
+    cg_widened = false;
     drop_graphs();  // the step graph holds the previous choice
 }
 
