@@ -54,16 +54,28 @@ __global__ void tc_mult_kernel(Mult m, int P, float *tab) {
     tab[(size_t)c * P + r] = (kx != 0 && ky != 0) ? (float)m(kx, ky) : 0.0f;
 }
 
-// Plain CG with B as a matrix.  An application of B is some twenty dependent
-// launches (about 90 us at 512^2 x 4, however small the body), while its n = 2 np
-// columns in batches cost about 0.2 n of them and CG takes about 0.3 n iterations
-// per decade of residual.  So where the first residual is more than kDenseGain
-// above the tolerance, B is assembled once for the step and the iterations run in
-// one cluster: at most kDenseN rows, those of each of kDenseCtas blocks in its
-// shared memory.  512^2 x 4, 101 points, reltol 1e-12, 530 iterations: a step took
-// 49.7 ms with B applied each time, 6.3 so.  The iteration is the same; only the
-// rounding of B u differs.
+// Plain CG with B as a matrix: where CG will take more iterations than B's n = 2 np
+// columns cost in batches, B is assembled once for the step and the iterations run
+// in one cluster, at most kDenseN rows, those of each of kDenseCtas blocks in its
+// shared memory.  The iteration is the same; only the rounding of B u differs.
+// 512^2 x 4, 101 points, reltol 1e-12, 530 iterations: a step took 45.8 ms with B
+// applied each time, 6.4 so.
 constexpr double kDenseGain = 30.0;
+// The first residual over the tolerance from which on B is assembled, for batches
+// of kb columns on L levels of ng points.  One application of B is some twenty
+// dependent launches, so on a small grid a batch costs little more than one column;
+// on a large one its columns share the memory's bandwidth.  A column's cost in loop
+// iterations, measured: in batches of 16 0.13 (128^2 x 3), 0.25 (512^2 x 4), 0.45
+// (768^2 x 4), 0.40 (1024^2 x 1), 0.54 (1024^2 x 5), in batches of two 0.57, 0.64,
+// 0.78, 0.72, 0.78.  CG takes 25 to 50 iterations per decade of the residual, fewer
+// than 20 below a factor of kDenseGain.  Assembled against B applied each iteration,
+// ms a step: 1024^2 x 2, 201 points, first residual over tolerance 1e2 17.1 / 4.2,
+// 1e4 17.6 / 13.4, 1e6 18.1 / 22.0; 1024^2 x 5, 101 points, 1e2 17.8 / 9.1, 1e3 17.9 /
+// 14.0; 512^2 x 4, 101 points, 1e2 4.9 / 8.0.
+inline double dense_gain(int n, long long ng, int L, int kb) {
+    const double s = (double)ng / ((double)ng + 1e6 * (1 + 1.0 / L)), per_col = s + (1 - s) / kb;
+    return std::max(kDenseGain, std::pow(10.0, per_col * n / 33));
+}
 constexpr int kDenseCtas = 8, kDenseN = 448, kDenseThreads = 256;
 constexpr size_t dense_smem(int n) {
     const int rows = (n + kDenseCtas - 1) / kDenseCtas;
@@ -1448,7 +1460,7 @@ int Engine<T>::batch_width() const {
     return (int)std::min<long long>(2 * np, std::max(1LL, std::min<long long>(64, (4LL << 30) / per_col)));
 }
 
-// Before the first step whose CG may assemble B (kDenseGain): column work for up
+// Before the first step whose CG may assemble B (dense_gain): column work for up
 // to sixteen columns, within 1 GB and a 64th of the free memory, so that handles
 // that share a GPU leave each other room.  Fewer columns mean more batches an
 // assembly (512^2 x 4, 101 points: 16, 8, 4, 2 columns 6.4, 7.3, 9.4, 12.2 ms a
@@ -1589,8 +1601,8 @@ struct CgArgs {
     int pre;
     double *z;
     const double *rref;
-    int dense;     // the assembled form may take over (kDenseGain)
-    int captured;  // inside a graph: it[1] counts the loop's iterations and it[2] the assembled solves
+    double dense_gain;  // where the assembled form takes over (0: nowhere)
+    int captured;       // inside a graph: it[1] counts the loop's iterations and it[2] the assembled solves
 };
 
 __device__ __forceinline__ double cg_block_sum(double v, double *red) {
@@ -1630,9 +1642,9 @@ __global__ void cg_init_kernel(CgArgs a, cudaGraphConditionalHandle h, cudaGraph
         a.s[4] = res;  // initial residual, for reports
         a.s[8] = 1.0;  // rho before the first direction (u = 0 makes it immaterial)
         a.it[0] = 0;
-        const bool dense = a.dense && cont && res > kDenseGain * tol;
+        const bool dense = a.dense_gain > 0 && cont && res > a.dense_gain * tol;
         if (use_h) cudaGraphSetConditional(h, cont && !dense ? 1u : 0u);
-        if (use_h && a.dense) cudaGraphSetConditional(h_dense, dense ? 1u : 0u);
+        if (use_h && a.dense_gain > 0) cudaGraphSetConditional(h_dense, dense ? 1u : 0u);
     }
 }
 
@@ -1857,7 +1869,7 @@ void Engine<T>::cg(double *x, const double *b, bool have_bx, bool precond, const
     CK(cudaStreamIsCapturing(st, &cs));
     const bool captured = cs == cudaStreamCaptureStatusActive;
     CgArgs a{n, x, cg_r, cg_u, cg_c, b, cg_s, cg_it, err, opt.cg_maxiter, opt.cg_reltol, opt.cg_abstol, precond ? 1 : 0,
-             cg_z, rref, dense ? 1 : 0, captured ? 1 : 0};
+             cg_z, rref, dense ? dense_gain(n, ng, L, kbatch) : 0.0, captured ? 1 : 0};
     // the direction: plain, or preconditioned by Binv (z = Binv r)
     auto direction = [&]() {
         if (precond) {
@@ -1940,7 +1952,7 @@ void Engine<T>::cg(double *x, const double *b, bool have_bx, bool precond, const
         CK(cudaMemcpyAsync(cg_s_h, cg_s, sizeof(double) * 4, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         if (cg_s_h[3] == 0.0) break;
-        if (first && dense && cg_s_h[0] > kDenseGain * cg_s_h[2]) {
+        if (first && dense && cg_s_h[0] > a.dense_gain * cg_s_h[2]) {
             assembled();
             break;
         }

@@ -37,6 +37,15 @@ def test_path_taken(ib, npts, cg, assembled):
     assert (_first_iteration(ib, _problem(ib, npts), **cg) > loop) == assembled
 
 
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("npts,cg,assembled", [(201, {}, True), (201, dict(reltol=1e-2), False),
+                                               (13, dict(reltol=1e-2), True)])
+def test_a_large_grid_assembles_only_for_many_iterations(ib, npts, cg, assembled):
+    size = dict(nx=640, ny=640, L=1)
+    loop = _first_iteration(ib, _problem(ib, 400, **size))
+    assert (_first_iteration(ib, _problem(ib, npts, **size), **cg) > loop) == assembled
+
+
 @pytest.mark.parametrize("npts,cg", [(13, {}), (101, {}), (225, {}), (40, dict(reltol=0.2)),
                                      (40, dict(reltol=0.0, abstol=1e-10))])
 def test_graph_and_eager_steps_launch_the_same_kernels(ib, npts, cg):
