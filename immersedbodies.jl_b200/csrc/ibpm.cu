@@ -1132,7 +1132,15 @@ struct Engine final : ibpm_handle {
     T *diag_q = nullptr, *diag_g = nullptr;  // diag_vort2flux buffers
     void set_state(const ibpm_state_view *s) override;
     void get_field(int field, int level, double *out) override;
-    double *field_d = nullptr;  // one level of an output field
+    // One level of an output field, in memory that is idle between steps: an
+    // allocation of its own at the first read cost a fresh group of 48 FP32 cases 34
+    // instead of 19 ms for its 48 reads.
+    double *field_work() {
+        if constexpr (std::is_same<T, double>::value)
+            return qw;  // nq per column
+        else
+            return staging((size_t)nq);  // as large since set_state
+    }
     void set_warm_start(ibpm_net *net, int mode, int depth) override;
     void set_rebuild_transform(int products) override;
     void warm_start_sample(float *features, float *target, float *prediction) override;
@@ -2505,7 +2513,7 @@ void Engine<T>::get_field(int field, int level, double *out) {
     else
         throw ApiError{IBPM_ERR_INVALID, "unknown field"};
     if (!out) throw ApiError{IBPM_ERR_INVALID, "null output"};
-    if (!field_d) field_d = dalloc<double>((size_t)std::max<long long>(nq, ng));
+    double *field_d = field_work();
     if (field != IBPM_FIELD_VORTICITY) {
         ensure_q();
         materialise_q0();
