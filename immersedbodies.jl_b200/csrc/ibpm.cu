@@ -480,7 +480,7 @@ struct Engine final : ibpm_handle {
         const size_t k = (size_t)kb, g = (size_t)ng * L;
         return {sizeof(T) * (size_t)nt * (size_t)std::max(kb, L), sizeof(T) * (size_t)patch_stride * k, sizeof(T) * g * k,
                 sizeof(T) * g * k, sizeof(T) * (size_t)nq * k, sizeof(double) * 2 * (size_t)np * k,
-                sizeof(double) * (size_t)line_len() * k};
+                by_transforms ? 0 : sizeof(double) * (size_t)line_len() * k};
     }
     long long batch_bytes(int kb) const {
         size_t total = 0;
@@ -1223,9 +1223,10 @@ void Engine<T>::setup() {
         const bool f32 = !std::is_same<T, double>::value;
         const size_t n = 2 * (size_t)np, g = (size_t)ng, f = (size_t)nq;
         const bool dense = static_bodies || (!f32 && n <= (size_t)kDenseN);
+        const size_t direct = by_transforms ? 0 : (size_t)(nx - 1);
         reserve(sizeof(T) * ((size_t)nt + (f32 ? 2 : 1) * g * L + f) + (f32 ? sizeof(double) * (g + f + (size_t)nt) : 0) +
-                sizeof(double) * ((size_t)ring_ld() * (nx - 1) + (n + 63) / 64 * n + 2 * 49 * n + (dense ? n * n : 0)) +
-                sizeof(YCol) * (size_t)(nx - 1) * (L + 1) + ((size_t)1 << 19));
+                sizeof(double) * ((size_t)ring_ld() * direct + (n + 63) / 64 * n + 2 * 49 * n + (dense ? n * n : 0)) +
+                sizeof(YCol) * direct * (L + 1) + ((size_t)1 << 19));
     }
     // transform tables
     auto tables = [&](int M, C *&tw, T *&sn, double *&cs, PlanT<T> &pl) {
@@ -1256,12 +1257,14 @@ void Engine<T>::setup() {
         std::vector<double> hc(L);
         for (int lev = 1; lev <= L; ++lev) hc[lev - 1] = coef(lev);
         double *cd = coef_lev = dalloc<double>(L);
-        ycols = dalloc<YCol>((size_t)(nx - 1) * (L + 1));
-        ydiff = dalloc<double>((size_t)kYDiff * (L + 1));
-        yphase = dalloc<double2>((kYChunks + 1) * kYFull);
         CK(cudaMemcpyAsync(cd, hc.data(), sizeof(double) * L, cudaMemcpyHostToDevice, st));
-        CK(launch_ycols(ycols, ydiff, yphase, cx, cy, nx, ny, nullptr, 1, st));
-        CK(launch_ycols(ycols + (nx - 1), ydiff + kYDiff, yphase, cx, cy, nx, ny, cd, L, st));
+        if (!by_transforms) {
+            ycols = dalloc<YCol>((size_t)(nx - 1) * (L + 1));
+            ydiff = dalloc<double>((size_t)kYDiff * (L + 1));
+            yphase = dalloc<double2>((kYChunks + 1) * kYFull);
+            CK(launch_ycols(ycols, ydiff, yphase, cx, cy, nx, ny, nullptr, 1, st));
+            CK(launch_ycols(ycols + (nx - 1), ydiff + kYDiff, yphase, cx, cy, nx, ny, cd, L, st));
+        }
         CK(cudaStreamSynchronize(st));
     }
     if (!std::is_same<T, double>::value) {
@@ -1360,7 +1363,7 @@ void Engine<T>::setup() {
     reserve((size_t)batch_bytes(kbatch));
     t1 = dalloc<T>(nt * kb);
     t1_fields = kb;
-    lines = dalloc<double>(line_len() * kbatch);
+    if (!by_transforms) lines = dalloc<double>(line_len() * kbatch);
     patch = dalloc<T>(patch_stride * kbatch);
     Gw = dalloc<T>(ng * L * kbatch);
     psiw = dalloc<T>(ng * L * kbatch);
@@ -1398,18 +1401,21 @@ void Engine<T>::setup() {
     cg_it = dalloc<int>(4);
     CK(cudaStreamCreateWithFlags(&st_side, cudaStreamNonBlocking));
 
-    // 2 sin(pi kx i / nx) of the columns nx/4 and 3 nx/4
-    std::vector<double> hw(2 * (size_t)nx, 0.0);
-    for (int c = 0; c < 2; ++c)
-        for (long long k = 1; k < nx; ++k)
-            hw[c * nx + k - 1] = (double)(2 * sinl(3.14159265358979323846264338327950288L *
-                                                   (long double)(k * ((c ? 3 : 1) * nx / 4) % (2 * nx)) / (long double)nx));
-    ring_q = dalloc<double>((size_t)ring_ld() * (nx - 1));
-    ring_matrix_kernel<<<dim3((ring_ld() + 127) / 128, nx - 1), 128, 0, st>>>(ring_q, ring_ld(), ring_step(), nx,
-                                                                            plan_x<double>().sn);
-    check_launch();
-    line_w = dalloc<double>(2 * (size_t)nx);
-    CK(cudaMemcpyAsync(line_w, hw.data(), sizeof(double) * 2 * nx, cudaMemcpyHostToDevice, st));
+    if (!by_transforms) {
+        // 2 sin(pi kx i / nx) of the columns nx/4 and 3 nx/4
+        std::vector<double> hw(2 * (size_t)nx, 0.0);
+        for (int c = 0; c < 2; ++c)
+            for (long long k = 1; k < nx; ++k)
+                hw[c * nx + k - 1] = (double)(2 * sinl(3.14159265358979323846264338327950288L *
+                                                       (long double)(k * ((c ? 3 : 1) * nx / 4) % (2 * nx)) / (long double)nx));
+        ring_q = dalloc<double>((size_t)ring_ld() * (nx - 1));
+        ring_matrix_kernel<<<dim3((ring_ld() + 127) / 128, nx - 1), 128, 0, st>>>(ring_q, ring_ld(), ring_step(), nx,
+                                                                                plan_x<double>().sn);
+        check_launch();
+        line_w = dalloc<double>(2 * (size_t)nx);
+        CK(cudaMemcpyAsync(line_w, hw.data(), sizeof(double) * 2 * nx, cudaMemcpyHostToDevice, st));
+        CK(cudaStreamSynchronize(st));
+    }
     // a window's rows: what a curl of faces j0 .. j1 reads, j0 - 1 .. j1
     std::vector<int> hc(4 * (size_t)L, 0);
     for (int lev = 1; lev <= L; ++lev) {
@@ -2991,7 +2997,6 @@ struct CaseGroup {
         nl[0] = alloc<T>(ngL * C);
         nl[1] = alloc<T>(ngL * C);
         t1 = alloc<T>((size_t)(e0->nt * L) * C);
-        lines = alloc<double>((size_t)e0->line_len() * C);
         if (!std::is_same<T, double>::value) t2 = alloc<T>(ngL * C);
         rest = alloc<T>(ngL * C);
         qs1 = alloc<T>((size_t)nq * C);
@@ -3009,11 +3014,14 @@ struct CaseGroup {
         }
         coef_all = alloc<double>(ca.size());
         re_tab = alloc<double>(C);
-        ycols = alloc<YCol>((size_t)(e0->nx - 1) * C * L);
-        ydiff = alloc<double>((size_t)kYDiff * C * L);
         CK(cudaMemcpyAsync(coef_all, ca.data(), sizeof(double) * ca.size(), cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(re_tab, re.data(), sizeof(double) * C, cudaMemcpyHostToDevice, st));
-        CK(launch_ycols(ycols, ydiff, e0->yphase, e0->cx, e0->cy, e0->nx, e0->ny, coef_all, C * L, st));
+        if (!e0->by_transforms) {
+            lines = alloc<double>((size_t)e0->line_len() * C);
+            ycols = alloc<YCol>((size_t)(e0->nx - 1) * C * L);
+            ydiff = alloc<double>((size_t)kYDiff * C * L);
+            CK(launch_ycols(ycols, ydiff, e0->yphase, e0->cx, e0->cy, e0->nx, e0->ny, coef_all, C * L, st));
+        }
         std::vector<CaseView> hv(C);
         views = alloc<CaseView>(C);
         bbox_tab = alloc<int>(4 * (size_t)C);
