@@ -151,17 +151,19 @@ bool make_plan(int M, PlanT<T> &pl) {
 }
 
 // ---- pass-shape autotuner ----
-// The Y pass (ytri.cuh) runs with NG column pairs per block, NG in {1, 2, 4, 8}
-// (8 runs as 4).  Every NG evaluates the same per-column arithmetic, so the
+// The Y pass (ytri.cuh, or by transforms) runs with NG column pairs per block, NG in
+// {1, 2, 4, 8} (the direct solve runs 8 as 4).  Every NG evaluates the same per-column arithmetic, so the
 // choice changes speed only, never results.
 // The best NG depends on the transform length, the precision and how many
 // fields one launch covers (one level, all levels, an ensemble group, a batch
 // of B columns), so the table is keyed by (GPU name, transform length,
-// precision, batch bucket).  With IBPM_TUNE=1 an engine times every NG on its
+// precision, batch bucket), and for the direct solve by its form and nx too: a
+// launch has nx - 1 columns a field, and choices timed on the transforms, which
+// had the shorter key, say nothing about it.  With IBPM_TUNE=1 an engine times every NG on its
 // own scratch fields for each key it will launch (before any graph capture) and
 // keeps the fastest; IBPM_TUNE_CACHE names a text file the table is read from
 // at first use and appended to after tuning, so later processes start tuned.
-// Keys never tuned use the fixed rule (ytri_wshift).
+// Keys never tuned use the fixed rule (ypass_ng).
 // IBPM_TUNE_FORCE_NG forces one NG everywhere (a test knob).
 constexpr int kTuneNGs[4] = {1, 2, 4, 8};
 inline int batch_bucket(int nb) { return nb <= 1 ? 0 : nb <= 4 ? 1 : nb <= 15 ? 2 : nb <= 63 ? 3 : 4; }
@@ -629,7 +631,7 @@ struct Engine final : ibpm_handle {
     template <class R>
     std::string ypass_key(int M, int nbatch) const {
         return devname + " ypass M=" + std::to_string(M) + (sizeof(R) == 8 ? " fp64" : " fp32") +
-               " batch=" + std::to_string(batch_bucket(nbatch));
+               " batch=" + std::to_string(batch_bucket(nbatch)) + (by_transforms ? "" : " direct nx=" + std::to_string(nx));
     }
     // The solves' y direction by transforms, as the FP32 engine does it in both
     // precisions (see ypass_kernel); the FP64 engine only where it assembles the
@@ -695,6 +697,7 @@ struct Engine final : ibpm_handle {
         float best = 1e30f;
         int best_ng = kNG;
         for (int ngy : kTuneNGs) {
+            if (!by_transforms && 2 * ngy > kYMaxW) continue;  // the shape before it again
             auto run = [&] {
                 if constexpr (std::is_same<T, double>::value)
                     ypass_launch(ngy, f, nbatch, ysolve(MULT_LAPINV, 1, 0), nt);
