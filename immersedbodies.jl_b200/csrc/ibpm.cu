@@ -610,8 +610,20 @@ struct Engine final : ibpm_handle {
                                  st, in, out, pl, nrows, o.rows, o.zero_outside, o.rows_stride, o.rows_mod));
         });
         check_launch();
-        prof_end(pe, IBPM_KCLASS_XPASS, 2.0 * sizeof(R) * (double)ng * nbatch);
+        const double rin = window_rows(o, nbatch), rout = o.zero_outside ? (double)nrows * nbatch : rin;
+        prof_end(pe, IBPM_KCLASS_XPASS, sizeof(R) * (double)(nx - 1) * (rin + rout * (ReadsTarget<Out>::value ? 2 : 1)));
     }
+    // the rows of nbatch fields that an X pass reads, for the profile's byte counts
+    double window_rows(const XOpt &o, int nbatch) const {
+        if (o.rows == nullptr) return (double)(ny - 1) * nbatch;
+        if (o.rows == P.bbox) return (double)std::max(0, std::min(ny - 1, bbox_h[3]) - std::max(1, bbox_h[2] - 1) + 1) * nbatch;
+        if (o.rows < central_win || o.rows >= central_win + 4 * L) return (double)(ny - 1) * nbatch;  // a group's windows
+        double n = 0;
+        for (int k = 0; k < o.rows_mod; ++k)
+            n += (o.rows - central_win) / 4 + k == 0 ? ny - 1 : (3 * ny / 4 - 1) - (ny / 4 + 1) + 1;
+        return n * (nbatch / o.rows_mod);
+    }
+    int bbox_h[4] = {1, 0, 1, 0};  // the body's window on the host, while profiling
     // the finer level's boundary values alone, from a solved scratch field
     // (psi_, pbs, win, win_stride: see xlines_kernel)
     void xlines(const InPlain<T> &in, int nbatch, T *psi_, long long pbs, const int *win, int win_stride) {
@@ -1018,7 +1030,12 @@ struct Engine final : ibpm_handle {
             CK(launch_overlapped(overlap(nbatch), curl_kernel<T, T, T>, grd, blk, 0, st, qout, qbs, psi_, bs,
                                  L > 1 ? psi_ + ng : nullptr, bs, g, win, 1, nullptr));
         check_launch();
-        prof_end(pe, IBPM_KCLASS_CURL, 8.0 * (double)(ng + nq) * grd.z);
+        double n = (double)(ng + nq) * grd.z;
+        if (win != nullptr && win == P.bbox) {  // both faces of each window position, and psi around them
+            const double w = std::max(0, bbox_h[1] - bbox_h[0] + 1), h = std::max(0, bbox_h[3] - bbox_h[2] + 1);
+            n = (2 * w * h + (w + 1) * (h + 1)) * nbatch;
+        }
+        prof_end(pe, IBPM_KCLASS_CURL, sizeof(T) * n);
     }
 
     // The telescoping solves with the tensor-core transforms (a rebuild's B).
@@ -1096,7 +1113,9 @@ struct Engine final : ibpm_handle {
     void check_region_error() {
         cg_collect();
         CK(cudaMemcpyAsync(err_h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        if (prof) CK(cudaMemcpyAsync(err_h + 12, P.bbox, sizeof(bbox_h), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        if (prof) std::copy(err_h + 12, err_h + 16, bbox_h);
         const int e = *err_h;
         if (e > 0) {
             CK(cudaMemsetAsync(err, 0, sizeof(int), st));
@@ -2123,7 +2142,7 @@ void Engine<T>::step_body() {
         else
             nonlinear_kernel<T><<<grd, blk, 0, st>>>(a);
         check_launch();
-        prof_end(pe, IBPM_KCLASS_NONLINEAR, 8.0 * (double)(nq + 4 * ng) * L);
+        prof_end(pe, IBPM_KCLASS_NONLINEAR, sizeof(T) * (double)((q_given ? nq : ng) + 4 * ng) * L);
     }
     if constexpr (std::is_same<T, double>::value)
         trial(rest, Gnew, L, ysolve(MULT_AIMPL, 1, 1), t1);
@@ -2784,6 +2803,7 @@ template <class T>
 void Engine<T>::set_profile(int enable) {
     CK(cudaStreamSynchronize(st));
     prof = enable != 0;
+    if (prof) CK(cudaMemcpy(bbox_h, P.bbox, sizeof(bbox_h), cudaMemcpyDeviceToHost));
     prof_recs.clear();
     ev_next = 0;
 }

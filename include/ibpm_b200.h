@@ -203,7 +203,8 @@ int64_t ibpm_kernel_launches(const ibpm_handle *h);
  * launch of the classes below is bracketed by CUDA events on the handle's
  * stream.  ibpm_profile(h, 1) clears the counters; ibpm_profile_read gives the
  * launches, summed device time (ms) and algorithmic bytes (one read of each
- * input field and one write of each output field) of a class. */
+ * input field and one write of each output field, of a launch over the body's
+ * window those inside it) of a class. */
 #define IBPM_KCLASS_XPASS 0         /* DST along x (row pass) */
 #define IBPM_KCLASS_YPASS 1         /* the multiplier along y: FP64 a direct solve per column, else DST,
                                        multiply, DST */
