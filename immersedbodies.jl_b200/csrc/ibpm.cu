@@ -1768,7 +1768,7 @@ __global__ void __cluster_dims__(kDenseCtas, 1, 1) __launch_bounds__(kDenseThrea
         a.s[1] = prev;
         a.s[3] = 0.0;
         a.it[0] = it;
-        if (a.captured) ++a.it[2];
+        if (a.captured) atomicAdd(&a.it[2], 1);
         if (bad) a.err[2] = 1;
     }
     cl.sync();  // no block leaves while another may still write to its shared memory
@@ -1882,7 +1882,7 @@ __global__ void cg_update_kernel(CgArgs a, cudaGraphConditionalHandle h, int use
         a.s[0] = res;
         a.s[3] = cont;
         a.it[0] = it;
-        if (a.captured) ++a.it[1];
+        if (a.captured) atomicAdd(&a.it[1], 1);  // no result wanted: nothing waits for it
         if (use_h) cudaGraphSetConditional(h, cont ? 1u : 0u);
     }
 }
@@ -2004,19 +2004,18 @@ template <class T>
 void Engine<T>::cg_collect() {
     if (!cg_pending) return;
     CK(cudaMemcpyAsync(cg_s_h, cg_s, sizeof(double) * 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(err_h + 2, cg_it, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(err_h + 8, cg_it + 1, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(err_h + 8, cg_it, sizeof(int) * 3, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(err_h + 3, err + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
     if (uses_binv_start()) CK(cudaMemcpyAsync(err_h + 1, err + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     if (tc) CK(cudaMemcpyAsync(err_h + 4, err + 4, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     cg_pending = false;
     // running counts, taken as differences: they may wrap
-    const unsigned loops = (unsigned)err_h[8], solves = (unsigned)err_h[9];
+    const unsigned loops = (unsigned)err_h[9], solves = (unsigned)err_h[10];
     launches += (long long)(loops - cg_loops_seen) * cg_loop_launches + (long long)(solves - cg_solves_seen) * cg_dense_launches;
     cg_loops_seen = loops;
     cg_solves_seen = solves;
-    last_cg_iters = err_h[2];
+    last_cg_iters = err_h[8];
     last_cg_res = cg_s_h[0];
     first_cg_res = cg_s_h[4];
     // projected: directions kept; extrapolated, learned: the Galerkin coefficient
