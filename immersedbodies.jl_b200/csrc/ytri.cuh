@@ -20,7 +20,8 @@
 // written once (in place if wanted), about 14 FP64 operations a row, two
 // barriers: the two transforms it replaces are 60 operations a row each through
 // seven shared-memory round trips.  Measured, back to back in a graph: one
-// 1024^2 FP64 field 6.5 us (20.6 as transforms; 2.6 TB/s read and written), five
+// 1024^2 FP64 field 6.5 us with the correction of the low modes described below, 5.2
+// without (20.6 as transforms; 2.6 TB/s read and written with it), five
 // in one launch 20.3 us (78), one 512^2 field 4.7 us.  Bound by latency for one
 // field (load, scan, store in one wave), by memory for many.  1 - r is kept to full relative accuracy
 // (r as a two-part sum), so small t loses nothing.

@@ -181,8 +181,8 @@ int ibpm_ensemble_groups(const ibpm_ensemble *e, int32_t *ngroups, int32_t *nbat
  * DST-diagonalised solves runs with NG column pairs per block, NG in {1, 2, 4, 8}
  * (the FP64 engine's direct y solve runs 8 as 4); every NG gives the same bits.  With the environment variable
  * IBPM_TUNE=1, engines (and ensemble groups) time every NG on the device for
- * each (GPU, transform length, precision, batch bucket) they launch, before
- * their first step, and keep the fastest; IBPM_TUNE_CACHE=<file> reads the table
+ * each (GPU, transform length, precision, batch bucket; for the direct solve its
+ * form and nx too) they launch, before their first step, and keep the fastest; IBPM_TUNE_CACHE=<file> reads the table
  * from that file at first use and appends new choices to it.  Untuned keys use
  * a fixed rule on the columns per launch (FP32 and mixed: NG = 2, or 4 from 16
  * fields per launch).  IBPM_TUNE_FORCE_NG=<n> forces one NG.
@@ -196,7 +196,8 @@ const char *ibpm_last_error(const ibpm_handle *h);
 
 /* The library's CUDA stream (cudaStream_t) for callers that time on it. */
 void *ibpm_stream(ibpm_handle *h);
-/* Number of kernels this handle launched so far (instrumentation). */
+/* Number of kernels this handle launched so far (instrumentation); a step's CG
+ * bodies count as often as they ran. */
 int64_t ibpm_kernel_launches(const ibpm_handle *h);
 
 /* Kernel timing (instrumentation for roofline reports): when enabled, every
