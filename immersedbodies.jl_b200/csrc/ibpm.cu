@@ -3243,6 +3243,17 @@ struct CaseGroup {
         }
         CK(cudaMemcpyAsync(prm_tab, stage_h[k], sizeof(StepDev) * C, cudaMemcpyHostToDevice, st));
         CK(cudaEventRecord(stage_ev[k], st));
+        // a case stepped on its own since has its Gamma and last nonlinear term in the
+        // other buffer of each pair
+        for (int c = 0; c < C; ++c) {
+            Engine<T> &e = *cs[c];
+            if (e.gc == gc) continue;
+            const size_t at = (size_t)(ng * L) * c, bytes = sizeof(T) * (size_t)(ng * L);
+            CK(cudaMemcpyAsync(G[gc] + at, G[1 - gc] + at, bytes, cudaMemcpyDeviceToDevice, st));
+            CK(cudaMemcpyAsync(nl[1 - nc] + at, nl[nc] + at, bytes, cudaMemcpyDeviceToDevice, st));
+            e.gc = gc;
+            e.nc = nc;
+        }
         q_given = false;
         for (const Engine<T> *e : cs) q_given = q_given || e->q_given;
         if (q_given)
